@@ -37,7 +37,7 @@ def csr_from_dst(edge_dst: torch.Tensor, num_nodes: int) -> Tuple[torch.Tensor, 
     rowptr = torch.empty(num_nodes + 1, dtype=torch.int64, device=dev)
     nbytes = core.e3b_csr_scratch_bytes(E, num_nodes)
     scratch = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev)
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    status = torch.empty(1, dtype=torch.int32, device=dev)      # (zeroed by the call)
     with torch.cuda.device(dev):
         rc = core.e3b_csr_from_dst(_lib._ptr(edge_dst), E, num_nodes, _lib._ptr(perm), _lib._ptr(rowptr),
                                    _lib._ptr(scratch), scratch.numel(), _lib._ptr(status), _lib.stream_ptr())

@@ -88,7 +88,7 @@ int e3b_csr_from_dst(const int64_t* dst, int64_t num_edges, int64_t num_nodes, i
  * Limits and rules:
  *   - at most e3b_csr_static_max_edges() edges (262,144) and e3b_csr_static_max_nodes() nodes
  *     (65,536); larger problems are rejected with E3B_ERR_ARG and a message naming the limits;
- *   - every GPU that loads the library holds the work area (about 4.4 MiB) until the process exits;
+ *   - every GPU that loads the library holds the work area (about 4.1 MiB) until the process exits;
  *   - the first call on each device looks up the work area's device address (with that device
  *     current); make that first call before starting any stream capture;
  *   - all calls on a device share the one work area: it keeps the previous call's contents, the
