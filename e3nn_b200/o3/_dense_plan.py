@@ -1,8 +1,10 @@
-"""Host-side construction of "dense plans" for ``e3b_dense_fwd`` (layout in csrc/dense.cu).
+"""Host-side construction of "dense plans" for ``e3b_dense_fwd`` (layouts in csrc/dense.cu and csrc/dense_tile.cu).
 
-A plan lists, per output irrep, the (path, u, v) triples that are contracted against the
+The first part of a plan lists, per output irrep, the (path, u, v) triples that are contracted against the
 shared weights, and for every path the Clebsch-Gordan non-zeros (with the path coefficient
-folded in) that turn a pair of input rows into the left operand of that contraction.
+folded in) that turn a pair of input rows into the left operand of that contraction.  The second part describes the
+same contraction by whole paths, cut into chunks of 32 channels, for the register-tile kernels; the plan's last word
+is its offset.
 """
 from __future__ import annotations
 
@@ -28,6 +30,17 @@ class _Builder:
         self.paths: List[List[Tuple[int, int]]] = []   # per path, per k: (cg_start, cg_count)
         self.cg: List[int] = []
         self.max_k = 0
+        # second part
+        self.wpaths: List[dict] = []
+        self.wgroups: List[Tuple[int, int, int, List[int]]] = []     # out_off, mul_out, dim3, whole paths
+
+    def add_whole_path(self, **path) -> int:
+        """x1off, m1, d1; x2off (-1: no second operand), m2, d2; out_off, mo, d3; wbase, su, sv, sw; c [d1, d2, d3] or coef."""
+        self.wpaths.append(path)
+        return len(self.wpaths) - 1
+
+    def add_whole_group(self, out_off: int, mul_out: int, dim3: int, paths: Sequence[int]):
+        self.wgroups.append((out_off, mul_out, dim3, list(paths)))
 
     def add_path(self, per_k: Sequence[Sequence[Tuple[int, int, float]]]) -> int:
         entry = []
@@ -60,14 +73,75 @@ class _Builder:
             for s, c in entry:
                 pathk_words += [s, c]
         off_cg = base + len(pathk_words)
-        total = off_cg + len(self.cg)
+        second, where = self._second_part(off_cg + len(self.cg))
+        total = off_cg + len(self.cg) + len(second) + 1
         words = [MAGIC, self.d1, self.d2, self.dout, len(self.groups), n_paths, total,
                  off_groups, off_kent, off_pathk, off_cg, self.max_k]
         for g in self.groups:
             words += g
-        words += self.kent + dir_words + pathk_words + self.cg
+        words += self.kent + dir_words + pathk_words + self.cg + second + [where]
         assert len(words) == total
         return np.asarray(words, dtype=np.int64).astype(np.int32)
+
+    def _second_part(self, base: int) -> Tuple[List[int], int]:
+        """Words of the second part, which starts at word ``base`` of the plan, and the offset of its header."""
+        words: List[int] = []
+
+        def segments(lists) -> int:
+            """Pairs (index, coefficient) of every list, then the word offsets of the lists' ends; returns where those start."""
+            ends = [base + len(words)]
+            for pairs in lists:
+                for i, c in pairs:
+                    words.extend([i, _f2i(c)])
+                ends.append(base + len(words))
+            at = base + len(words)
+            words.extend(ends)
+            return at
+
+        rows, d1max, d3max = [], 1, 1
+        for p in self.wpaths:
+            d1, d2, d3 = p["d1"], p["d2"], p["d3"]
+            d1max, d3max = max(d1max, d1), max(d3max, d3)
+            ki = jj = 0
+            if p["x2off"] >= 0:
+                c = p["c"]
+                ki = segments([[(j, float(c[i, j, k])) for j in range(d2) if c[i, j, k] != 0.0] for k in range(d3) for i in range(d1)])
+                jj = segments([[(i * d3 + k, float(c[i, j, k])) for i in range(d1) for k in range(d3) if c[i, j, k] != 0.0] for j in range(d2)])
+            rows.append([d1, d2, d3, p["su"], p["sw"], ki, jj, p["x1off"], p["m1"], p["x2off"], p["m2"], p["out_off"], p["mo"],
+                         p["wbase"], p["sv"], _f2i(p.get("coef", 0.0))])
+        chunks, groups = [], []
+        for out_off, mo, d3, members in self.wgroups:
+            first = len(chunks)
+            for n in members:
+                p = self.wpaths[n]
+                for v in range(p["m2"]):
+                    x2off = p["x2off"] + v * p["d2"] if p["x2off"] >= 0 else -1
+                    for u0 in range(0, p["m1"], 32):
+                        chunks.append([n, p["x1off"] + u0 * p["d1"], min(32, p["m1"] - u0), x2off,
+                                       p["wbase"] + u0 * p["su"] + v * p["sv"], int(u0 == 0)])
+            groups.append([out_off, mo, d3, first, len(chunks) - first, 0])
+        # the paths that leave each block of the first operand (operand gradients of a product)
+        blocks = {}
+        for n, p in enumerate(self.wpaths):
+            if p["x2off"] >= 0 and p["m1"] * p["m2"] * p["mo"] > 0:
+                blocks.setdefault((p["x1off"], p["m1"], p["d1"]), []).append(n)
+        in_paths = [n for members in blocks.values() for n in members]
+        in_groups, at = [], 0
+        for (x1off, m1, d1), members in blocks.items():
+            in_groups.append([x1off, m1, d1, at, len(members)])
+            at += len(members)
+        covered = sum(m1 * d1 for _, m1, d1 in blocks) == self.d1
+        offs = []
+        for table in (groups, chunks, rows, in_groups):
+            offs.append(base + len(words))
+            for r in table:
+                words.extend(r)
+        offs.append(base + len(words))
+        words.extend(in_paths)
+        header = base + len(words)
+        words.extend([len(groups), offs[0], len(chunks), offs[1], len(rows), offs[2], len(in_groups), offs[3], d1max, d3max, offs[4],
+                      int(covered)])
+        return words, header
 
 
 def uvw_plan(spec, instruction_ids: Optional[Sequence[int]] = None) -> Tuple[np.ndarray, List[int]]:
@@ -81,7 +155,7 @@ def uvw_plan(spec, instruction_ids: Optional[Sequence[int]] = None) -> Tuple[np.
         live = [(n, ins) for n, ins in live if n in set(instruction_ids)]
     written = sorted({ins.i_out for _, ins in live})
     for out_idx in written:
-        kents = []
+        kents, whole = [], []
         mul_out, ir_out = io[out_idx]
         for n, ins in live:
             if ins.i_out != out_idx:
@@ -96,7 +170,11 @@ def uvw_plan(spec, instruction_ids: Optional[Sequence[int]] = None) -> Tuple[np.
                 for v in range(m2):
                     kents.append((pid, o1[ins.i_in1] + u * ir1.dim, o2[ins.i_in2] + v * ir2.dim,
                                   woffs[n] + (u * m2 + v) * mul_out))
+            whole.append(b.add_whole_path(x1off=o1[ins.i_in1], m1=m1, d1=ir1.dim, x2off=o2[ins.i_in2], m2=m2, d2=ir2.dim,
+                                          out_off=oo[out_idx], mo=mul_out, d3=ir_out.dim, wbase=woffs[n], su=m2 * mul_out, sv=mul_out,
+                                          sw=1, c=c))
         b.add_group(oo[out_idx], mul_out, ir_out.dim, kents, 1)
+        b.add_whole_group(oo[out_idx], mul_out, ir_out.dim, whole)
     return b.finish(), written
 
 
@@ -122,7 +200,7 @@ def linear_plan(irreps_in: Irreps, irreps_out: Irreps, instructions, transpose: 
         mul_t, ir = dst[t]
         # a group reads W with one stride: forward 1; transposed the output multiplicity of the path, so the
         # paths out of one input irrep are grouped by it (the caller accumulates the groups of a target)
-        by_stride = {}
+        by_stride, whole = {}, []
         for n, ins in live:
             if (ins.i_in if transpose else ins.i_out) != t:
                 continue
@@ -135,6 +213,10 @@ def linear_plan(irreps_in: Irreps, irreps_out: Irreps, instructions, transpose: 
                 # forward: W[u=q, w] contiguous in w; transpose: W[u, w=q] strided by mul_out in u
                 wbase = offs[n] + (q if transpose else q * mul_out)
                 kents.append((pid, so[s] + q * ir.dim, -1, wbase))
+            whole.append(b.add_whole_path(x1off=so[s], m1=mul_s, d1=ir.dim, x2off=-1, m2=1, d2=1, out_off=do[t], mo=mul_t, d3=ir.dim,
+                                          wbase=offs[n], su=1 if transpose else mul_out, sv=0, sw=mul_out if transpose else 1,
+                                          coef=float(ins.path_weight)))
         for stride, kents in by_stride.items():
             b.add_group(do[t], mul_t, ir.dim, kents, stride)
+        b.add_whole_group(do[t], mul_t, ir.dim, whole)
     return b.finish(), targets

@@ -83,11 +83,11 @@ class _LinearFunction(torch.autograd.Function):
             gx = torch.empty(Z, lin.irreps_in.dim, dtype=torch.float32, device=dev)
             _lib.tc_gemm_module(lin._tc_bwd).run(grad_out, None, w, gx, lin._precision)
             return gx, gw, gb, None
-        gx = torch.zeros(Z, lin.irreps_in.dim, dtype=torch.float32, device=dev)
+        gx = (torch.empty if lin._reads_all else torch.zeros)(Z, lin.irreps_in.dim, dtype=torch.float32, device=dev)
         if lin.weight_numel > 0:
             with torch.cuda.device(dev):
                 rc = _lib.core().e3b_dense_fwd(lin._plan_t_host.ctypes.data, _lib._ptr(lin._plan_on(dev, True)),
-                                               _lib._ptr(grad_out), None, _lib._ptr(w), 0, _lib._ptr(gx), Z, 1,
+                                               _lib._ptr(grad_out), None, _lib._ptr(w), 0, _lib._ptr(gx), Z, 0,
                                                _lib.stream_ptr())
             _lib.check(rc, "e3b_dense_fwd (transposed)")
         return gx, gw, gb, None
@@ -138,7 +138,8 @@ class Linear(torch.nn.Module):
         # the flat weight vector skips empty instructions, exactly as the reference's code generator does
         packed = [ins if 0 not in ins.path_shape else ins._replace(path_shape=(0, 0)) for ins in self.instructions]
         self._plan_host, written = linear_plan(irreps_in, irreps_out, packed, transpose=False)
-        self._plan_t_host, _ = linear_plan(irreps_in, irreps_out, packed, transpose=True)
+        self._plan_t_host, read = linear_plan(irreps_in, irreps_out, packed, transpose=True)
+        self._reads_all = all(i in read for i, (mul, ir) in enumerate(irreps_in) if mul * ir.dim > 0)
         self._plan_dev = {}
         # tensor-core modules (None when the multiplicities do not fit the 32-wide K chunks / 16-wide N)
         tag = hashlib.sha1(repr((str(irreps_in), str(irreps_out), [(i.i_in, i.i_out, i.path_shape, repr(i.path_weight))

@@ -60,8 +60,8 @@ class _UvuFunction(torch.autograd.Function):
 
 class _UvwFunction(torch.autograd.Function):
     """Weight-shared or per-row 'uvw' paths: forward on the engine the module's ``math_mode`` selects; gradients
-    w.r.t. the two operands as two derived 'uvw' products of the cotangent (``TensorProduct._vjp_module``), w.r.t.
-    shared weights by ``e3b_dense_bwd_w``, w.r.t. per-row weights by ``TensorProduct._uvw_row_weight_grad``."""
+    w.r.t. the two operands by ``e3b_dense_bwd_x``, or as two derived 'uvw' products of the cotangent
+    (``TensorProduct._vjp_module``: per-row weights, l > 3, a tensor-core mode's first operand alone), w.r.t. shared weights by ``e3b_dense_bwd_w``, w.r.t. per-row weights by ``TensorProduct._uvw_row_weight_grad``."""
 
     @staticmethod
     def forward(ctx, x1, x2, w, out, tp, accumulate: bool):
@@ -80,6 +80,17 @@ class _UvwFunction(torch.autograd.Function):
         g = grad_out.contiguous()
         g1 = g2 = gw = None
         with torch.no_grad():
+            # both operand gradients share one intermediate per path: one kernel.  A tensor-core mode that only needs
+            # the first operand's gradient takes its derived product instead, which runs on the tensor cores.
+            if tp._uvw_bwd_x_ok() and (need2 or (need1 and tp.math_mode == "fp32")):
+                g1 = torch.empty_like(x1) if need1 else None
+                g2 = torch.empty_like(x2) if need2 else None
+                with torch.cuda.device(g.device):
+                    rc = _lib.core().e3b_dense_bwd_x(tp._plan_host.ctypes.data, _lib._ptr(tp._plan_on(g.device)), _lib._ptr(x1),
+                                                     _lib._ptr(x2), _lib._ptr(w), _lib._ptr(g), _lib._ptr(g1), _lib._ptr(g2),
+                                                     x1.shape[0], _lib.stream_ptr())
+                _lib.check(rc, "e3b_dense_bwd_x")
+                need1 = need2 = False
             if need1:
                 g1 = tp._vjp_module(0)(g, x2, tp._vjp_weights(0, w))
             if need2:
@@ -426,6 +437,12 @@ class TensorProduct(torch.nn.Module):
                                            int(accumulate), _lib.stream_ptr())
         _lib.check(rc, "e3b_dense_fwd")
         return out
+
+    def _uvw_bwd_x_ok(self) -> bool:
+        """Whether ``e3b_dense_bwd_x`` covers the 'uvw' paths (shared weights, l <= 3)."""
+        if not hasattr(self, "_bwd_x_ok"):
+            self._bwd_x_ok = bool(self.shared_weights and _lib.core().e3b_dense_bwd_x_supported(self._plan_host.ctypes.data))
+        return self._bwd_x_ok
 
     # ---- gradients of the 'uvw' paths w.r.t. the operands -----------------------------------------------
     # The product is trilinear, so its transpose in one operand is again a 'uvw' product: of the cotangent and

@@ -191,7 +191,7 @@ int e3b_gate_bwd(const float* x, const float* grad_out, const int32_t* in_table,
  * (e3nn/o3/_tensor_product/_codegen.py:148-165 with the accumulation of :312-343) and the
  * per-irrep Linear out[z,w,i] = pw sum_u W[u,w] x[z,u,i] (e3nn/o3/_linear.py:445-469).
  * The contraction is described by a "dense plan": int32 words built on the host
- * (layout documented in e3nn_b200/csrc/dense.cu); plan_host is that array in HOST memory,
+ * (layout documented in e3nn_b200/csrc/dense.cu and dense_tile.cu); plan_host is that array in HOST memory,
  * plan_dev a copy in device memory.  x2 may be NULL for plans that never read it (Linear).
  * weight_row_stride: 0 for shared weights [weight_numel]; otherwise row z reads its own weights at
  * weight + z * weight_row_stride (e3nn's shared_weights=False).
@@ -226,6 +226,19 @@ int e3b_dense_fwd_gate(const int32_t* plan_host, const int32_t* plan_dev, const 
  */
 int e3b_dense_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2,
                     const float* grad_out, float* grad_weight, int64_t num_rows, void* stream);
+
+/*
+ * Gradients of a 'uvw' product with SHARED weights w.r.t. its two operands (what autograd derives from the einsums of
+ * e3nn/o3/_tensor_product/_codegen.py:148-165 for x and y), with the plan of the forward call:
+ *   grad_x1[z,u,i] = sum pw W[u,v,w] C_ijk x2[z,v,j] g[z,w,k],   grad_x2[z,v,j] = sum pw W[u,v,w] C_ijk x1[z,u,i] g[z,w,k].
+ * Either output may be NULL.  grad_x1 [rows, d1] and grad_x2 [rows, d2] are overwritten (columns no path reads become
+ * zero); grad_x2 is summed with float atomics over the blocks of x1's irreps.
+ * e3b_dense_bwd_x_supported(plan_host): 1 when every irrep of the plan has l <= 3 and x2's row fits the kernel's shared
+ * memory, else 0 (the caller then evaluates the two transposed products with e3b_dense_fwd).
+ */
+int e3b_dense_bwd_x_supported(const int32_t* plan_host);
+int e3b_dense_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
+                    const float* grad_out, float* grad_x1, float* grad_x2, int64_t num_rows, void* stream);
 
 /*
  * out[z, col0 + c] = (add ? out[z, col0 + c] : 0) + (bias ? bias[c] : 0) for c < ncol: zero fill of

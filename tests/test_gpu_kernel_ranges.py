@@ -4,6 +4,8 @@ import torch
 
 import e3nn_b200
 from conftest import rel_err
+from e3nn_b200 import nn as bnn
+from e3nn_b200 import o3
 from oracle import e3nn_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -30,7 +32,7 @@ def test_neighbor_list_dense_rows(extra):
     box, n_gas = 20.0, 37
     ball = torch.nn.functional.normalize(torch.randn(extra, 3, generator=g), dim=-1) * 2.0 * torch.rand(extra, 1, generator=g) ** (1 / 3)
     pos = torch.cat([ball + 0.5, torch.rand(n_gas, 3, generator=g) * box])      # the ball lies across the corner of the box
-    src, dst, shift, rowptr = e3nn_b200.nn.neighbor_list_pbc(pos.to(DEV), box, 5.0)
+    src, dst, shift, rowptr = bnn.neighbor_list_pbc(pos.to(DEV), box, 5.0)
     p = pos.double() - torch.floor(pos.double() / box) * box
     d = p[None, :, :] - p[:, None, :]
     d = d - box * torch.round(d / box)
@@ -43,3 +45,57 @@ def test_neighbor_list_dense_rows(extra):
     # coordinates of up to 20 in fp32: three roundings of 2^-24 * 20
     assert (vec.cpu().double() - d[ref_dst, ref_src]).abs().max().item() < 4e-6
     assert int(rowptr[-1]) == src.numel()
+
+
+# ----------------------------------------------------------------------------- fp32 contractions on register tiles
+TILE_LAYOUTS = [
+    ("1x0e+33x1o", "0e+2x1o", "17x0e+3x1o+16x1e"),                 # one channel, a chunk of 32 + 1, two second-operand channels
+    ("65x0e+5x1o+2x2e", "1x0e+1x1o+1x2e", "130x0e+64x1o+1x2e"),    # column blocks of 128 + 2, one output channel
+    ("4x3o+7x2e", "3o+2e+1o", "9x0e+33x3o+2x1o"),                  # l = 3 throughout
+    ("3x4e+2x0e", "2x1o+4e", "5x4e+2x0e+3x3o"),                    # l = 4: staged without the unrolled irreps, derived products backward
+    ("8x0e+8x1o", "5x0e", "8x0e+8x1o+4x2e"),                       # scalar second operand, an output no path writes
+]
+
+
+@pytest.mark.parametrize("rows", [1, 31, 129, 1000])
+@pytest.mark.parametrize("layout", TILE_LAYOUTS)
+def test_fp32_product_tiles(layout, rows):
+    """Forward and all gradients; bound: 1e-5 x RMS, the fp32 parity bound of this path."""
+    g = torch.Generator().manual_seed(rows)
+    tp = o3.FullyConnectedTensorProduct(*layout)
+    x = torch.randn(rows, tp.irreps_in1.dim, generator=g)
+    y = torch.randn(rows, tp.irreps_in2.dim, generator=g)
+    go = torch.randn(rows, tp.irreps_out.dim, generator=g)
+    ins = [(i.i_in1, i.i_in2, i.i_out, i.connection_mode, i.has_weight) for i in tp.instructions]
+    x64, y64, w64 = (t.detach().double().requires_grad_(True) for t in (x, y, tp.weight))
+    ref = orc.tensor_product(*(str(i) for i in (tp.irreps_in1, tp.irreps_in2, tp.irreps_out)), ins, x64, y64, w64, True)
+    ref_g = torch.autograd.grad(ref, [x64, y64, w64], go.double())
+    tp = tp.to(DEV)
+    xd, yd = x.to(DEV).requires_grad_(True), y.to(DEV).requires_grad_(True)
+    out = tp(xd, yd)
+    got_g = torch.autograd.grad(out, [xd, yd, tp.weight], go.to(DEV))
+    assert rel_err(out.detach().cpu(), ref.detach()) < 1e-5
+    for got, want in zip(got_g, ref_g):
+        assert rel_err(got.cpu(), want) < 1e-5
+    # each operand gradient on its own takes another instance of the kernel
+    for n, leaf in enumerate((xd, yd)):
+        other = tp(xd if n == 0 else xd.detach(), yd if n == 1 else yd.detach(), tp.weight.detach())
+        assert rel_err(torch.autograd.grad(other, leaf, go.to(DEV))[0].cpu(), ref_g[n]) < 1e-5
+
+
+@pytest.mark.parametrize("rows", [1, 257])
+@pytest.mark.parametrize("irreps", [("1x0e+40x1o+3x2e", "200x0e+2x0e+17x1o"), ("70x0e+9x4e", "9x4e+16x0e+5x1o"), ("64x0e+64x3o", "32x0e+64x3o")])
+def test_fp32_linear_tiles(irreps, rows):
+    """Forward, transposed (two outputs of different width from one input, an input nothing reads) and weight gradient."""
+    g = torch.Generator().manual_seed(rows)
+    lin = o3.Linear(*irreps)
+    x, go = torch.randn(rows, lin.irreps_in.dim, generator=g), torch.randn(rows, lin.irreps_out.dim, generator=g)
+    x64, w64 = x.double().requires_grad_(True), lin.weight.detach().double().requires_grad_(True)
+    ref = orc.linear(irreps[0], irreps[1], x64, w64)
+    ref_g = torch.autograd.grad(ref, [x64, w64], go.double())
+    lin, xd = lin.to(DEV), x.to(DEV).requires_grad_(True)
+    out = lin(xd)
+    got_g = torch.autograd.grad(out, [xd, lin.weight], go.to(DEV))
+    assert rel_err(out.detach().cpu(), ref.detach()) < 1e-5
+    for got, want in zip(got_g, ref_g):
+        assert rel_err(got.cpu(), want) < 1e-5
