@@ -32,18 +32,6 @@ constexpr int kKBlock = 32;                               // summation block of 
 
 struct DenseGroup { int out_off, mul_out, dim3, K, kent_start, w_stride; };
 
-// Gate applied where the contraction's result is still in registers (Linear followed by Gate).  Column c of the
-// contraction's output row is described by tbl[4 c ..] = {kind, destination column, activation, gate slot} and
-// cst[c]: kind 0 = scalar: final[z, dst] = cst * act(v); kind 2 = gate: gates[z, slot] = cst * act(v);
-// kind 1 = gated component: final[z, dst] = v * gates[z, slot] (its gate's launch ran before); kind 3 = unused.
-struct DenseGateEpilogue {
-    const int32_t* tbl;
-    const float* cst;
-    float* gates;       // [rows, n_slots] activated gates
-    float* final_out;   // [rows, dout_final]
-    int n_slots, dout_final;
-};
-
 template <bool VEC4>
 __global__ void __launch_bounds__(kDenseThreads) dense_fwd_kernel(const int32_t* __restrict__ plan,
         const float* __restrict__ x1, const float* __restrict__ x2, const float* __restrict__ W,
@@ -298,6 +286,9 @@ extern "C" int e3b_dense_fwd_gate(const int32_t* plan_host, const int32_t* plan_
         return fail(E3B_ERR_ARG, "dense_fwd_gate: null pointer");
     const DenseGateEpilogue ep{gate_table, gate_const, gates, out, n_slots, dout};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    bool done = false;
+    if (int rc = launch_dense_rows_gate(plan_host, plan_dev, x, weight, ep, num_rows, s, &done)) return rc;
+    if (done) return E3B_OK;
     // scalars and gates first: the launches of the gated irreps read the activated gates of the same rows
     if (int rc = launch_dense_groups(plan_host, plan_dev, x, nullptr, weight, 0, out, num_rows, 0, ep, 1, s)) return rc;
     return launch_dense_groups(plan_host, plan_dev, x, nullptr, weight, 0, out, num_rows, 0, ep, 2, s);

@@ -19,6 +19,7 @@
 //   segments      : word offsets s[0..n] of (index, coefficient) pairs: (j, C) per (k, i); (i * d3 + k, C) per j
 #include "common.cuh"
 #include "dense_plan.cuh"
+#include "gate_act.cuh"
 
 namespace e3b {
 namespace {
@@ -137,7 +138,7 @@ __device__ __forceinline__ void stage_weights(const float* __restrict__ W, int s
     }
 }
 
-// ---------------------------------------------------------------------------------------------- forward
+// ---------------------------------------------------------------------------------------------- forward, any irrep
 struct FwdLaunch {
     int n;                               // groups of this launch
     int first_block[kMaxGroups + 1];
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(kThreads) dense_tile_fwd_kernel(const int32_t*
 // Columns of a tile: the narrowest that holds the group's channels in one pass, so that the coupled operand is built once.
 inline int columns_for(int mo) { return mo <= 16 ? 16 : mo <= 32 ? 32 : mo <= 64 ? 64 : 128; }
 
-// ---------------------------------------------------------------------------------------------- weight gradient
+// ---------------------------------------------------------------------------------------------- weight gradient, any irrep
 // grad_W_p[u, v, w] += sum_{z, k} A[z, k, u] grad_out[z, w, k]: a block owns the K entries of up to 128 / 64 / 32 channels
 // (whole chunks) x 32 / 64 / 128 output channels in registers and walks every splits-th tile of 64 (z, k) rows.
 constexpr int kBwRows = 64;
@@ -373,6 +374,535 @@ __global__ void __launch_bounds__(kThreads, 4) dense_tile_bwd_w_kernel(const int
     }
 }
 
+// ---------------------------------------------------------------------------------------------- irreps of l <= 3
+// For output irreps of dimension D3 <= 7 (compile time) operands stay in row order, [z][channel * D + component], the
+// order they have in memory: a thread owns whole rows z, so 4 channels of one row are D3 aligned 16-byte reads, the
+// sum over components needs no transposed copy, rows arrive by cp.async while the chunk before is multiplied, and
+// results leave as 16-byte stores.  (The form above, used for l > 3, transposes every chunk into (z, k) rows with
+// loads that wait for memory one after another: 1.86 ms for the weight gradient of a 6336 -> 1024 Linear on 16,384
+// rows, 13 GFLOP.)
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool live) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(live ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool live) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// dst[z * ld + e] <- src[z * row + e], e < n (zero for n <= e < width and for z >= nz_live), z < BZ; width, ld % 4 == 0.
+template <int BZ>
+__device__ __forceinline__ void fetch_rows(float* dst, int ld, const float* __restrict__ src, int row, int n, int width, int nz_live) {
+    if ((row & 3) == 0 && (n & 3) == 0 && aligned16(src)) {
+        const int q = width >> 2;
+        for (int idx = threadIdx.x; idx < BZ * q; idx += kThreads) {
+            const int z = idx / q, e = (idx - z * q) * 4;
+            const bool live = z < nz_live && e < n;
+            cp_async16(dst + z * ld + e, live ? src + static_cast<int64_t>(z) * row + e : src, live);
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < BZ * width; idx += kThreads) {
+            const int z = idx / width, e = idx - z * width;
+            const bool live = z < nz_live && e < n;
+            cp_async4(dst + z * ld + e, live ? src + static_cast<int64_t>(z) * row + e : src, live);
+        }
+    }
+}
+
+// dst[kk * ld + n] <- W[kk * su + n * sw], kk < 32, n < BN, zero outside len x cols.
+template <int BN>
+__device__ __forceinline__ void fetch_weights(float* dst, int ld, const float* __restrict__ W, int su, int sw, int len, int cols) {
+    if (sw == 1 && (su & 3) == 0 && (cols & 3) == 0 && aligned16(W)) {
+        for (int idx = threadIdx.x; idx < kKC * BN / 4; idx += kThreads) {
+            const int kk = idx / (BN / 4), n = (idx % (BN / 4)) * 4;
+            const bool live = kk < len && n < cols;
+            cp_async16(dst + kk * ld + n, live ? W + static_cast<int64_t>(kk) * su + n : W, live);
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < kKC * BN; idx += kThreads) {
+            const int kk = sw == 1 ? idx / BN : idx % kKC, n = sw == 1 ? idx % BN : idx / kKC;
+            const bool live = kk < len && n < cols;
+            cp_async4(dst + kk * ld + n, live ? W + static_cast<int64_t>(kk) * su + static_cast<int64_t>(n) * sw : W, live);
+        }
+    }
+}
+
+// T[z][k * d1 + i] of BZ rows from the second operand's rows in shared memory.
+template <int BZ>
+__device__ __forceinline__ void couple_rows(const int32_t* plan, const int32_t* path, const float* sY, int ldy, int x2off, float* sT, int ldt) {
+    const int n = path[0] * path[2];
+    const int32_t* seg = plan + path[5];
+    for (int idx = threadIdx.x; idx < BZ * n; idx += kThreads) {
+        const int z = idx / n, ki = idx - z * n;
+        const float* y = sY + z * ldy + x2off;
+        float t = 0.0f;
+        for (int s = seg[ki]; s < seg[ki + 1]; s += 2) t = fmaf(__int_as_float(plan[s + 1]), y[plan[s]], t);
+        sT[z * ldt + ki] = t;
+    }
+}
+
+// A[z][u * D3 + k] = sum_i T[z][k * D1 + i] X[z][u * D1 + i], u < 32.
+template <int D3, int D1, int BZ>
+__device__ __forceinline__ void build_rows_d(const float* sX, int ldx, const float* sT, int ldt, float* sA, int lda) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int z = warp; z < BZ; z += kThreads / 32) {
+        float x[D1];
+#pragma unroll
+        for (int i = 0; i < D1; ++i) x[i] = sX[z * ldx + lane * D1 + i];
+        const float* t = sT + z * ldt;
+#pragma unroll
+        for (int k = 0; k < D3; ++k) {
+            float v = 0.0f;
+#pragma unroll
+            for (int i = 0; i < D1; ++i) v = fmaf(t[k * D1 + i], x[i], v);
+            sA[z * lda + lane * D3 + k] = v;
+        }
+    }
+}
+
+template <int D3, int BZ>
+__device__ __forceinline__ void build_rows(int d1, const float* sX, int ldx, const float* sT, int ldt, float* sA, int lda) {
+    switch (d1) {
+        case 1: build_rows_d<D3, 1, BZ>(sX, ldx, sT, ldt, sA, lda); break;
+        case 3: build_rows_d<D3, 3, BZ>(sX, ldx, sT, ldt, sA, lda); break;
+        case 5: build_rows_d<D3, 5, BZ>(sX, ldx, sT, ldt, sA, lda); break;
+        default: build_rows_d<D3, 7, BZ>(sX, ldx, sT, ldt, sA, lda); break;
+    }
+}
+
+// Rows of a forward tile.  TX threads share a row (8 channels each); a thread owns rows_per_thread rows.
+template <int D3, int TX, bool COUPLED>
+__host__ __device__ constexpr int rows_per_thread() {
+    // uncoupled: up to 56 accumulators; coupled: at most 32 rows a block, so that the chunk of the first operand and the
+    // coupled chunk (32 x 7 floats a row each) leave room for several blocks on an SM
+    return COUPLED ? (D3 == 1 ? TX / 4 : D3 == 3 ? (TX >= 8 ? 2 : 1) : 1) : (D3 == 1 ? 4 : D3 == 3 ? 2 : 1);
+}
+
+__host__ __device__ constexpr int pad_row(int floats) { return floats + 4; }      // rows 4 banks apart
+
+template <int D3, int TX, bool COUPLED>
+constexpr int fwd_rows() { return kThreads / TX * rows_per_thread<D3, TX, COUPLED>(); }
+
+// Shared floats of a forward tile: two row buffers, two weight buffers, coupling, second operand.
+template <int D3, int TX, bool COUPLED>
+inline size_t fwd_floats(int d1max, int d2row) {
+    constexpr int BZ = fwd_rows<D3, TX, COUPLED>();
+    const size_t w = 2 * kKC * (8 * TX + 4);
+    if (!COUPLED) return w + 2 * static_cast<size_t>(BZ) * pad_row(32 * D3);
+    return w + static_cast<size_t>(BZ) * (pad_row(32 * d1max) + pad_row(32 * D3) + (d1max * D3 | 1) + (d2row | 1));
+}
+
+template <int D3, int TX, bool COUPLED, bool GATE>
+__device__ __forceinline__ void fwd_rows_tile(const Part2& P, const int32_t* g, const float* __restrict__ x1, const float* __restrict__ x2,
+                                              const float* __restrict__ W, float* __restrict__ out, int64_t Z, int tile, int accumulate,
+                                              const DenseGateEpilogue& ep, float* smem) {
+    constexpr int ZPT = rows_per_thread<D3, TX, COUPLED>(), TZ = kThreads / TX, BZ = TZ * ZPT, BN = 8 * TX, ldw = BN + 4;
+    const int out_off = g[0], mo = g[1], nch = g[4], d1row = P.plan[1], d2row = P.plan[2], dout = P.plan[3];
+    const int col_blocks = (mo + BN - 1) / BN;
+    const int64_t z0 = static_cast<int64_t>(tile / col_blocks) * BZ;
+    const int live = static_cast<int>(min(static_cast<int64_t>(BZ), Z - z0));
+    const int c0 = (tile % col_blocks) * BN, cols = min(BN, mo - c0);
+    const int ldx = pad_row(32 * (COUPLED ? P.d1max() : D3)), ldy = d2row | 1;
+    constexpr int lda = pad_row(32 * D3);
+    float* sW = smem;                                        // [2][32][ldw]
+    float* sX = smem + 2 * kKC * ldw;                        // coupled: one chunk of x1; uncoupled: [2] chunks
+    float* sA = sX + BZ * ldx;                               // coupled operand
+    float* sT = sA + BZ * lda;
+    float* sY = sT + (COUPLED ? BZ * (P.d1max() * D3 | 1) : 0);
+    const int tid = threadIdx.x, tx = tid % TX, tz = tid / TX;
+
+    auto fetch = [&](int c) {
+        const int32_t* ch = P.chunk(g[3] + c);
+        const int32_t* path = P.path(ch[0]);
+        const int d1 = COUPLED ? path[0] : D3;
+        fetch_rows<BZ>(sX + (COUPLED ? 0 : (c & 1) * BZ * ldx), ldx, x1 + z0 * d1row + ch[1], d1row, ch[2] * d1, 32 * d1, live);
+        fetch_weights<BN>(sW + (c & 1) * kKC * ldw, ldw, W + ch[4] + static_cast<int64_t>(c0) * path[4], path[3], path[4], ch[2], cols);
+        cp_async_commit();
+    };
+
+    float acc[ZPT][D3][8];
+#pragma unroll
+    for (int p = 0; p < ZPT; ++p)
+#pragma unroll
+        for (int k = 0; k < D3; ++k)
+#pragma unroll
+            for (int n = 0; n < 8; ++n) acc[p][k][n] = 0.0f;
+
+    if (COUPLED)
+        for (int idx = tid; idx < BZ * d2row; idx += kThreads) {
+            const int z = idx / d2row, e = idx - z * d2row;
+            cp_async4(sY + z * ldy + e, z < live ? x2 + (z0 + z) * d2row + e : x2, z < live);
+        }
+    fetch(0);
+    for (int c = 0; c < nch; ++c) {
+        const int32_t* ch = P.chunk(g[3] + c);
+        const int32_t* path = P.path(ch[0]);
+        const float* A = sX + (c & 1) * BZ * ldx;
+        float coef = 1.0f;
+        if (COUPLED) {
+            const int d1 = path[0], ldt = (d1 * D3) | 1;
+            cp_async_wait<0>();
+            __syncthreads();          // this chunk is there; everyone is done with the previous coupled operand
+            if (ch[5]) {
+                couple_rows<BZ>(P.plan, path, sY, ldy, ch[3], sT, ldt);
+                __syncthreads();
+            }
+            build_rows<D3, BZ>(d1, sX, ldx, sT, ldt, sA, lda);
+            __syncthreads();
+            if (c + 1 < nch) fetch(c + 1);
+            A = sA;
+        } else {
+            coef = __int_as_float(path[15]);
+            if (c + 1 < nch) { fetch(c + 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
+            __syncthreads();
+        }
+        const float* w = sW + (c & 1) * kKC * ldw;
+        // the chunk's sum in accumulators of its own: the rounding error grows with sqrt(32) + sqrt(K / 32)
+        float part[ZPT][D3][8];
+#pragma unroll
+        for (int p = 0; p < ZPT; ++p)
+#pragma unroll
+            for (int k = 0; k < D3; ++k)
+#pragma unroll
+                for (int n = 0; n < 8; ++n) part[p][k][n] = 0.0f;
+        const int uend = (ch[2] + 3) & ~3;
+#pragma unroll 1
+        for (int u = 0; u < uend; u += 4) {
+            float wv[4][8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 lo = *reinterpret_cast<const float4*>(w + (u + q) * ldw + tx * 4);
+                const float4 hi = *reinterpret_cast<const float4*>(w + (u + q) * ldw + BN / 2 + tx * 4);
+                wv[q][0] = lo.x; wv[q][1] = lo.y; wv[q][2] = lo.z; wv[q][3] = lo.w;
+                wv[q][4] = hi.x; wv[q][5] = hi.y; wv[q][6] = hi.z; wv[q][7] = hi.w;
+            }
+#pragma unroll
+            for (int p = 0; p < ZPT; ++p) {
+                float a[4 * D3];
+#pragma unroll
+                for (int e = 0; e < D3; ++e) {
+                    const float4 t = *reinterpret_cast<const float4*>(A + (tz + TZ * p) * (COUPLED ? lda : ldx) + u * D3 + 4 * e);
+                    a[4 * e] = t.x; a[4 * e + 1] = t.y; a[4 * e + 2] = t.z; a[4 * e + 3] = t.w;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int k = 0; k < D3; ++k)
+#pragma unroll
+                        for (int n = 0; n < 8; ++n) part[p][k][n] = fmaf(a[q * D3 + k], wv[q][n], part[p][k][n]);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < ZPT; ++p)
+#pragma unroll
+            for (int k = 0; k < D3; ++k)
+#pragma unroll
+                for (int n = 0; n < 8; ++n) acc[p][k][n] = fmaf(coef, part[p][k][n], acc[p][k][n]);
+        if (!COUPLED) __syncthreads();          // the buffers are fetched into again
+    }
+    const bool vec = (dout & 3) == 0 && (cols & 3) == 0 && aligned16(out + out_off + c0 * D3) && !accumulate;
+#pragma unroll
+    for (int p = 0; p < ZPT; ++p) {
+        const int z = tz + TZ * p;
+        if (z >= live) continue;
+        float* o = out + (z0 + z) * dout + out_off + c0 * D3;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int n0 = h * (BN / 2) + tx * 4;
+            if (n0 >= cols) continue;
+            if (GATE) {
+                // one table entry per channel (its components are consecutive columns and share the gate)
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    if (n0 + n >= cols) continue;
+                    const int col = out_off + (c0 + n0 + n) * D3;
+                    const int4 e = __ldg(reinterpret_cast<const int4*>(ep.tbl) + col);      // kind, destination, activation, gate slot
+                    if (e.x == 1) {
+                        const float gate = ep.gates[(z0 + z) * ep.n_slots + e.w];
+#pragma unroll
+                        for (int k = 0; k < D3; ++k) ep.final_out[(z0 + z) * ep.dout_final + e.y + k] = acc[p][k][4 * h + n] * gate;
+                    } else if (e.x == 0 || e.x == 2) {
+                        const float v = ep.cst[col] * gate_act(e.z, acc[p][0][4 * h + n]);
+                        if (e.x == 0) ep.final_out[(z0 + z) * ep.dout_final + e.y] = v;
+                        else ep.gates[(z0 + z) * ep.n_slots + e.w] = v;
+                    }
+                }
+            } else if (vec) {
+#pragma unroll
+                for (int e = 0; e < D3; ++e) {
+                    // element 4 e + r of the 4 channels' run is channel (4 e + r) / D3, component (4 e + r) % D3
+                    float4 t;
+                    t.x = acc[p][(4 * e) % D3][4 * h + (4 * e) / D3];
+                    t.y = acc[p][(4 * e + 1) % D3][4 * h + (4 * e + 1) / D3];
+                    t.z = acc[p][(4 * e + 2) % D3][4 * h + (4 * e + 2) / D3];
+                    t.w = acc[p][(4 * e + 3) % D3][4 * h + (4 * e + 3) / D3];
+                    *reinterpret_cast<float4*>(o + n0 * D3 + 4 * e) = t;
+                }
+            } else {
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    if (n0 + n >= cols) continue;
+#pragma unroll
+                    for (int k = 0; k < D3; ++k) {
+                        float* q = o + (n0 + n) * D3 + k;
+                        *q = accumulate ? *q + acc[p][k][4 * h + n] : acc[p][k][4 * h + n];
+                    }
+                }
+            }
+        }
+    }
+}
+
+struct FwdShape { int rows; size_t floats; };
+
+template <int D3, bool COUPLED>
+inline FwdShape fwd_shape_tx(int tx, int d1max, int d2row) {
+    if (tx == 4) return {fwd_rows<D3, 4, COUPLED>(), fwd_floats<D3, 4, COUPLED>(d1max, d2row)};
+    if (tx == 8) return {fwd_rows<D3, 8, COUPLED>(), fwd_floats<D3, 8, COUPLED>(d1max, d2row)};
+    return {fwd_rows<D3, 16, COUPLED>(), fwd_floats<D3, 16, COUPLED>(d1max, d2row)};
+}
+
+template <bool COUPLED>
+inline FwdShape fwd_shape(int d3, int tx, int d1max, int d2row) {
+    switch (d3) {
+        case 1: return fwd_shape_tx<1, COUPLED>(tx, d1max, d2row);
+        case 3: return fwd_shape_tx<3, COUPLED>(tx, d1max, d2row);
+        case 5: return fwd_shape_tx<5, COUPLED>(tx, d1max, d2row);
+        default: return fwd_shape_tx<7, COUPLED>(tx, d1max, d2row);
+    }
+}
+
+template <int D3, bool COUPLED, bool GATE>
+__device__ __forceinline__ void fwd_rows_tx(int tx, const Part2& P, const int32_t* g, const float* __restrict__ x1, const float* __restrict__ x2,
+                                            const float* __restrict__ W, float* __restrict__ out, int64_t Z, int tile, int accumulate,
+                                            const DenseGateEpilogue& ep, float* smem) {
+    if (tx == 4) fwd_rows_tile<D3, 4, COUPLED, GATE>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
+    else if (tx == 8) fwd_rows_tile<D3, 8, COUPLED, GATE>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
+    else fwd_rows_tile<D3, 16, COUPLED, GATE>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
+}
+
+struct RowsLaunch {
+    int n;                               // groups of this launch
+    int first_block[kMaxGroups + 1];
+    int splits[kMaxGroups];              // (weight gradient)
+    int16_t group[kMaxGroups];
+    int16_t shape[kMaxGroups];           // forward: threads a row; weight gradient: output channels of a block
+};
+
+template <bool COUPLED, bool GATE>
+__global__ void __launch_bounds__(kThreads, 3) dense_rows_fwd_kernel(const int32_t* __restrict__ plan, const float* __restrict__ x1,
+                                                                     const float* __restrict__ x2, const float* __restrict__ W,
+                                                                     float* __restrict__ out, int64_t Z, int accumulate, RowsLaunch L,
+                                                                     DenseGateEpilogue ep) {
+    extern __shared__ __align__(16) float smem[];
+    const Part2 P(plan);
+    int s = 0;
+    while (s + 1 < L.n && static_cast<int>(blockIdx.x) >= L.first_block[s + 1]) ++s;
+    const int32_t* g = P.group(L.group[s]);
+    const int tile = static_cast<int>(blockIdx.x) - L.first_block[s];
+    switch (g[2]) {
+        case 1: fwd_rows_tx<1, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+        case 3: fwd_rows_tx<3, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+        case 5: fwd_rows_tx<5, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+        default: fwd_rows_tx<7, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+    }
+}
+
+// ---- weight gradient: 4096 = KB x BW entries of one group in registers (8 x 4 a thread), rows streamed
+template <int D3, bool COUPLED>
+__host__ __device__ constexpr int wgrad_rows() { return COUPLED ? 8 : D3 == 1 ? 32 : D3 == 3 ? 16 : 8; }
+
+template <int D3, int BW, bool COUPLED>
+inline size_t wgrad_floats(int d1max, int d2row) {
+    constexpr int KB = 4096 / BW, BZ = wgrad_rows<D3, COUPLED>(), NCH = KB / kKC;
+    const size_t gbuf = 2 * static_cast<size_t>(BZ) * pad_row(BW * D3);
+    if (!COUPLED) return gbuf + 2 * static_cast<size_t>(BZ) * pad_row(KB * D3);
+    return gbuf + static_cast<size_t>(BZ) * (pad_row(KB * d1max) + pad_row(KB * D3) + NCH * (d1max * D3 | 1) + 2 * (d2row | 1));
+}
+
+template <int D3, int BW, bool COUPLED>
+__device__ __forceinline__ void wgrad_block(const Part2& P, const int32_t* g, const float* __restrict__ x1, const float* __restrict__ x2,
+                                            const float* __restrict__ gout, float* __restrict__ grad_w, int64_t Z, int block, int splits,
+                                            float* smem) {
+    constexpr int KB = 4096 / BW, NCH = KB / kKC, BZ = wgrad_rows<D3, COUPLED>(), ldg = pad_row(BW * D3), lda = pad_row(KB * D3);
+    constexpr int CX = BW / kTN, WC = CX / 8;
+    const int out_off = g[0], mo = g[1], d1row = P.plan[1], d2row = P.plan[2], dout = P.plan[3];
+    const int kblocks = (g[4] + NCH - 1) / NCH, wblocks = (mo + BW - 1) / BW;
+    const int split = block / (kblocks * wblocks), rest = block % (kblocks * wblocks);
+    const int ch0 = (rest / wblocks) * NCH, nch = min(NCH, g[4] - ch0);
+    const int w0 = (rest % wblocks) * BW, cols = min(BW, mo - w0);
+    const int d1max = P.d1max(), ldx = COUPLED ? pad_row(KB * d1max) : lda, ldy = d2row | 1, ldt = COUPLED ? (d1max * D3 | 1) : 0;
+    float* sG = smem;                                   // [2][BZ][ldg]
+    float* sX = smem + 2 * BZ * ldg;                    // uncoupled: [2][BZ][lda]; coupled: one set of x1 chunks
+    float* sA = sX + BZ * ldx;
+    float* sT = sA + BZ * lda;                          // [NCH][BZ][ldt]
+    float* sY = sT + NCH * BZ * ldt;                    // [2][BZ][ldy]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = (warp % WC) * 8 + (lane & 7), ty = (warp / WC) * 4 + (lane >> 3);
+
+    auto fetch = [&](int64_t tile, int buf) {
+        const int64_t z0 = tile * BZ;
+        const int live = static_cast<int>(min(static_cast<int64_t>(BZ), Z - z0));
+        int col = 0;
+        for (int c = 0; c < nch; ++c) {
+            const int32_t* ch = P.chunk(g[3] + ch0 + c);
+            const int d1 = COUPLED ? P.path(ch[0])[0] : D3;
+            fetch_rows<BZ>(sX + (COUPLED ? 0 : buf * BZ * lda) + col, ldx, x1 + z0 * d1row + ch[1], d1row, ch[2] * d1, 32 * d1, live);
+            col += 32 * d1;
+        }
+        fetch_rows<BZ>(sG + buf * BZ * ldg, ldg, gout + z0 * dout + out_off + w0 * D3, dout, cols * D3, BW * D3, live);
+        if (COUPLED)
+            for (int idx = tid; idx < BZ * d2row; idx += kThreads) {
+                const int z = idx / d2row, e = idx - z * d2row;
+                cp_async4(sY + (buf * BZ + z) * ldy + e, z < live ? x2 + (z0 + z) * d2row + e : x2, z < live);
+            }
+        cp_async_commit();
+    };
+
+    float acc[kTM][kTN];
+#pragma unroll
+    for (int i = 0; i < kTM; ++i)
+#pragma unroll
+        for (int j = 0; j < kTN; ++j) acc[i][j] = 0.0f;
+
+    const int64_t tiles = (Z + BZ - 1) / BZ;
+    int buf = 0;
+    if (split < tiles) fetch(split, 0);
+    for (int64_t tile = split; tile < tiles; tile += splits, buf ^= 1) {
+        const bool more = tile + splits < tiles;
+        const float* A = sX + buf * BZ * lda;
+        if (COUPLED) {
+            cp_async_wait<0>();
+            __syncthreads();
+            for (int c = 0; c < nch; ++c) {
+                const int32_t* ch = P.chunk(g[3] + ch0 + c);
+                if (ch[5] || c == 0) {
+                    const int32_t* path = P.path(ch[0]);
+                    couple_rows<BZ>(P.plan, path, sY + buf * BZ * ldy, ldy, ch[3], sT + c * BZ * ldt, (path[0] * D3) | 1);
+                }
+            }
+            __syncthreads();
+            int col = 0, tc = 0;
+            for (int c = 0; c < nch; ++c) {
+                const int32_t* ch = P.chunk(g[3] + ch0 + c);
+                const int d1 = P.path(ch[0])[0];
+                if (ch[5] || c == 0) tc = c;
+                build_rows<D3, BZ>(d1, sX + col, ldx, sT + tc * BZ * ldt, (d1 * D3) | 1, sA + c * kKC * D3, lda);
+                col += 32 * d1;
+            }
+            __syncthreads();
+            if (more) fetch(tile + splits, buf ^ 1);
+            A = sA;
+        } else {
+            if (more) { fetch(tile + splits, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
+            __syncthreads();
+        }
+        const float* G = sG + buf * BZ * ldg;
+        if (ty * kTM < nch * kKC) {
+            float part[kTM][kTN];
+#pragma unroll
+            for (int i = 0; i < kTM; ++i)
+#pragma unroll
+                for (int j = 0; j < kTN; ++j) part[i][j] = 0.0f;
+#pragma unroll 1
+            for (int z = 0; z < BZ; ++z) {
+                float b[kTN * D3];
+#pragma unroll
+                for (int e = 0; e < D3; ++e) {
+                    const float4 t = *reinterpret_cast<const float4*>(G + z * ldg + tx * kTN * D3 + 4 * e);
+                    b[4 * e] = t.x; b[4 * e + 1] = t.y; b[4 * e + 2] = t.z; b[4 * e + 3] = t.w;
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float a[4 * D3];
+#pragma unroll
+                    for (int e = 0; e < D3; ++e) {
+                        const float4 t = *reinterpret_cast<const float4*>(A + z * lda + (ty * kTM + 4 * h) * D3 + 4 * e);
+                        a[4 * e] = t.x; a[4 * e + 1] = t.y; a[4 * e + 2] = t.z; a[4 * e + 3] = t.w;
+                    }
+#pragma unroll
+                    for (int k = 0; k < D3; ++k)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int j = 0; j < kTN; ++j) part[4 * h + i][j] = fmaf(a[i * D3 + k], b[j * D3 + k], part[4 * h + i][j]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kTM; ++i)
+#pragma unroll
+                for (int j = 0; j < kTN; ++j) acc[i][j] += part[i][j];
+        }
+        if (!COUPLED) __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < kTM; ++i) {
+        const int kk = ty * kTM + i, c = kk / kKC, u = kk - c * kKC;
+        if (c >= nch) continue;
+        const int32_t* ch = P.chunk(g[3] + ch0 + c);
+        if (u >= ch[2]) continue;
+        const int32_t* path = P.path(ch[0]);
+        const float coef = COUPLED ? 1.0f : __int_as_float(path[15]);
+        const int sw = path[4], n0 = tx * kTN;
+        float* p = grad_w + ch[4] + static_cast<int64_t>(u) * path[3] + static_cast<int64_t>(w0 + n0) * sw;
+        if (sw == 1 && n0 + kTN <= cols && aligned16(p)) {
+            atomicAdd(reinterpret_cast<float4*>(p), make_float4(coef * acc[i][0], coef * acc[i][1], coef * acc[i][2], coef * acc[i][3]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < kTN; ++j)
+                if (n0 + j < cols) atomicAdd(p + static_cast<int64_t>(j) * sw, coef * acc[i][j]);
+        }
+    }
+}
+
+template <int D3, bool COUPLED>
+inline size_t wgrad_floats_bw(int bw, int d1max, int d2row) {
+    return bw == 32 ? wgrad_floats<D3, 32, COUPLED>(d1max, d2row) : bw == 64 ? wgrad_floats<D3, 64, COUPLED>(d1max, d2row)
+                                                                             : wgrad_floats<D3, 128, COUPLED>(d1max, d2row);
+}
+
+template <bool COUPLED>
+inline FwdShape wgrad_shape(int d3, int bw, int d1max, int d2row) {
+    switch (d3) {
+        case 1: return {wgrad_rows<1, COUPLED>(), wgrad_floats_bw<1, COUPLED>(bw, d1max, d2row)};
+        case 3: return {wgrad_rows<3, COUPLED>(), wgrad_floats_bw<3, COUPLED>(bw, d1max, d2row)};
+        case 5: return {wgrad_rows<5, COUPLED>(), wgrad_floats_bw<5, COUPLED>(bw, d1max, d2row)};
+        default: return {wgrad_rows<7, COUPLED>(), wgrad_floats_bw<7, COUPLED>(bw, d1max, d2row)};
+    }
+}
+
+template <int D3, bool COUPLED>
+__device__ __forceinline__ void wgrad_bw(int bw, const Part2& P, const int32_t* g, const float* __restrict__ x1, const float* __restrict__ x2,
+                                         const float* __restrict__ gout, float* __restrict__ grad_w, int64_t Z, int block, int splits,
+                                         float* smem) {
+    if (bw == 32) wgrad_block<D3, 32, COUPLED>(P, g, x1, x2, gout, grad_w, Z, block, splits, smem);
+    else if (bw == 64) wgrad_block<D3, 64, COUPLED>(P, g, x1, x2, gout, grad_w, Z, block, splits, smem);
+    else wgrad_block<D3, 128, COUPLED>(P, g, x1, x2, gout, grad_w, Z, block, splits, smem);
+}
+
+template <bool COUPLED>
+__global__ void __launch_bounds__(kThreads, 4) dense_rows_wgrad_kernel(const int32_t* __restrict__ plan, const float* __restrict__ x1,
+                                                                       const float* __restrict__ x2, const float* __restrict__ gout,
+                                                                       float* __restrict__ grad_w, int64_t Z, RowsLaunch L) {
+    extern __shared__ __align__(16) float smem[];
+    const Part2 P(plan);
+    int s = 0;
+    while (s + 1 < L.n && static_cast<int>(blockIdx.x) >= L.first_block[s + 1]) ++s;
+    const int32_t* g = P.group(L.group[s]);
+    const int block = static_cast<int>(blockIdx.x) - L.first_block[s];
+    switch (g[2]) {
+        case 1: wgrad_bw<1, COUPLED>(L.shape[s], P, g, x1, x2, gout, grad_w, Z, block, L.splits[s], smem); break;
+        case 3: wgrad_bw<3, COUPLED>(L.shape[s], P, g, x1, x2, gout, grad_w, Z, block, L.splits[s], smem); break;
+        case 5: wgrad_bw<5, COUPLED>(L.shape[s], P, g, x1, x2, gout, grad_w, Z, block, L.splits[s], smem); break;
+        default: wgrad_bw<7, COUPLED>(L.shape[s], P, g, x1, x2, gout, grad_w, Z, block, L.splits[s], smem); break;
+    }
+}
+
 // ---------------------------------------------------------------------------------------------- operand gradients
 // Both operand gradients of a 'uvw' product come from one intermediate per path:
 //     Q[z, u, k]       = sum_w W_p[u, v, w] g[z, w, k]
@@ -389,108 +919,128 @@ struct BwdXLaunch {
 };
 
 struct BwdXShared {
-    float *a, *w, *x, *t, *m, *g2;
-    int ldx, ldt, ldm, ld2;
+    float *g, *w, *t, *m, *g2;      // g: [2] cotangent chunks, w: [2] weight chunks [channel of w][channel of u]
+    int ldt, ldm, ld2, g_floats;    // g_floats: one cotangent buffer
 };
 
+// The walk over (path, second-operand channel, chunk of 32 output channels); the next step is fetched while one is used.
+struct BwdXStep {
+    int n, v, c0;
+    const int32_t* path;
+};
+
+__device__ __forceinline__ bool bwd_x_next(const Part2& P, const int32_t* in, BwdXStep& s) {
+    s.c0 += kKC;
+    if (s.c0 < s.path[12]) return true;
+    s.c0 = 0;
+    if (++s.v < s.path[10]) return true;
+    s.v = 0;
+    if (++s.n >= in[4]) return false;
+    s.path = P.path(P.in_path(in[3] + s.n));
+    return true;
+}
+
+__device__ __forceinline__ void bwd_x_fetch(const Part2& P, const BwdXStep& s, const float* __restrict__ W, const float* __restrict__ gout,
+                                            int64_t z0, int live, int u0, int nu, const BwdXShared& S, int buf) {
+    const int d3 = s.path[2], su = s.path[3], sw = s.path[4], len = min(kKC, s.path[12] - s.c0), dout = P.plan[3];
+    fetch_rows<kBxZ>(S.g + buf * S.g_floats, pad_row(32 * d3), gout + z0 * dout + s.path[11] + s.c0 * d3, dout, len * d3, 32 * d3, live);
+    const float* w = W + s.path[13] + static_cast<int64_t>(u0) * su + static_cast<int64_t>(s.v) * s.path[14] + static_cast<int64_t>(s.c0) * sw;
+    float* dst = S.w + buf * kKC * kLda;
+    for (int idx = threadIdx.x; idx < kKC * 32; idx += kThreads) {
+        const int ww = idx & 31, u = idx >> 5;
+        const bool ok = ww < len && u < nu;
+        cp_async4(dst + ww * kLda + u, ok ? w + static_cast<int64_t>(u) * su + static_cast<int64_t>(ww) * sw : W, ok);
+    }
+    cp_async_commit();
+}
+
+// One step: the chunk's share of Q and, at once, what it adds to both gradients (both are linear in Q, and a chunk's sum
+// of 32 terms is then the only long chain of additions).
 template <int D1, int D3, bool NEED1, bool NEED2>
-__device__ __forceinline__ void bwd_x_path(const Part2& P, const int32_t* path, const float* __restrict__ x2, const float* __restrict__ W,
-                                           const float* __restrict__ gout, int64_t z0, int64_t Z, int u0, int nu, const BwdXShared& S,
-                                           float (&gx)[D1][kBxU]) {
-    const int su = path[3], sw = path[4], x2off = path[9], m2 = path[10], out_off = path[11], mo = path[12], wbase = path[13], sv = path[14];
-    const int d2 = path[1], d2row = P.plan[2], dout = P.plan[3];
+__device__ __forceinline__ void bwd_x_step(const Part2& P, const BwdXStep& s, const float* __restrict__ xrow, bool xvec, int nu,
+                                           const BwdXShared& S, int buf, float (&gx)[D1][kBxU]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = lane & 3, ty = warp * 8 + (lane >> 2);
-    const int ldt = (D1 * D3) | 1;
-    for (int v = 0; v < m2; ++v) {
-        float q[D3][kBxU];
+    constexpr int ldg = pad_row(32 * D3), ldt = (D1 * D3) | 1;
+    const float* G = S.g + buf * S.g_floats + ty * ldg;
+    const float* w = S.w + buf * kKC * kLda + tx * kBxU;
+    float q[D3][kBxU];
+#pragma unroll
+    for (int k = 0; k < D3; ++k)
+#pragma unroll
+        for (int u = 0; u < kBxU; ++u) q[k][u] = 0.0f;
+    const int end = (min(kKC, s.path[12] - s.c0) + 3) & ~3;
+#pragma unroll 1
+    for (int c = 0; c < end; c += 4) {
+        float a[4 * D3];
+#pragma unroll
+        for (int e = 0; e < D3; ++e) {
+            const float4 t = *reinterpret_cast<const float4*>(G + c * D3 + 4 * e);
+            a[4 * e] = t.x; a[4 * e + 1] = t.y; a[4 * e + 2] = t.z; a[4 * e + 3] = t.w;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float4 lo = *reinterpret_cast<const float4*>(w + (c + r) * kLda);
+            const float4 hi = *reinterpret_cast<const float4*>(w + (c + r) * kLda + 4);
+            const float wv[kBxU] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+            for (int k = 0; k < D3; ++k)
+#pragma unroll
+                for (int u = 0; u < kBxU; ++u) q[k][u] = fmaf(a[r * D3 + k], wv[u], q[k][u]);
+        }
+    }
+    if (NEED1) {
 #pragma unroll
         for (int k = 0; k < D3; ++k)
 #pragma unroll
-            for (int u = 0; u < kBxU; ++u) q[k][u] = 0.0f;
-        for (int c0 = 0; c0 < mo; c0 += kKC) {
-            const int len = min(kKC, mo - c0);
-            __syncthreads();
-            if (NEED1 && c0 == 0) stage_coupling(P.plan, path, x2, d2row, x2off + v * d2, z0, kBxZ, Z, S.t, ldt);
-            // W[w][u]
-            for (int idx = tid; idx < kKC * 32; idx += kThreads) {
-                const int ww = idx & 31, u = idx >> 5;
-                S.w[ww * kLda + u] = (ww < len && u < nu) ? __ldg(W + wbase + static_cast<int64_t>(u0 + u) * su + static_cast<int64_t>(v) * sv
-                                                                  + static_cast<int64_t>(c0 + ww) * sw) : 0.0f;
-            }
-            if (v == 0 || mo > kKC) stage_rows_d<D3>(gout, dout, out_off + c0 * D3, len, z0, kBxZ, Z, D3, false, 1.0f, nullptr, 0, S.a, kLda);
-            __syncthreads();
-            float part[D3][kBxU];
-#pragma unroll
-            for (int k = 0; k < D3; ++k)
-#pragma unroll
-                for (int u = 0; u < kBxU; ++u) part[k][u] = 0.0f;
-            const int kend = (len + 3) & ~3;
-#pragma unroll 1
-            for (int kk = 0; kk < kend; kk += 4) {
-                float w[4][kBxU];
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const float4 lo = *reinterpret_cast<const float4*>(S.w + (kk + s) * kLda + tx * kBxU);
-                    const float4 hi = *reinterpret_cast<const float4*>(S.w + (kk + s) * kLda + tx * kBxU + 4);
-                    w[s][0] = lo.x; w[s][1] = lo.y; w[s][2] = lo.z; w[s][3] = lo.w;
-                    w[s][4] = hi.x; w[s][5] = hi.y; w[s][6] = hi.z; w[s][7] = hi.w;
-                }
-#pragma unroll
-                for (int k = 0; k < D3; ++k) {
-                    const float4 a = *reinterpret_cast<const float4*>(S.a + (ty * D3 + k) * kLda + kk);
-                    const float av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-                    for (int s = 0; s < 4; ++s)
-#pragma unroll
-                        for (int u = 0; u < kBxU; ++u) part[k][u] = fmaf(av[s], w[s][u], part[k][u]);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < D3; ++k)
-#pragma unroll
-                for (int u = 0; u < kBxU; ++u) q[k][u] += part[k][u];
-        }
-        if (NEED1) {
-#pragma unroll
-            for (int k = 0; k < D3; ++k)
-#pragma unroll
-                for (int i = 0; i < D1; ++i) {
-                    const float t = S.t[ty * ldt + k * D1 + i];
-#pragma unroll
-                    for (int u = 0; u < kBxU; ++u) gx[i][u] = fmaf(t, q[k][u], gx[i][u]);
-                }
-        }
-        if (NEED2) {
-#pragma unroll
             for (int i = 0; i < D1; ++i) {
-                float m[D3];
+                const float t = S.t[ty * ldt + k * D1 + i];
 #pragma unroll
-                for (int k = 0; k < D3; ++k) m[k] = 0.0f;
+                for (int u = 0; u < kBxU; ++u) gx[i][u] = fmaf(t, q[k][u], gx[i][u]);
+            }
+    }
+    if (NEED2) {
+        float m[D1 * D3];
 #pragma unroll
-                for (int u = 0; u < kBxU; ++u) {
-                    const float x = S.x[ty * S.ldx + (tx * kBxU + u) * D1 + i];
+        for (int e = 0; e < D1 * D3; ++e) m[e] = 0.0f;
 #pragma unroll
-                    for (int k = 0; k < D3; ++k) m[k] = fmaf(x, q[k][u], m[k]);
-                }
+        for (int h = 0; h < 2; ++h) {
+            float x[4 * D1];      // 4 channels of the row (cached: every path reads them again)
 #pragma unroll
-                for (int k = 0; k < D3; ++k) {
-                    m[k] += __shfl_xor_sync(0xffffffffu, m[k], 1);
-                    m[k] += __shfl_xor_sync(0xffffffffu, m[k], 2);
-                    if (tx == 0) S.m[ty * S.ldm + i * D3 + k] = m[k];
+            for (int e = 0; e < D1; ++e) {
+                const int at = (tx * kBxU + 4 * h) * D1 + 4 * e;
+                if (xvec) {
+                    const float4 t = at < nu * D1 ? __ldg(reinterpret_cast<const float4*>(xrow + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    x[4 * e] = t.x; x[4 * e + 1] = t.y; x[4 * e + 2] = t.z; x[4 * e + 3] = t.w;
+                } else {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) x[4 * e + r] = at + r < nu * D1 ? __ldg(xrow + at + r) : 0.0f;
                 }
             }
-            __syncwarp();
-            // the 8 rows of a warp are its own: no barrier
-            const int32_t* seg = P.plan + path[6];
-            for (int t = lane; t < 8 * d2; t += 32) {
-                const int zl = warp * 8 + t / d2, j = t % d2;
-                float s = 0.0f;
-                for (int e = seg[j]; e < seg[j + 1]; e += 2) s = fmaf(__int_as_float(P.plan[e + 1]), S.m[zl * S.ldm + P.plan[e]], s);
-                S.g2[zl * S.ld2 + x2off + v * d2 + j] += s;
-            }
-            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int i = 0; i < D1; ++i)
+#pragma unroll
+                    for (int k = 0; k < D3; ++k) m[i * D3 + k] = fmaf(x[u * D1 + i], q[k][4 * h + u], m[i * D3 + k]);
         }
+#pragma unroll
+        for (int e = 0; e < D1 * D3; ++e) {
+            m[e] += __shfl_xor_sync(0xffffffffu, m[e], 1);
+            m[e] += __shfl_xor_sync(0xffffffffu, m[e], 2);
+            if (tx == (e & 3)) S.m[ty * S.ldm + e] = m[e];
+        }
+        __syncwarp();
+        // the 8 rows of a warp are its own: no barrier
+        const int d2 = s.path[1], x2off = s.path[9] + s.v * d2;
+        const int32_t* seg = P.plan + s.path[6];
+        for (int t = lane; t < 8 * d2; t += 32) {
+            const int zl = warp * 8 + t / d2, j = t % d2;
+            float r = 0.0f;
+            for (int e = seg[j]; e < seg[j + 1]; e += 2) r = fmaf(__int_as_float(P.plan[e + 1]), S.m[zl * S.ldm + P.plan[e]], r);
+            S.g2[zl * S.ld2 + x2off + j] += r;
+        }
+        __syncwarp();
     }
 }
 
@@ -509,36 +1059,45 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
     for (int i = 0; i < D1; ++i)
 #pragma unroll
         for (int u = 0; u < kBxU; ++u) gx[i][u] = 0.0f;
-    if (NEED2) {
-        for (int zl = warp; zl < kBxZ; zl += kThreads / 32) {
-            const float* p = x1 + (z0 + zl) * d1row + x1off + u0 * D1;
-            for (int e = lane; e < 32 * D1; e += 32) S.x[zl * S.ldx + e] = (z0 + zl < Z && e < nu * D1) ? __ldg(p + e) : 0.0f;
-            for (int e = lane; e < d2row; e += 32) S.g2[zl * S.ld2 + e] = 0.0f;
+    const int live = static_cast<int>(min(static_cast<int64_t>(kBxZ), Z - z0));
+    if (NEED2)
+        for (int idx = lane; idx < 8 * S.ld2; idx += 32) S.g2[warp * 8 * S.ld2 + idx] = 0.0f;
+    const float* xrow = x1 + (z0 + min(ty, live - 1)) * d1row + x1off + u0 * D1;
+    const bool xvec = (d1row & 3) == 0 && (nu & 3) == 0 && aligned16(x1 + x1off);
+
+    BwdXStep step{0, 0, 0, P.path(P.in_path(in[3]))};
+    bwd_x_fetch(P, step, W, gout, z0, live, u0, nu, S, 0);
+    for (int buf = 0;; buf ^= 1) {
+        BwdXStep next = step;
+        const bool more = bwd_x_next(P, in, next);
+        if (more) bwd_x_fetch(P, next, W, gout, z0, live, u0, nu, S, buf ^ 1);
+        if (NEED1 && step.c0 == 0)
+            stage_coupling(P.plan, step.path, x2, d2row, step.path[9] + step.v * step.path[1], z0, kBxZ, Z, S.t, (D1 * step.path[2]) | 1);
+        if (more) cp_async_wait<1>(); else cp_async_wait<0>();
+        __syncthreads();
+        switch (step.path[2]) {
+            case 1: bwd_x_step<D1, 1, NEED1, NEED2>(P, step, xrow, xvec, nu, S, buf, gx); break;
+            case 3: bwd_x_step<D1, 3, NEED1, NEED2>(P, step, xrow, xvec, nu, S, buf, gx); break;
+            case 5: bwd_x_step<D1, 5, NEED1, NEED2>(P, step, xrow, xvec, nu, S, buf, gx); break;
+            default: bwd_x_step<D1, 7, NEED1, NEED2>(P, step, xrow, xvec, nu, S, buf, gx); break;
         }
-    }
-    for (int n = 0; n < in[4]; ++n) {
-        const int32_t* path = P.path(P.in_path(in[3] + n));
-        switch (path[2]) {
-            case 1: bwd_x_path<D1, 1, NEED1, NEED2>(P, path, x2, W, gout, z0, Z, u0, nu, S, gx); break;
-            case 3: bwd_x_path<D1, 3, NEED1, NEED2>(P, path, x2, W, gout, z0, Z, u0, nu, S, gx); break;
-            case 5: bwd_x_path<D1, 5, NEED1, NEED2>(P, path, x2, W, gout, z0, Z, u0, nu, S, gx); break;
-            default: bwd_x_path<D1, 7, NEED1, NEED2>(P, path, x2, W, gout, z0, Z, u0, nu, S, gx); break;
-        }
+        __syncthreads();      // the buffers and the coupling are written again
+        if (!more) break;
+        step = next;
     }
     if (NEED1) {
-        __syncthreads();
-        // [row][u * D1 + i] over the staged cotangent, then contiguous row segments
+        // [row][u * D1 + i] over the cotangent buffers, then contiguous row segments
         constexpr int ld = 32 * D1 + 1;
 #pragma unroll
         for (int i = 0; i < D1; ++i)
 #pragma unroll
-            for (int u = 0; u < kBxU; ++u) S.a[ty * ld + (tx * kBxU + u) * D1 + i] = gx[i][u];
+            for (int u = 0; u < kBxU; ++u) S.g[ty * ld + (tx * kBxU + u) * D1 + i] = gx[i][u];
         __syncwarp();
         for (int r = 0; r < 8; ++r) {
             const int zl = warp * 8 + r;
             if (z0 + zl >= Z) break;
             float* o = g1 + (z0 + zl) * d1row + x1off + u0 * D1;
-            for (int e = lane; e < nu * D1; e += 32) o[e] = S.a[zl * ld + e];
+            for (int e = lane; e < nu * D1; e += 32) o[e] = S.g[zl * ld + e];
         }
     }
     if (NEED2) {
@@ -552,22 +1111,21 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
 }
 
 template <bool NEED1, bool NEED2>
-__global__ void __launch_bounds__(kThreads, 2) dense_tile_bwd_x_kernel(const int32_t* __restrict__ plan, const float* __restrict__ x1,
+__global__ void __launch_bounds__(kThreads, 3) dense_tile_bwd_x_kernel(const int32_t* __restrict__ plan, const float* __restrict__ x1,
                                                                        const float* __restrict__ x2, const float* __restrict__ W,
                                                                        const float* __restrict__ gout, float* __restrict__ g1,
-                                                                       float* __restrict__ g2, int64_t Z, int a_floats, BwdXLaunch L) {
+                                                                       float* __restrict__ g2, int64_t Z, int g_floats, BwdXLaunch L) {
     extern __shared__ __align__(16) float smem[];
     const Part2 P(plan);
     BwdXShared S;
-    S.ldx = 32 * P.d1max() + 1;
     S.ldt = (P.d1max() * P.d3max()) | 1;
     S.ldm = S.ldt;
     S.ld2 = plan[2] | 1;
-    S.a = smem;
-    S.w = S.a + a_floats;
-    S.t = S.w + kKC * kLda;
-    S.x = S.t + kBxZ * S.ldt;
-    S.m = S.x + (NEED2 ? kBxZ * S.ldx : 0);
+    S.g_floats = g_floats;
+    S.g = smem;
+    S.w = S.g + 2 * g_floats;
+    S.t = S.w + 2 * kKC * kLda;
+    S.m = S.t + kBxZ * S.ldt;
     S.g2 = S.m + (NEED2 ? kBxZ * S.ldm : 0);
     int s = 0;
     while (s + 1 < L.n && static_cast<int>(blockIdx.x) >= L.first_block[s + 1]) ++s;
@@ -583,13 +1141,15 @@ __global__ void __launch_bounds__(kThreads, 2) dense_tile_bwd_x_kernel(const int
 
 constexpr int kMaxShared = 227 * 1024;
 
-// Floats of the operand buffer of dense_tile_bwd_x_kernel: the staged cotangent, later the grad_x1 tile.
-inline int bwd_x_a_floats(int d1max, int d3max) { return std::max(kBxZ * d3max * kLda, (kBxZ * (32 * d1max + 1) + 3) & ~3); }
+// Floats of one cotangent buffer of dense_tile_bwd_x_kernel; the two together later hold the grad_x1 tile.
+inline int bwd_x_g_floats(int d1max, int d3max) {
+    return std::max(kBxZ * pad_row(32 * d3max), ((kBxZ * (32 * d1max + 1) + 1) / 2 + 3) & ~3);
+}
 
 inline size_t bwd_x_shared(const int32_t* plan, int d1max, int d3max, bool need2) {
     const int ldt = (d1max * d3max) | 1;
-    size_t f = bwd_x_a_floats(d1max, d3max) + kKC * kLda + kBxZ * ldt;
-    if (need2) f += static_cast<size_t>(kBxZ) * (32 * d1max + 1) + kBxZ * ldt + kBxZ * (plan[2] | 1);
+    size_t f = 2 * static_cast<size_t>(bwd_x_g_floats(d1max, d3max)) + 2 * kKC * kLda + kBxZ * ldt;
+    if (need2) f += static_cast<size_t>(kBxZ) * (ldt + (plan[2] | 1));
     return f * sizeof(float);
 }
 
@@ -597,9 +1157,125 @@ bool too_many_blocks(int64_t blocks) { return blocks > 2147483647LL; }
 
 }  // namespace
 
+// Whether every group of the plan suits the row kernels: l <= 3 on both sides of every path.
+static bool rows_plan(const Part2& P) {
+    if (P.d1max() > 7 || P.d3max() > 7) return false;
+    for (int g = 0; g < P.n_groups(); ++g)
+        if (P.group(g)[2] > 7) return false;
+    return true;
+}
+
+// A plan couples a second operand in all of its paths (a product) or in none (a Linear).
+static bool coupled_plan(const Part2& P) { return P.h[2] > 0 && P.chunk(0)[3] >= 0; }
+
+// pass: 0 every group, 1 the groups of scalars, 2 the others.
+template <bool COUPLED, bool GATE>
+static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
+                           float* out, int64_t Z, int accumulate, const DenseGateEpilogue& ep, int pass, cudaStream_t s, bool* done) {
+    const Part2 P(plan_host);
+    int g0 = 0;
+    while (g0 < P.n_groups()) {
+        RowsLaunch L;
+        L.n = 0;
+        int64_t blocks = 0;
+        size_t floats = 0;
+        for (; g0 < P.n_groups() && L.n < kMaxGroups; ++g0) {
+            const int32_t* g = P.group(g0);
+            if (g[1] == 0 || g[4] == 0 || (pass == 1 && g[2] != 1) || (pass == 2 && g[2] == 1)) continue;
+            // the narrowest tile that holds the group's channels in one pass, so that the coupled operand is built once
+            const int tx = g[1] <= 32 ? 4 : g[1] <= 64 ? 8 : 16;
+            const FwdShape shape = fwd_shape<COUPLED>(g[2], tx, P.d1max(), plan_host[2]);
+            L.first_block[L.n] = static_cast<int>(blocks);
+            L.group[L.n] = static_cast<int16_t>(g0);
+            L.shape[L.n] = static_cast<int16_t>(tx);
+            blocks += ceil_div(Z, shape.rows) * ceil_div(g[1], 8 * tx);
+            if (too_many_blocks(blocks)) return fail(E3B_ERR_ARG, "dense_fwd: too many rows");
+            floats = std::max(floats, shape.floats);
+            ++L.n;
+        }
+        if (L.n == 0) continue;
+        L.first_block[L.n] = static_cast<int>(blocks);
+        const size_t bytes = floats * sizeof(float);
+        if (bytes > static_cast<size_t>(kMaxShared)) return E3B_OK;      // a very wide second operand: *done stays false
+        auto kernel = dense_rows_fwd_kernel<COUPLED, GATE>;
+        E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+        kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, weight, out, Z, accumulate, L, ep);
+        if (int rc = check_launch("e3b_dense_fwd")) return rc;
+        *done = true;
+    }
+    *done = true;
+    return E3B_OK;
+}
+
+template <bool COUPLED>
+static int launch_rows_wgrad(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* gout,
+                             float* grad_w, int64_t Z, cudaStream_t s, bool* done) {
+    const Part2 P(plan_host);
+    int g0 = 0;
+    while (g0 < P.n_groups()) {
+        RowsLaunch L;
+        L.n = 0;
+        int64_t blocks = 0, work[kMaxGroups], total_work = 0, tiles[kMaxGroups], parts[kMaxGroups];
+        size_t floats = 0;
+        for (; g0 < P.n_groups() && L.n < kMaxGroups; ++g0) {
+            const int32_t* g = P.group(g0);
+            if (g[1] == 0 || g[4] == 0) continue;
+            const int bw = g[1] <= 32 ? 32 : g[1] <= 64 ? 64 : 128;
+            const FwdShape shape = wgrad_shape<COUPLED>(g[2], bw, P.d1max(), plan_host[2]);
+            L.group[L.n] = static_cast<int16_t>(g0);
+            L.shape[L.n] = static_cast<int16_t>(bw);
+            parts[L.n] = ceil_div(g[4], 4096 / bw / kKC) * ceil_div(g[1], bw);
+            tiles[L.n] = ceil_div(Z, shape.rows);
+            work[L.n] = parts[L.n] * tiles[L.n] * shape.rows * g[2];
+            total_work += work[L.n];
+            floats = std::max(floats, shape.floats);
+            ++L.n;
+        }
+        if (L.n == 0) continue;
+        const size_t bytes = floats * sizeof(float);
+        if (bytes > static_cast<size_t>(kMaxShared)) return E3B_OK;
+        // one wave of resident blocks over all groups, in proportion to their rows x components
+        const int64_t resident = kNumSMs * std::max<int64_t>(1, std::min<int64_t>(4, kMaxShared / static_cast<int64_t>(bytes + 1024)));
+        for (int n = 0; n < L.n; ++n) {
+            const int64_t share = resident * work[n] / total_work;
+            L.splits[n] = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(tiles[n], share / parts[n])));
+            L.first_block[n] = static_cast<int>(blocks);
+            blocks += parts[n] * L.splits[n];
+        }
+        L.first_block[L.n] = static_cast<int>(blocks);
+        if (too_many_blocks(blocks)) return fail(E3B_ERR_ARG, "dense_bwd_w: too many blocks");
+        auto kernel = dense_rows_wgrad_kernel<COUPLED>;
+        E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+        kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, gout, grad_w, Z, L);
+        if (int rc = check_launch("e3b_dense_bwd_w")) return rc;
+        *done = true;
+    }
+    *done = true;
+    return E3B_OK;
+}
+
+int launch_dense_rows_gate(const int32_t* plan_host, const int32_t* plan_dev, const float* x, const float* weight,
+                           const DenseGateEpilogue& ep, int64_t Z, cudaStream_t s, bool* done) {
+    const Part2 P(plan_host);
+    *done = false;
+    if (!rows_plan(P) || coupled_plan(P)) return E3B_OK;
+    // scalars and gates first: the gated irreps read the activated gates of the same rows
+    if (int rc = launch_rows_fwd<false, true>(plan_host, plan_dev, x, nullptr, weight, nullptr, Z, 0, ep, 1, s, done)) return rc;
+    if (!*done) return E3B_OK;
+    return launch_rows_fwd<false, true>(plan_host, plan_dev, x, nullptr, weight, nullptr, Z, 0, ep, 2, s, done);
+}
+
 int launch_dense_tile_fwd(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
                           float* out, int64_t Z, int accumulate, cudaStream_t s) {
     const Part2 P(plan_host);
+    if (rows_plan(P)) {
+        bool done = false;
+        const DenseGateEpilogue none{nullptr, nullptr, nullptr, nullptr, 0, 0};
+        const int rc = coupled_plan(P)
+                           ? launch_rows_fwd<true, false>(plan_host, plan_dev, x1, x2, weight, out, Z, accumulate, none, 0, s, &done)
+                           : launch_rows_fwd<false, false>(plan_host, plan_dev, x1, x2, weight, out, Z, accumulate, none, 0, s, &done);
+        if (rc != E3B_OK || done) return rc;
+    }
     int g0 = 0;
     while (g0 < P.n_groups()) {
         FwdLaunch L;
@@ -634,6 +1310,12 @@ int launch_dense_tile_fwd(const int32_t* plan_host, const int32_t* plan_dev, con
 int launch_dense_tile_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* gout,
                             float* grad_w, int64_t Z, cudaStream_t s) {
     const Part2 P(plan_host);
+    if (rows_plan(P)) {
+        bool done = false;
+        const int rc = coupled_plan(P) ? launch_rows_wgrad<true>(plan_host, plan_dev, x1, x2, gout, grad_w, Z, s, &done)
+                                       : launch_rows_wgrad<false>(plan_host, plan_dev, x1, x2, gout, grad_w, Z, s, &done);
+        if (rc != E3B_OK || done) return rc;
+    }
     int g0 = 0;
     while (g0 < P.n_groups()) {
         BwdWLaunch L;
@@ -697,7 +1379,7 @@ static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const
         auto kernel = dense_tile_bwd_x_kernel<NEED1, NEED2>;
         E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
         kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, weight, gout, g1, g2, Z,
-                                                                      bwd_x_a_floats(P.d1max(), P.d3max()), L);
+                                                                      bwd_x_g_floats(P.d1max(), P.d3max()), L);
         if (int rc = check_launch("e3b_dense_bwd_x")) return rc;
     }
     return E3B_OK;
