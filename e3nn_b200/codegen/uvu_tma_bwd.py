@@ -173,13 +173,14 @@ constexpr int kB2RingBytes = kB2Depth * kV2StageBytes;
 constexpr int kB2YStride = kV2YStride;
 constexpr int kB2DyStride = 17;                            // floats per edge of a warp's partial grad_Y (conflict-free columns)
 constexpr int kB2BatchFloats = 32 * kB2YStride + kB2T * 32 * kB2DyStride;
-constexpr int kB2SmemBytes = kB2Teams * kB2RingBytes + kB2Teams * 2 * kB2Depth * 8 + 128 + kB2Teams * kB2BatchFloats * 4;
+constexpr int kB2SmemBytes = kB2Teams * kB2RingBytes + kB2Teams * 2 * kB2Depth * 8 + 128 + kB2Teams * kB2BatchFloats * 4 +
+                             kB2Teams * kV2IdBytes;
 
 // One lane per edge: sum the warps' partial grad_Y of a finished batch, apply the harmonics Jacobian, store.
-__device__ __forceinline__ void b2_batch_finish(const float* __restrict__ vec, float* __restrict__ grad_vec, int64_t e0, int count,
-                                                const float* dybuf, int lane) {{
+__device__ __forceinline__ void b2_batch_finish(const float* __restrict__ vec, float* __restrict__ grad_vec, const V2Ids& ids, uint32_t it0,
+                                                int count, const float* dybuf, int lane) {{
     if (lane < count) {{
-        const int64_t ee = e0 + lane;
+        const int64_t ee = ids.edge[(it0 + lane) & 63u];
         float gY[kD2];
 #pragma unroll
         for (int j = 0; j < kD2; ++j) {{
@@ -210,8 +211,8 @@ __device__ __forceinline__ void b2_halve(float* dy, int lane) {{
 // their output slots); staging, harmonics, reduction and stores are one copy of code for all of them, which
 // keeps the kernel's hot code inside the SM's instruction cache.
 __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float* __restrict__ node_x, const float* __restrict__ vec,
-        const int64_t* __restrict__ edge_src, const int64_t* __restrict__ rowptr, const float* __restrict__ w,
-        const float* __restrict__ gout, float* __restrict__ grad_w, float* __restrict__ grad_vec, int64_t num_nodes,
+        const int64_t* __restrict__ edge_src, const int64_t* __restrict__ rowptr, const int64_t* __restrict__ perm,
+        const float* __restrict__ w, const float* __restrict__ gout, float* __restrict__ grad_w, float* __restrict__ grad_vec, int64_t num_nodes,
         int64_t num_src, int64_t num_edges, float scale, int* __restrict__ status) {{
     extern __shared__ __align__(128) uint8_t v2_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -223,6 +224,9 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + kB2Teams * 2 * kB2Depth);
     float* ybuf = reinterpret_cast<float*>(v2_smem + kB2Teams * kB2RingBytes + kB2Teams * 2 * kB2Depth * 8 + 128) + team * kB2BatchFloats;
     float* dybuf = ybuf + 32 * kB2YStride;
+    V2Ids ids;
+    ids.edge = reinterpret_cast<int64_t*>(v2_smem + kB2SmemBytes - kB2Teams * kV2IdBytes + team * kV2IdBytes);
+    ids.src = ids.edge + 64;
     if (threadIdx.x == 0) *abort_flag = 0;
     if (tw == 0 && lane == 0) {{
         for (int s = 0; s < kB2Depth; ++s) {{ tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], kB2T); }}
@@ -235,18 +239,20 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
     const int64_t n_hi = team_id + 1 == num_teams ? num_nodes : v2_lower_bound(rowptr, num_nodes, (num_edges * (team_id + 1)) / num_teams);
     if (n_lo >= n_hi) return;
     const bool leader = tw == 0 && lane == 0;
-    int64_t e = rowptr[n_lo];
-    const int64_t e_hi = rowptr[n_hi];
+    const int64_t e_lo = rowptr[n_lo], e_hi = rowptr[n_hi];
+    int64_t e = e_lo;
     int64_t issue = e;
-    int64_t src_pref = 0;
     bool ok = true;
-    if (leader) {{
-        for (int s = 0; s < kB2Depth && issue < e_hi; ++s, ++issue) {{
-            int64_t sidx = edge_src[issue];
-            if (sidx < 0 || sidx >= num_src) {{ atomicExch(status, 2); sidx = 0; }}
-            v2_issue(ring + s * kV2StageBytes, &full[s], w + issue * kWn, node_x + sidx * kD1);
-        }}
-        if (issue < e_hi) src_pref = edge_src[issue];
+    auto stage_next = [&](int s) {{
+        const int at = static_cast<int>((issue - e_lo) & 63);
+        const int64_t sidx = ids.src[at];
+        v2_issue(ring + s * kV2StageBytes, &full[s], w + ids.edge[at] * kWn, node_x + (sidx < 0 ? 0 : sidx) * kD1);
+        ++issue;
+    }};
+    if (tw == 0) {{
+        ids.load(perm, edge_src, e_lo, e_lo, e_hi, num_edges, num_src, lane, status);
+        __syncwarp();
+        if (leader) for (int s = 0; s < kB2Depth && issue < e_hi; ++s) stage_next(s);
     }}
 {_indent(g_decl, 4)}
     uint32_t it = 0;
@@ -265,8 +271,10 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
                 __syncwarp();
                 v2_team_sync<kB2T>(team);
                 if (tw == 0) {{
-                    if (it > 0) b2_batch_finish(vec, grad_vec, e - 32, 32, dybuf, lane);
-                    v2_batch_harmonics(vec, e, e_hi, ybuf, lane);
+                    if (it > 0) b2_batch_finish(vec, grad_vec, ids, it - 32, 32, dybuf, lane);
+                    __syncwarp();
+                    ids.load(perm, edge_src, e + 32, e_lo, e_hi, num_edges, num_src, lane, status);
+                    v2_batch_harmonics(vec, ids, it, e_hi - e, ybuf, lane);
                 }}
                 __syncwarp();
                 v2_team_sync<kB2T>(team);
@@ -278,7 +286,7 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
             if (!ok) continue;
             const float* sw = reinterpret_cast<const float*>(ring + s * kV2StageBytes);
             const float* sx = reinterpret_cast<const float*>(ring + s * kV2StageBytes + kV2StageW);
-            float* gwrow = grad_w + e * kWn;
+            float* gwrow = grad_w + ids.edge[it & 63u] * kWn;
             float Y[kD2];
 #pragma unroll
             for (int j = 0; j < kD2; ++j) Y[j] = ybuf[slot * kB2YStride + j];
@@ -290,12 +298,8 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
                 const int sp = (it - 1) % kB2Depth;
                 const uint32_t php = ((it - 1) / kB2Depth) & 1u;
                 if (tc::mbar_wait(&empty[sp], php, abort_flag)) {{
-                    int64_t sidx = src_pref;
-                    if (sidx < 0 || sidx >= num_src) {{ atomicExch(status, 2); sidx = 0; }}
                     tc::fence_proxy_async_smem();
-                    v2_issue(ring + sp * kV2StageBytes, &full[sp], w + issue * kWn, node_x + sidx * kD1);
-                    ++issue;
-                    if (issue < e_hi) src_pref = edge_src[issue];
+                    stage_next(sp);
                 }}
             }}
             // sum grad_Y over the 64 channels: fold the pairs, then recursive halving over the lanes
@@ -310,7 +314,7 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
         const int count = (it & 31u) != 0u ? static_cast<int>(it & 31u) : (it > 0 ? 32 : 0);
         __syncwarp();
         v2_team_sync<kB2T>(team);
-        if (tw == 0 && ok) b2_batch_finish(vec, grad_vec, e - count, count, dybuf, lane);
+        if (tw == 0 && ok) b2_batch_finish(vec, grad_vec, ids, it - count, count, dybuf, lane);
     }}
     if (!ok) {{
         if (lane == 0) atomicExch(status, 3);
@@ -319,14 +323,13 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
 }}
 """
     launch = """
-    if (in2_mode == 1 && perm == nullptr && g_conv_impl != 1 &&
+    if (in2_mode == 1 && g_conv_impl != 1 &&
         reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(node_x) % 16 == 0) {
         cudaError_t err = cudaFuncSetAttribute(conv_bwd_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kB2SmemBytes);
         if (err != cudaSuccess) return e3b_layout_fail(-2, "conv_bwd: smem attribute: %s", cudaGetErrorString(err));
-        const int64_t want = (num_nodes + kB2Teams - 1) / kB2Teams;
-        const unsigned b2grid = static_cast<unsigned>(want < 148 ? want : 148);
-        conv_bwd_tma_kernel<<<b2grid, kB2Threads, kB2SmemBytes, s>>>(node_x, x2, edge_src, rowptr, w, grad_out, grad_w, grad_x2,
-                                                                     num_nodes, num_src, num_edges, scale, status);
+        const unsigned b2grid = static_cast<unsigned>(num_nodes < 148 ? num_nodes : 148);
+        conv_bwd_tma_kernel<<<b2grid, kB2Threads, kB2SmemBytes, s>>>(node_x, x2, edge_src, rowptr, perm, w, grad_out, grad_w,
+                                                                     grad_x2, num_nodes, num_src, num_edges, scale, status);
         return e3b_layout_check("conv_bwd (bulk-copy pipeline)");
     }
 """

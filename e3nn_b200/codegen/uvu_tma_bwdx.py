@@ -116,7 +116,7 @@ constexpr int kX2StageBytes = {stage};       // one edge's weight row
 constexpr int kX2RingBytes = kX2Depth * kX2StageBytes;
 constexpr int kX2RowFloats = (kD1 + 31) / 32 * 32;   // one gradient row, padded to whole 128-byte lines
 constexpr int kX2SmemBytes = kX2Teams * kX2RingBytes + kX2Teams * 2 * kX2Depth * 8 + 128 + kX2Teams * 32 * kV2YStride * 4 +
-                             kX2Teams * 2 * kX2T * kX2RowFloats * 4;
+                             kX2Teams * 2 * kX2T * kX2RowFloats * 4 + kX2Teams * kV2IdBytes;
 
 __device__ __forceinline__ void x2_issue(uint8_t* stage, uint64_t* bar, const float* wrow) {{
     const uint32_t b = tc::smem_u32(bar);
@@ -126,9 +126,9 @@ __device__ __forceinline__ void x2_issue(uint8_t* stage, uint64_t* bar, const fl
 }}
 
 __global__ void __launch_bounds__(kX2Threads, 1) conv_bwd_x_tma_kernel(const float* __restrict__ vec,
-        const int64_t* __restrict__ edge_src, const int64_t* __restrict__ rowptr, const float* __restrict__ w,
-        const float* __restrict__ gout, float* __restrict__ grad_node_x, int64_t num_nodes, int64_t num_src,
-        int64_t num_edges, float scale, int* __restrict__ status) {{
+        const int64_t* __restrict__ edge_src, const int64_t* __restrict__ rowptr, const int64_t* __restrict__ perm,
+        const float* __restrict__ w, const float* __restrict__ gout, float* __restrict__ grad_node_x, int64_t num_nodes,
+        int64_t num_src, int64_t num_edges, float scale, int* __restrict__ status) {{
     extern __shared__ __align__(128) uint8_t v2_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int team = warp / kX2T, tw = warp % kX2T;
@@ -142,6 +142,9 @@ __global__ void __launch_bounds__(kX2Threads, 1) conv_bwd_x_tma_kernel(const flo
     // the table receives one row per edge in whole 128-byte lines instead of one strided float at a time per warp
     float* xrows = reinterpret_cast<float*>(v2_smem + kX2Teams * kX2RingBytes + kX2Teams * 2 * kX2Depth * 8 + 128) +
                    kX2Teams * 32 * kV2YStride + team * 2 * kX2T * kX2RowFloats;
+    V2Ids ids;
+    ids.edge = reinterpret_cast<int64_t*>(v2_smem + kX2SmemBytes - kX2Teams * kV2IdBytes + team * kV2IdBytes);
+    ids.src = ids.edge + 64;
     if (threadIdx.x == 0) *abort_flag = 0;
     if (tw == 0 && lane == 0) {{
         for (int s = 0; s < kX2Depth; ++s) {{ tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], kX2T); }}
@@ -154,12 +157,18 @@ __global__ void __launch_bounds__(kX2Threads, 1) conv_bwd_x_tma_kernel(const flo
     const int64_t n_hi = team_id + 1 == num_teams ? num_nodes : v2_lower_bound(rowptr, num_nodes, (num_edges * (team_id + 1)) / num_teams);
     if (n_lo >= n_hi) return;
     const bool leader = tw == 0 && lane == 0;
-    int64_t e = rowptr[n_lo];
-    const int64_t e_hi = rowptr[n_hi];
+    const int64_t e_lo = rowptr[n_lo], e_hi = rowptr[n_hi];
+    int64_t e = e_lo;
     int64_t issue = e;
     bool ok = true;
-    if (leader) {{
-        for (int s = 0; s < kX2Depth && issue < e_hi; ++s, ++issue) x2_issue(ring + s * kX2StageBytes, &full[s], w + issue * kWn);
+    auto stage_next = [&](int s) {{
+        x2_issue(ring + s * kX2StageBytes, &full[s], w + ids.edge[(issue - e_lo) & 63] * kWn);
+        ++issue;
+    }};
+    if (tw == 0) {{
+        ids.load(perm, edge_src, e_lo, e_lo, e_hi, num_edges, num_src, lane, status);
+        __syncwarp();
+        if (leader) for (int s = 0; s < kX2Depth && issue < e_hi; ++s) stage_next(s);
     }}
 {_indent(g_decl, 4)}
     uint32_t it = 0;
@@ -176,14 +185,16 @@ __global__ void __launch_bounds__(kX2Threads, 1) conv_bwd_x_tma_kernel(const flo
             if (slot == 0) {{
                 __syncwarp();
                 v2_team_sync<kX2T>(team);
-                if (tw == 0) v2_batch_harmonics(vec, e, e_hi, ybuf, lane);
+                if (tw == 0) {{
+                    ids.load(perm, edge_src, e + 32, e_lo, e_hi, num_edges, num_src, lane, status);
+                    v2_batch_harmonics(vec, ids, it, e_hi - e, ybuf, lane);
+                }}
                 __syncwarp();
                 v2_team_sync<kX2T>(team);
             }}
             if (!ok) {{ __syncwarp(); v2_team_sync<kX2T>(team); continue; }}   // keep the team barriers in step
             const int s = it % kX2Depth;
             const uint32_t ph = (it / kX2Depth) & 1u;
-            int64_t sidx = edge_src[e];   // issued before the wait: its latency overlaps the wait for the staged row
             ok = __all_sync(0xffffffffu, tc::mbar_wait(&full[s], ph, abort_flag));
             if (!ok) {{ __syncwarp(); v2_team_sync<kX2T>(team); continue; }}
             const float* sw = reinterpret_cast<const float*>(ring + s * kX2StageBytes);
@@ -199,8 +210,7 @@ __global__ void __launch_bounds__(kX2Threads, 1) conv_bwd_x_tma_kernel(const flo
                 const uint32_t php = ((it - 1) / kX2Depth) & 1u;
                 if (tc::mbar_wait(&empty[sp], php, abort_flag)) {{
                     tc::fence_proxy_async_smem();
-                    x2_issue(ring + sp * kX2StageBytes, &full[sp], w + issue * kWn);
-                    ++issue;
+                    stage_next(sp);
                 }}
             }}
             {{
@@ -209,8 +219,8 @@ __global__ void __launch_bounds__(kX2Threads, 1) conv_bwd_x_tma_kernel(const flo
             }}
             __syncwarp();
             v2_team_sync<kX2T>(team);
-            const bool in_range = sidx >= 0 && sidx < num_src;
-            if (!in_range && lane == 0) atomicExch(status, 2);
+            const int64_t sidx = ids.src[it & 63u];
+            const bool in_range = sidx >= 0;      // (reported when the number was read)
             {{
                 // flush: every warp takes its share of the columns, sums the warps' partial rows, adds to the table
                 const float* xb = xrows + (it & 1u) * kX2T * kX2RowFloats;
@@ -232,13 +242,12 @@ __global__ void __launch_bounds__(kX2Threads, 1) conv_bwd_x_tma_kernel(const flo
 }}
 """
     launch = """
-    if (in2_mode == 1 && perm == nullptr && g_conv_impl != 1 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
+    if (in2_mode == 1 && g_conv_impl != 1 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
         err = cudaFuncSetAttribute(conv_bwd_x_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kX2SmemBytes);
         if (err != cudaSuccess) return e3b_layout_fail(-2, "conv_bwd_x: smem attribute: %s", cudaGetErrorString(err));
-        const int64_t want = (num_nodes + kX2Teams - 1) / kX2Teams;
-        const unsigned x2grid = static_cast<unsigned>(want < 148 ? want : 148);
-        conv_bwd_x_tma_kernel<<<x2grid, kX2Threads, kX2SmemBytes, s>>>(x2, edge_src, rowptr, w, grad_out, grad_node_x, num_nodes,
-                                                                        num_src, num_edges, scale, status);
+        const unsigned x2grid = static_cast<unsigned>(num_nodes < 148 ? num_nodes : 148);
+        conv_bwd_x_tma_kernel<<<x2grid, kX2Threads, kX2SmemBytes, s>>>(x2, edge_src, rowptr, perm, w, grad_out, grad_node_x,
+                                                                        num_nodes, num_src, num_edges, scale, status);
         return e3b_layout_check("conv_bwd_x (bulk-copy pipeline)");
     }
 """
