@@ -12,7 +12,10 @@
 // Chebyshev recurrence of sin(k theta), because fp32 argument reduction alone costs a digit of the 1e-5
 // error budget), then one edge per step with the hidden units across the lanes (coalesced rows of h).
 // The gradient kernel recomputes the pre-activations instead of storing [E, hidden], reduces the basis
-// cotangent over the lanes by recursive halving and adds the position gradient with float atomics.
+// cotangent over the lanes by recursive halving and adds the position gradient with float atomics.  It also forms the
+// gradient of the layer's weights: a lane keeps the (basis, hidden unit) entries of its columns in registers over all its
+// edges, a block sums its warps in order and writes one partial matrix, a second kernel adds the partials in a fixed order
+// (429,000 edges, 8 x 64: 138 us against some 25 torch launches of 440 us for the training step's embedding and gradient).
 #include "common.cuh"
 
 namespace e3b {
@@ -233,15 +236,17 @@ __device__ __forceinline__ void halve(float* v, int lane) {
     }
 }
 
-template <int H2, int NB>
+// GP: position gradient (grad_vec is read too); GW: partial weight gradients, partial[block][nb * H] (without w_scale).
+template <int H2, int NB, bool GP, bool GW>
 __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
         const float* __restrict__ pos, const int64_t* __restrict__ src, const int64_t* __restrict__ dst,
         const float* __restrict__ shift, const float* __restrict__ w0, const float* __restrict__ grad_h,
         const float* __restrict__ grad_vec, int64_t num_edges, int64_t num_nodes, RadialSpec sp, float w_scale,
-        float act_scale, int act, float* __restrict__ grad_pos, int* __restrict__ status) {
+        float act_scale, int act, float* __restrict__ grad_pos, float* __restrict__ partial, int* __restrict__ status) {
     __shared__ float s_basis[kEmbedWarps][32][kMaxBasis + 1];
-    __shared__ float s_cot[kEmbedWarps][32][kMaxBasis + 1];
+    __shared__ float s_cot[GP ? kEmbedWarps : 1][32][kMaxBasis + 1];
     __shared__ float s_env[kEmbedWarps][32];     // envelope value of the batch's edges
+    __shared__ float s_gw[GW ? NB * 32 * H2 : 1];
     __shared__ float s_genv[kEmbedWarps][32];    // cotangent of the envelope
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = sp.nb;
@@ -251,6 +256,13 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
     for (int k = 0; k < NB; ++k)
 #pragma unroll
         for (int j = 0; j < H2; ++j) w[k][j] = k < nb ? w0[k * H + lane + 32 * j] * w_scale : 0.0f;
+    float gw[GW ? NB : 1][GW ? H2 : 1];
+    if (GW) {
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+#pragma unroll
+            for (int j = 0; j < H2; ++j) gw[GW ? k : 0][GW ? j : 0] = 0.0f;
+    }
     const int64_t batches = (num_edges + 31) / 32;
     for (int64_t b = static_cast<int64_t>(blockIdx.x) * kEmbedWarps + warp; b < batches;
          b += static_cast<int64_t>(gridDim.x) * kEmbedWarps) {
@@ -262,7 +274,7 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
         for (int k = 0; k < kMaxBasis; ++k) dbasis[k] = 0.0f;
         if (e < num_edges) {
             g = edge_geom(pos, src, dst, shift, e, num_nodes, status);
-            radial_basis(sp, g.r, s_basis[warp][lane], dbasis);
+            radial_basis(sp, g.r, s_basis[warp][lane], GP ? dbasis : nullptr);
             radial_envelope(sp, g.r, env, denv);
             s_env[warp][lane] = env;
         }
@@ -299,22 +311,30 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
 #pragma unroll
             for (int j = 0; j < H2; ++j) {
                 const float gh = gh_cur[j];
-                if (sp.envelope) genv = fmaf(gh * act_scale, act_fwd(act, pre[j]), genv);
+                if (GP && sp.envelope) genv = fmaf(gh * act_scale, act_fwd(act, pre[j]), genv);
                 const float dpre = gh * (envi * act_scale) * act_grad(act, pre[j]);
+                if (GP) {
 #pragma unroll
-                for (int k = 0; k < NB; ++k) cot[k] = fmaf(w[k][j], dpre, cot[k]);
+                    for (int k = 0; k < NB; ++k) cot[k] = fmaf(w[k][j], dpre, cot[k]);
+                }
+                if (GW) {
+#pragma unroll
+                    for (int k = 0; k < NB; ++k)
+                        if (k < nb) gw[GW ? k : 0][GW ? j : 0] = fmaf(s_basis[warp][i][k], dpre, gw[GW ? k : 0][GW ? j : 0]);
+                }
             }
+            if (!GP) continue;
             if (NB == 16) {
                 halve<16, NB / 2>(cot, lane); halve<8, 4>(cot, lane); halve<4, 2>(cot, lane); halve<2, 1>(cot, lane);
                 cot[0] += __shfl_xor_sync(0xffffffffu, cot[0], 1);
                 // after the four halvings lane l holds component (l >> 1) & 15 (bit 4 chose the upper 8, bit 3 the upper 4, ...)
-                if ((lane & 1) == 0) s_cot[warp][i][(lane >> 1) & 15] = cot[0];
+                if ((lane & 1) == 0) s_cot[GP ? warp : 0][i][(lane >> 1) & 15] = cot[0];
             } else {
                 halve<16, 4>(cot, lane); halve<8, 2>(cot, lane); halve<4, 1>(cot, lane);
                 cot[0] += __shfl_xor_sync(0xffffffffu, cot[0], 2);
                 cot[0] += __shfl_xor_sync(0xffffffffu, cot[0], 1);
                 // three halvings over lane bits 4, 3, 2: lane l holds component (l >> 2) & 7
-                if ((lane & 3) == 0) s_cot[warp][i][(lane >> 2) & 7] = cot[0];
+                if ((lane & 3) == 0) s_cot[GP ? warp : 0][i][(lane >> 2) & 7] = cot[0];
             }
             if (sp.envelope) {
 #pragma unroll
@@ -323,11 +343,11 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
             }
         }
         __syncwarp();
-        if (e < num_edges) {
+        if (GP && e < num_edges) {
             double dr = sp.envelope ? static_cast<double>(s_genv[warp][lane]) * denv : 0.0;
 #pragma unroll
             for (int k = 0; k < kMaxBasis; ++k)
-                if (k < nb) dr += static_cast<double>(s_cot[warp][lane][k]) * dbasis[k];
+                if (k < nb) dr += static_cast<double>(s_cot[GP ? warp : 0][lane][k]) * dbasis[k];
             float gx = 0.0f, gy = 0.0f, gz = 0.0f;
             if (grad_vec) { gx = grad_vec[e * 3]; gy = grad_vec[e * 3 + 1]; gz = grad_vec[e * 3 + 2]; }
             if (g.r > 0.0) {
@@ -339,6 +359,39 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
         }
         __syncwarp();
     }
+    if (GW) {
+        for (int q = 0; q < kEmbedWarps; ++q) {
+            if (warp == q) {
+#pragma unroll
+                for (int k = 0; k < NB; ++k)
+#pragma unroll
+                    for (int j = 0; j < H2; ++j) {
+                        float* at = s_gw + (k * H + lane + 32 * j);
+                        *at = (q > 0 ? *at : 0.0f) + gw[GW ? k : 0][GW ? j : 0];
+                    }
+            }
+            __syncthreads();
+        }
+        for (int c = threadIdx.x; c < nb * H; c += kEmbedWarps * 32) partial[static_cast<int64_t>(blockIdx.x) * nb * H + c] = s_gw[c];
+    }
+}
+
+// grad_w0[c] = w_scale * sum over the blocks of partial[block][c]: 32 columns a block, 32 warps over the rows.
+__global__ void __launch_bounds__(1024) radial_embed_weight_sum_kernel(const float* __restrict__ partial, int blocks, int cols, float w_scale,
+                                                                       float* __restrict__ grad_w0) {
+    __shared__ float s[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+    float v = 0.0f;
+    if (c < cols) {
+#pragma unroll 8
+        for (int b = warp; b < blocks; b += 32) v += partial[static_cast<int64_t>(b) * cols + c];
+    }
+    s[warp][lane] = v;
+    __syncthreads();
+    v = s[lane][warp];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0 && blockIdx.x * 32 + warp < cols) grad_w0[blockIdx.x * 32 + warp] = w_scale * v;
 }
 
 int check_embed_args(int64_t num_edges, int64_t num_nodes, int num_basis, int hidden, int act) {
@@ -403,31 +456,70 @@ extern "C" int e3b_radial_embed_fwd(const float* pos, const int64_t* edge_src, c
     return check_launch("radial_embed_fwd");
 }
 
+namespace e3b {
+namespace {
+int embed_bwd(const float* pos, const int64_t* edge_src, const int64_t* edge_dst, const float* shift, const float* w0,
+              const float* grad_h, const float* grad_edge_vec, int64_t num_edges, int64_t num_nodes, int num_basis, int hidden,
+              int basis, int cutoff, int envelope, float start, float end, float basis_scale, float w_scale, float act_scale, int act,
+              float* grad_pos, float* grad_w0, void* scratch, int64_t scratch_bytes, int32_t* status, void* stream) {
+    if (int rc = check_embed_args(num_edges, num_nodes, num_basis, hidden, act)) return rc;
+    RadialSpec sp;
+    if (int rc = make_spec(&sp, basis, cutoff, envelope, num_basis, start, end, basis_scale)) return rc;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int cols = num_basis * hidden;
+    if (num_edges == 0) {
+        if (grad_w0) E3B_CUDA_TRY(cudaMemsetAsync(grad_w0, 0, sizeof(float) * cols, s));
+        return E3B_OK;
+    }
+    if (!pos || !edge_src || !edge_dst || !w0 || !grad_h || (!grad_pos && !grad_w0) || !status)
+        return fail(E3B_ERR_ARG, "radial_embed_bwd: null pointer");
+    const int grid = embed_grid(num_edges), threads = kEmbedWarps * 32;
+    if (grad_w0 && (!scratch || scratch_bytes < static_cast<int64_t>(sizeof(float)) * grid * cols))
+        return fail(E3B_ERR_ARG, "radial_embed_bwd: scratch too small");
+    float* partial = static_cast<float*>(scratch);
+#define E3B_LAUNCH(H2, NBP, GP, GW)                                                                                          \
+    radial_embed_bwd_kernel<H2, NBP, GP, GW><<<grid, threads, 0, s>>>(pos, edge_src, edge_dst, shift, w0, grad_h, grad_edge_vec, \
+                                                                      num_edges, num_nodes, sp, w_scale, act_scale, act, grad_pos, partial, status)
+#define E3B_LAUNCH_G(H2, NBP)                                                                                                \
+    if (!grad_w0) E3B_LAUNCH(H2, NBP, true, false);                                                                          \
+    else if (grad_pos) E3B_LAUNCH(H2, NBP, true, true);                                                                      \
+    else E3B_LAUNCH(H2, NBP, false, true)
+#define E3B_LAUNCH_H(H2)                                                                                                     \
+    if (num_basis <= 8) { E3B_LAUNCH_G(H2, 8); } else { E3B_LAUNCH_G(H2, 16); }
+    switch (hidden / 32) {
+        case 1: E3B_LAUNCH_H(1) break;
+        case 2: E3B_LAUNCH_H(2) break;
+        case 3: E3B_LAUNCH_H(3) break;
+        default: E3B_LAUNCH_H(4) break;
+    }
+#undef E3B_LAUNCH
+#undef E3B_LAUNCH_G
+#undef E3B_LAUNCH_H
+    if (grad_w0) radial_embed_weight_sum_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, grid, cols, w_scale, grad_w0);
+    return check_launch("radial_embed_bwd");
+}
+}  // namespace
+}  // namespace e3b
+
+extern "C" int64_t e3b_radial_embed_scratch_bytes(int64_t num_edges, int num_basis, int hidden) {
+    return static_cast<int64_t>(sizeof(float)) * e3b::embed_grid(num_edges) * num_basis * hidden;
+}
+
+extern "C" int e3b_radial_embed_bwd_all(const float* pos, const int64_t* edge_src, const int64_t* edge_dst, const float* shift,
+                                        const float* w0, const float* grad_h, const float* grad_edge_vec, int64_t num_edges,
+                                        int64_t num_nodes, int num_basis, int hidden, int basis, int cutoff, int envelope,
+                                        float start, float end, float basis_scale, float w_scale, float act_scale, int act,
+                                        float* grad_pos, float* grad_w0, void* scratch, int64_t scratch_bytes, int32_t* status,
+                                        void* stream) {
+    return e3b::embed_bwd(pos, edge_src, edge_dst, shift, w0, grad_h, grad_edge_vec, num_edges, num_nodes, num_basis, hidden, basis, cutoff,
+                          envelope, start, end, basis_scale, w_scale, act_scale, act, grad_pos, grad_w0, scratch, scratch_bytes, status, stream);
+}
+
 extern "C" int e3b_radial_embed_bwd(const float* pos, const int64_t* edge_src, const int64_t* edge_dst, const float* shift,
                                     const float* w0, const float* grad_h, const float* grad_edge_vec, int64_t num_edges,
                                     int64_t num_nodes, int num_basis, int hidden, int basis, int cutoff, int envelope,
                                     float start, float end, float basis_scale, float w_scale, float act_scale, int act,
                                     float* grad_pos, int32_t* status, void* stream) {
-    using namespace e3b;
-    if (int rc = check_embed_args(num_edges, num_nodes, num_basis, hidden, act)) return rc;
-    RadialSpec sp;
-    if (int rc = make_spec(&sp, basis, cutoff, envelope, num_basis, start, end, basis_scale)) return rc;
-    if (num_edges == 0) return E3B_OK;
-    if (!pos || !edge_src || !edge_dst || !w0 || !grad_h || !grad_pos || !status) return fail(E3B_ERR_ARG, "radial_embed_bwd: null pointer");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int grid = embed_grid(num_edges), threads = kEmbedWarps * 32;
-#define E3B_LAUNCH(H2)                                                                                                   \
-    if (num_basis <= 8) E3B_LAUNCH_NB(H2, 8); else E3B_LAUNCH_NB(H2, 16)
-#define E3B_LAUNCH_NB(H2, NBP)                                                                                           \
-    radial_embed_bwd_kernel<H2, NBP><<<grid, threads, 0, s>>>(pos, edge_src, edge_dst, shift, w0, grad_h, grad_edge_vec,  \
-                                                              num_edges, num_nodes, sp, w_scale, act_scale, act, grad_pos, status)
-    switch (hidden / 32) {
-        case 1: E3B_LAUNCH(1); break;
-        case 2: E3B_LAUNCH(2); break;
-        case 3: E3B_LAUNCH(3); break;
-        default: E3B_LAUNCH(4); break;
-    }
-#undef E3B_LAUNCH
-#undef E3B_LAUNCH_NB
-    return check_launch("radial_embed_bwd");
+    return e3b::embed_bwd(pos, edge_src, edge_dst, shift, w0, grad_h, grad_edge_vec, num_edges, num_nodes, num_basis, hidden, basis, cutoff,
+                          envelope, start, end, basis_scale, w_scale, act_scale, act, grad_pos, nullptr, nullptr, 0, status, stream);
 }

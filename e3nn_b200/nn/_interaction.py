@@ -119,6 +119,19 @@ class InteractionBlock(torch.nn.Module):
         basis = bessel(edge_vec.double().norm(dim=-1), self.num_basis, self.r_max).to(edge_vec.dtype)
         return self.fc(basis)
 
+    def _embeds(self, pos, edge_src, edge_dst, shift) -> bool:
+        """Whether a training step (gradient of the first radial layer's weights wanted) may use the fused edge embedding:
+        operands in the one form that kernel reads, no gradient w.r.t. the shifts, and no hooks on the modules it stands for."""
+        E, dev = edge_src.numel(), pos.device
+        w0 = self.fc.layer0.weight
+        return (pos.dim() == 2 and pos.shape[1] == 3 and edge_src.shape == edge_dst.shape == (E,)
+                and edge_src.dtype == edge_dst.dtype == torch.int64 and edge_src.device == edge_dst.device == dev
+                and w0.device == dev and w0.dtype == torch.float32
+                and (shift is None or (shift.shape == (E, 3) and shift.dtype == torch.float32 and shift.device == dev
+                                       and not shift.requires_grad))
+                and not any(hooks for m in (self.fc, self.fc.layer0)
+                            for hooks in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks, m._backward_pre_hooks)))
+
     def forward(self, pos: torch.Tensor, node_features: torch.Tensor, edge_src: torch.Tensor, edge_dst: torch.Tensor,
                 rowptr: torch.Tensor, shift: Optional[torch.Tensor] = None, before_conv=None,
                 phase_mark=None) -> torch.Tensor:
@@ -133,12 +146,14 @@ class InteractionBlock(torch.nn.Module):
         gradient, after the transposed radial layer), e.g. to record CUDA events."""
         layer0 = self.fc.layer0
         fused = (pos.is_cuda and pos.dtype == torch.float32 and len(self.fc.hs) == 3 and self.num_basis <= 16
-                 and self.fc.hs[1] in (32, 64, 96, 128) and not (torch.is_grad_enabled() and layer0.weight.requires_grad))
+                 and self.fc.hs[1] in (32, 64, 96, 128)
+                 and (not (torch.is_grad_enabled() and layer0.weight.requires_grad)
+                      or self._embeds(pos, edge_src, edge_dst, shift)))
         if fused:
             # vectors, Bessel basis and the first radial layer in one kernel (and one for their gradient)
             act = getattr(layer0.act, "__name__", None) if layer0.act is not None else None
             edge_vec, h = edge_embed(pos, edge_src, edge_dst, shift, layer0.weight, self.r_max, layer0._scale(),
-                                     layer0.cst * layer0.var_out ** 0.5, act)
+                                     layer0.cst * layer0.var_out ** 0.5, act, weight_grad=True)
             # a transfer in flight (before_conv is its wait) runs a kernel of its own: leave it some SMs
             limit = 148 - self.overlap_reserved_sms if (before_conv is not None and self.overlap_reserved_sms > 0) else None
             with _lib.tc_gemm_cta_limit(limit):

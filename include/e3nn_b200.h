@@ -150,6 +150,10 @@ int e3b_neighbor_fill_rows(const float* pos, int64_t num_atoms, double box, doub
  * e3b_radial_embed_bwd: cotangents grad_h [num_edges,hidden] and grad_edge_vec [num_edges,3] (or NULL) are
  * pulled back to the positions; the result is ADDED to grad_pos [num_nodes,3] (float atomics; the caller
  * zeroes it).  Replaces autograd through the same reference lines.
+ *
+ * e3b_radial_embed_bwd_all: the same and / or the gradient of the layer's weights: grad_pos (added to) and grad_w0
+ * [num_basis, hidden] (overwritten) may each be NULL, not both; with grad_w0, scratch holds at least
+ * e3b_radial_embed_scratch_bytes(num_edges, num_basis, hidden) bytes.  The weight gradient is summed in a fixed order.
  */
 int e3b_radial_embed_fwd(const float* pos, const int64_t* edge_src, const int64_t* edge_dst, const float* shift,
                          const float* w0, int64_t num_edges, int64_t num_nodes, int num_basis, int hidden, int basis,
@@ -160,6 +164,12 @@ int e3b_radial_embed_bwd(const float* pos, const int64_t* edge_src, const int64_
                          int64_t num_nodes, int num_basis, int hidden, int basis, int cutoff, int envelope, float start,
                          float end, float basis_scale, float w_scale, float act_scale, int act, float* grad_pos,
                          int32_t* status, void* stream);
+int64_t e3b_radial_embed_scratch_bytes(int64_t num_edges, int num_basis, int hidden);
+int e3b_radial_embed_bwd_all(const float* pos, const int64_t* edge_src, const int64_t* edge_dst, const float* shift,
+                             const float* w0, const float* grad_h, const float* grad_edge_vec, int64_t num_edges,
+                             int64_t num_nodes, int num_basis, int hidden, int basis, int cutoff, int envelope, float start,
+                             float end, float basis_scale, float w_scale, float act_scale, int act, float* grad_pos,
+                             float* grad_w0, void* scratch, int64_t scratch_bytes, int32_t* status, void* stream);
 
 /*
  * Gate non-linearity on rows (e3nn/nn/_gate.py:127-144: Extract, two Activations of

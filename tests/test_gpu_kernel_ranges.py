@@ -135,3 +135,37 @@ def test_conv_pipelined_permuted_edges(layout, nodes, edges):
     # two fp32 summation orders of rows of up to 60 messages; 2e-5 x RMS as for the sorted form of these kernels
     for a, b in zip(permuted, direct):
         assert rel_err(a.cpu(), b.cpu().double()) < 2e-5
+
+
+# ----------------------------------------------------------------------------- edge embedding: gradient of its weights
+@pytest.mark.parametrize("edges", [1, 33, 4001])
+@pytest.mark.parametrize("act,hidden,nb,with_pos", [("silu", 64, 8, False), ("tanh", 32, 5, True), ("relu", 128, 16, True), ("silu", 96, 9, False)])
+def test_edge_embed_weight_gradient(act, hidden, nb, with_pos, edges):
+    """Against the same chain in fp64; 1e-5 x RMS, the fp32 parity bound of this path."""
+    g = torch.Generator().manual_seed(edges + nb)
+    N, c = 50, 5.0
+    pos = torch.rand(N, 3, generator=g) * 6.0
+    src = torch.randint(0, N, (edges,), generator=g)
+    dst = (src + 1 + torch.randint(0, N - 1, (edges,), generator=g)) % N
+    w0, gh = torch.randn(nb, hidden, generator=g), torch.randn(edges, hidden, generator=g)
+    w_scale, act_scale = nb ** -0.5, bnn.normalize2mom_constant(act)
+    f = {"silu": torch.nn.functional.silu, "tanh": torch.tanh, "relu": torch.relu}[act]
+    p64, w64 = pos.double().requires_grad_(True), w0.double().requires_grad_(True)
+    h64 = act_scale * f(bnn.bessel((p64[src] - p64[dst]).norm(dim=-1), nb, c) @ (w64 * w_scale))
+    ref = torch.autograd.grad(h64, [p64, w64], gh.double())
+
+    pd, wd = pos.to(DEV).requires_grad_(with_pos), w0.to(DEV).requires_grad_(True)
+
+    def embed(weight_grad):
+        return bnn.edge_embed(pd, src.to(DEV), dst.to(DEV), None, wd, c, w_scale, act_scale, act, check_indices=True, weight_grad=weight_grad)
+
+    vec, h = embed(True)
+    assert vec.requires_grad == with_pos
+    got = torch.autograd.grad(h, ([pd] if with_pos else []) + [wd], gh.to(DEV))
+    assert rel_err(got[-1].cpu(), ref[1]) < 1e-5
+    if with_pos:
+        assert rel_err(got[0].cpu(), ref[0]) < 1e-5
+    again = torch.autograd.grad(embed(True)[1], wd, gh.to(DEV))[0]
+    assert torch.equal(again, got[-1])           # fixed summation order
+    with pytest.raises(NotImplementedError):
+        torch.autograd.grad(embed(False)[1], wd, gh.to(DEV))
