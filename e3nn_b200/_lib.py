@@ -59,23 +59,18 @@ def require_cuda(*tensors: torch.Tensor) -> None:
 
 
 # ------------------------------------------------------------------------------------------- kernel status
-# Kernels report conditions they cannot raise themselves through a status word in device memory: 1 = a destination
-# index out of range (CSR builder), 2 = a source / edge index out of range (the access was skipped), 3 = a bounded
-# wait on an mbarrier gave up (the kernel returned early, its output is incomplete).  One word per device lives for
-# the life of the process.  After every launch that can raise it, a 4-byte copy into pinned host memory is enqueued
-# behind the kernel; the next call of any op on that device looks at the copy if it has landed (no
-# synchronisation) and raises; `check_status` synchronises and raises.  A code stays until it is raised once.
+# Kernels report conditions they cannot raise themselves through a status word: 1 = a destination index out of range
+# (CSR builder), 2 = a source / edge index out of range (the access was skipped), 3 = a bounded wait on an mbarrier gave
+# up (the kernel returned early, its output is incomplete).  One word per device lives for the life of the process, in
+# pinned host memory that the device addresses directly: a kernel writes it only when something is wrong, the next call
+# of any op on that device looks at it (no synchronisation) and raises; `check_status` synchronises and raises.  A code
+# stays until it is raised once.  (With the word in device memory a copy and an event followed every launch: nine copies
+# and 0.1 ms of host time in a molecular-dynamics step.)
 class _DeviceStatus:
     def __init__(self, device: torch.device):
         self.device = device
-        self.word = torch.zeros(1, dtype=torch.int32, device=device)
-        self.host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        self.event: Optional[torch.cuda.Event] = None
-
-    def clear(self) -> None:
-        self.word.zero_()
-        self.host.zero_()
-        self.event = None
+        self.word = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.value = c_int32.from_address(self.word.data_ptr())
 
 
 _status: Dict[int, _DeviceStatus] = {}
@@ -85,7 +80,10 @@ def _device_status(device: torch.device) -> _DeviceStatus:
     idx = device.index if device.index is not None else torch.cuda.current_device()
     st = _status.get(idx)
     if st is None:
-        st = _status[idx] = _DeviceStatus(torch.device("cuda", idx))
+        with _core_lock:
+            st = _status.get(idx)
+            if st is None:
+                st = _status[idx] = _DeviceStatus(torch.device("cuda", idx))
     return st
 
 
@@ -105,34 +103,24 @@ def _raise_status(code: int, what: str) -> None:
 
 
 def status_after_launch(device: torch.device) -> None:
-    """Enqueue the read-back of the status word behind the launches made so far on the current stream."""
-    if torch.cuda.is_current_stream_capturing():
-        return
-    st = _device_status(device)
-    with torch.cuda.device(st.device):
-        st.host.copy_(st.word, non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-    st.event = ev
+    """Nothing to enqueue: the kernels write the word in host memory themselves."""
 
 
 def poll_status(device: torch.device, what: str = "an earlier e3nn_b200 kernel") -> None:
-    """Raise if an earlier launch on `device` has reported a condition and its read-back has landed.  Never waits."""
+    """Raise if an earlier launch on `device` has reported a condition.  Never waits."""
     st = _status.get(device.index if device.index is not None else torch.cuda.current_device())
-    if st is None or st.event is None or torch.cuda.is_current_stream_capturing() or not st.event.query():
+    if st is None or st.value.value == 0 or torch.cuda.is_current_stream_capturing():
         return
-    code = int(st.host[0])
-    st.event = None
-    if code != 0:
-        st.clear()
-        _raise_status(code, what)
+    code, st.value.value = st.value.value, 0
+    _raise_status(code, what)
 
 
 def last_status_code(device: Optional[torch.device] = None) -> int:
     """Synchronise `device` (default: the current one) and return its status word without raising or clearing."""
     dev = device if device is not None else torch.device("cuda", torch.cuda.current_device())
     st = _device_status(dev)
-    return int(st.word.item())
+    torch.cuda.synchronize(st.device)
+    return st.value.value
 
 
 def check_status(device: Optional[torch.device] = None, what: str = "e3nn_b200 kernels") -> None:
@@ -140,7 +128,7 @@ def check_status(device: Optional[torch.device] = None, what: str = "e3nn_b200 k
     dev = device if device is not None else torch.device("cuda", torch.cuda.current_device())
     code = last_status_code(dev)
     if code != 0:
-        _device_status(dev).clear()
+        _device_status(dev).value.value = 0
         _raise_status(code, what)
 
 
@@ -371,7 +359,6 @@ class TcGemmModule:
             rc = self.lib.e3b_tc_gemm_fwd(_ptr(x1), _ptr(x2), _ptr(weight), _ptr(out), x1.shape[0], precision,
                                           _ptr(scratch), split, _ptr(status_word(dev)), stream_ptr())
         self.check(rc, "e3b_tc_gemm_fwd")
-        status_after_launch(dev)
         return out
 
     def run_gate(self, x1: torch.Tensor, weight: torch.Tensor, gate_tbl: torch.Tensor, gate_cst: torch.Tensor,
@@ -385,7 +372,6 @@ class TcGemmModule:
                                                gates.shape[1], _ptr(out), out.shape[1], x1.shape[0], precision,
                                                _ptr(scratch), _ptr(status_word(dev)), stream_ptr())
         self.check(rc, "e3b_tc_gemm_fwd_gate")
-        status_after_launch(dev)
         return out
 
 

@@ -59,7 +59,6 @@ class _ConvFunction(torch.autograd.Function):
                                       _lib._ptr(perm), _lib._ptr(weight), _lib._ptr(out), N, node_x.shape[0], E,
                                       scale, _lib._ptr(status), _lib.stream_ptr())
         mod.check(rc, "e3b_conv_fwd")
-        _lib.status_after_launch(node_x.device)
         ctx.save_for_backward(node_x, x2, weight, edge_src, rowptr, perm if perm is not None else torch.empty(0))
         ctx.meta = (mod, in2_mode, scale, perm is not None)
         return out
@@ -80,7 +79,6 @@ class _ConvFunction(torch.autograd.Function):
                                             _lib._ptr(perm) if has_perm else None, _lib._ptr(weight), _lib._ptr(grad_out),
                                             _lib._ptr(gx), N, node_x.shape[0], E, scale, _lib._ptr(st), _lib.stream_ptr())
             mod.check(rc, "e3b_conv_bwd_x")
-            _lib.status_after_launch(node_x.device)
             if not (ctx.needs_input_grad[1] or ctx.needs_input_grad[2]):
                 return gx, None, None, None, None, None, None, None, None
         gw = torch.empty_like(weight)
@@ -92,7 +90,6 @@ class _ConvFunction(torch.autograd.Function):
                                       _lib._ptr(gw), _lib._ptr(gx2), N, node_x.shape[0], E, scale, _lib._ptr(status),
                                       _lib.stream_ptr())
         mod.check(rc, "e3b_conv_bwd")
-        _lib.status_after_launch(node_x.device)
         return gx, gx2, gw, None, None, None, None, None, None
 
 

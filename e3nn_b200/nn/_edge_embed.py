@@ -33,7 +33,6 @@ class _EdgeEmbedFunction(torch.autograd.Function):
                 _lib._ptr(w0), E, N, nb, hidden, *spec, w_scale, act_scale, act, _lib._ptr(edge_vec), _lib._ptr(h),
                 _lib._ptr(status), _lib.stream_ptr())
         _lib.check(rc, "e3b_radial_embed_fwd")
-        _lib.status_after_launch(pos.device)
         ctx.save_for_backward(pos, edge_src, edge_dst, shift if shift is not None else torch.empty(0), w0)
         ctx.meta = (shift is not None, spec, w_scale, act_scale, act, weight_grad)
         ctx.set_materialize_grads(False)
@@ -66,7 +65,6 @@ class _EdgeEmbedFunction(torch.autograd.Function):
                 E, N, nb, hidden, *spec, w_scale, act_scale, act, _lib._ptr(grad_pos), _lib._ptr(grad_w0), _lib._ptr(scratch),
                 scratch.numel() if scratch is not None else 0, _lib._ptr(status), _lib.stream_ptr())
         _lib.check(rc, "e3b_radial_embed_bwd")
-        _lib.status_after_launch(dev)
         return grad_pos, None, None, None, grad_w0, None, None, None, None, None
 
 

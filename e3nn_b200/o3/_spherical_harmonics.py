@@ -6,7 +6,8 @@ Same constructor, attributes, error behaviour and call signature as
 """
 from __future__ import annotations
 
-from typing import Any, List, Union
+from functools import lru_cache
+from typing import Any, List, Tuple, Union
 
 import torch
 
@@ -114,8 +115,18 @@ class SphericalHarmonics(torch.nn.Module):
         return f"{self._ls_list}, normalize={self.normalize}, normalization={self.normalization}"
 
 
+@lru_cache(maxsize=64)
+def _module(l: Union[int, str, Irreps, Tuple[int, ...]], kind: type, normalize: bool, normalization: str) -> SphericalHarmonics:
+    """The (stateless) module of one set of arguments; ``kind`` keeps equal tuples of different types apart."""
+    return SphericalHarmonics(list(l) if kind is list else l, normalize, normalization)
+
+
 def spherical_harmonics(
     l: Union[int, List[int], str, Irreps], x: torch.Tensor, normalize: bool, normalization: str = "integral"
 ) -> torch.Tensor:
     """``e3nn.o3.spherical_harmonics`` (``_spherical_harmonics.py:115-190``) on the GPU."""
+    if type(l) in (int, str, Irreps) and type(normalize) is bool and type(normalization) is str:
+        return _module(l, type(l), normalize, normalization)(x)
+    if type(l) is list and all(type(v) is int for v in l) and type(normalize) is bool and type(normalization) is str:
+        return _module(tuple(l), list, normalize, normalization)(x)
     return SphericalHarmonics(l, normalize, normalization)(x)

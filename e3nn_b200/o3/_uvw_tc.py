@@ -20,7 +20,6 @@ def uvw_tc_forward(tp, x2d: torch.Tensor, y2d: torch.Tensor, w: torch.Tensor, ou
         rc = mod.lib.e3b_uvw_tc_fwd(_lib._ptr(x2d), _lib._ptr(y2d), _lib._ptr(w), _lib._ptr(target), x2d.shape[0], 0,
                                     _lib._ptr(_lib.status_word(out.device)), _lib.stream_ptr())
     mod.check(rc, "e3b_uvw_tc_fwd")
-    _lib.status_after_launch(out.device)
     if accumulate:
         offs = tp.irreps_out.offsets()
         for i_out in tp._uvw_written:

@@ -197,3 +197,17 @@ def test_transposed_linear_swaps_operands_only_where_it_pays():
     assert not any(g.swap for g in small._tc_bwd.groups)          # 64 channels: half an MMA tile
     for g in lin._tc_bwd.groups:
         assert not (g.swap and g.staged_epilogue())
+
+
+def test_spherical_harmonics_module_is_kept_by_its_arguments():
+    """The functional form keeps one module per set of arguments: equal arguments share it, different types do not."""
+    from e3nn_b200 import o3
+    from e3nn_b200.o3._spherical_harmonics import _module
+
+    irreps = o3.Irreps("1x0e+1x1o+1x2e")
+    kept = _module(irreps, o3.Irreps, True, "component")
+    assert kept is _module(o3.Irreps("0e+1o+2e"), o3.Irreps, True, "component")
+    assert kept is not _module(irreps, o3.Irreps, False, "component") and kept is not _module(irreps, o3.Irreps, True, "norm")
+    as_list = _module((0, 1, 2), list, True, "component")
+    assert as_list is not kept and as_list._ls_list == [0, 1, 2] and _module((2, 0), list, True, "component")._ls_list == [2, 0]
+    assert _module(2, int, True, "component")._ls_list == [2] and _module("2e", str, True, "component").irreps_out == o3.Irreps("1x2e")
