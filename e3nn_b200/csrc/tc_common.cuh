@@ -218,6 +218,18 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
                  : "memory");
 }
 
+// Shared memory -> one box of the tensor map (rows and columns past the matrix are not written), as part of the calling
+// thread's bulk group; bulk_wait_read<N>: all but the N latest groups have read their source.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int32_t x, int32_t y, const void* smem_src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(smem_src))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // Host: row-major fp32 matrix [rows, cols] (row stride = cols) as a 2-D tensor map with boxes of
 // box_rows x box_cols, 128-byte swizzle, zero fill outside the matrix.  Returns 0 or a driver error code
 // (-1: the driver entry point is not available).  The driver is reached through the runtime's entry-point
