@@ -194,6 +194,9 @@ def core() -> ctypes.CDLL:
         spec = [c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_float, c_int]
         lib.e3b_radial_embed_fwd.argtypes = [c_void_p] * 5 + [c_int64, c_int64] + spec + [c_void_p, c_void_p, c_void_p, c_void_p]
         lib.e3b_radial_embed_bwd.argtypes = [c_void_p] * 7 + [c_int64, c_int64] + spec + [c_void_p, c_void_p, c_void_p]
+        lib.e3b_matmul_tn_scratch_bytes.argtypes = [c_int64, c_int, c_int]
+        lib.e3b_matmul_tn_scratch_bytes.restype = c_int64
+        lib.e3b_matmul_tn.argtypes = [c_void_p, c_void_p, c_int64, c_int, c_int, c_float, c_void_p, c_void_p, c_int64, c_void_p]
         lib.e3b_radial_embed_scratch_bytes.argtypes = [c_int64, c_int, c_int]
         lib.e3b_radial_embed_scratch_bytes.restype = c_int64
         lib.e3b_radial_embed_bwd_all.argtypes = [c_void_p] * 7 + [c_int64, c_int64] + spec + [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p]
@@ -213,7 +216,7 @@ def core() -> ctypes.CDLL:
         lib.e3b_selftest_bounded_wait.restype = c_int
         for name in ("e3b_sh_fwd", "e3b_sh_bwd", "e3b_csr_from_dst", "e3b_dense_fwd", "e3b_dense_fwd_gate", "e3b_dense_bwd_w", "e3b_dense_bwd_x",
                      "e3b_dense_bwd_x_supported", "e3b_fill_columns",
-                     "e3b_radial_embed_fwd", "e3b_radial_embed_bwd", "e3b_radial_embed_bwd_all", "e3b_neighbor_count", "e3b_neighbor_fill",
+                     "e3b_radial_embed_fwd", "e3b_radial_embed_bwd", "e3b_radial_embed_bwd_all", "e3b_matmul_tn", "e3b_neighbor_count", "e3b_neighbor_fill",
                      "e3b_neighbor_count_rows", "e3b_neighbor_fill_rows",
                      "e3b_gate_fwd", "e3b_gate_fwd_channels", "e3b_gate_bwd"):
             getattr(lib, name).restype = c_int

@@ -45,8 +45,8 @@ def bessel(x: torch.Tensor, n: int, x_max: float = 1.0) -> torch.Tensor:
 
 class _ScaledMatmul(torch.autograd.Function):
     """``scale * x @ W`` on the tensor cores (hi/lo-split tf32 operands).  The gradient w.r.t. ``x`` is the
-    transposed module; the gradient w.r.t. ``W`` (``scale * x^T g``, a plain [h_in, rows] x [rows, h_out] product
-    needed only in training) is a library fp32 GEMM."""
+    transposed module; the gradient w.r.t. ``W`` (``scale * x^T g``, needed only in training) stays in fp32
+    (``e3b_matmul_tn``)."""
 
     @staticmethod
     def forward(ctx, x, weight, fwd_spec, bwd_spec, scale):
@@ -66,7 +66,14 @@ class _ScaledMatmul(torch.autograd.Function):
             gx = torch.empty(grad_out.shape[0], weight.shape[0], dtype=torch.float32, device=grad_out.device)
             _lib.tc_gemm_module(ctx.bwd_spec).run(grad_out, None, weight, gx, 2)
         if ctx.needs_input_grad[1]:
-            gw = (x.t() @ grad_out) * ctx.scale
+            core, dev = _lib.core(), grad_out.device
+            (h_in, h_out), rows = weight.shape, grad_out.shape[0]
+            gw = torch.empty(h_in, h_out, dtype=torch.float32, device=dev)
+            scratch = torch.empty(core.e3b_matmul_tn_scratch_bytes(rows, h_in, h_out), dtype=torch.uint8, device=dev)
+            with torch.cuda.device(dev), _lib.nvtx_range("e3b_matmul_tn"):
+                rc = core.e3b_matmul_tn(_lib._ptr(x), _lib._ptr(grad_out), rows, h_in, h_out, ctx.scale, _lib._ptr(gw),
+                                        _lib._ptr(scratch), scratch.numel(), _lib.stream_ptr())
+            _lib.check(rc, "e3b_matmul_tn")
         return gx, gw, None, None, None
 
 

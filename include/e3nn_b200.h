@@ -172,6 +172,15 @@ int e3b_radial_embed_bwd_all(const float* pos, const int64_t* edge_src, const in
                              float* grad_w0, void* scratch, int64_t scratch_bytes, int32_t* status, void* stream);
 
 /*
+ * Weight gradient of a dense layer (autograd of e3nn/nn/_fc.py:38-48): out[m, n] = scale * sum_z x[z, m] g[z, n] in fp32,
+ * x [rows, m] and g [rows, n] row-major, out [m, n] overwritten; summed in a fixed order.  scratch: at least
+ * e3b_matmul_tn_scratch_bytes(rows, m, n) bytes (may be NULL when that is 0).
+ */
+int64_t e3b_matmul_tn_scratch_bytes(int64_t rows, int m, int n);
+int e3b_matmul_tn(const float* x, const float* g, int64_t rows, int m, int n, float scale, float* out, void* scratch,
+                  int64_t scratch_bytes, void* stream);
+
+/*
  * Gate non-linearity on rows (e3nn/nn/_gate.py:127-144: Extract, two Activations of
  * e3nn/nn/_activation.py:80-98 and the scalar-gate ElementwiseTensorProduct, fused):
  *   out[z, j] = c_j * act_j(x[z, src_j])                      for scalar outputs,

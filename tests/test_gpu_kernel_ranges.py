@@ -169,3 +169,28 @@ def test_edge_embed_weight_gradient(act, hidden, nb, with_pos, edges):
     assert torch.equal(again, got[-1])           # fixed summation order
     with pytest.raises(NotImplementedError):
         torch.autograd.grad(embed(False)[1], wd, gh.to(DEV))
+
+
+# ----------------------------------------------------------------------------- weight gradient of a dense layer
+@pytest.mark.parametrize("rows,m,n,offset", [(1, 32, 16, 0), (63, 64, 144, 0), (1025, 96, 1472, 0), (20_011, 64, 128, 1), (777, 33, 130, 0)])
+def test_dense_layer_weight_gradient(rows, m, n, offset):
+    """64 x 128 tiles, stages of 16 rows, splits; `offset` floats in front of the operands (no 16-byte loads).  Bound: the random
+    walk of the roundings of runs of at most 2,048 rows, 2^-24 sqrt(rows of a run), relative to the sums' size."""
+    from e3nn_b200 import _lib
+
+    g = torch.Generator().manual_seed(rows)
+    x, go = torch.randn(rows, m, generator=g), torch.randn(rows, n, generator=g)
+    ref = 0.5 * (x.double().t() @ go.double())
+    xd, gd = torch.empty(offset + rows * m, device=DEV), torch.empty(offset + rows * n, device=DEV)
+    xd[offset:], gd[offset:] = x.to(DEV).view(-1), go.to(DEV).view(-1)
+    core, out = _lib.core(), torch.empty(m, n, device=DEV)
+    need = core.e3b_matmul_tn_scratch_bytes(rows, m, n)
+    scratch = torch.empty(max(need, 1), dtype=torch.uint8, device=DEV)
+    args = (_lib._ptr(xd[offset:]), _lib._ptr(gd[offset:]), rows, m, n, 0.5, _lib._ptr(out), _lib._ptr(scratch))
+    assert core.e3b_matmul_tn(*args, need, _lib.stream_ptr()) == 0
+    err = (out.cpu().double() - ref).norm() / ref.norm()
+    assert err < 2.0**-24 * (4 + min(rows, 2048) ** 0.5), err
+    first = out.clone()
+    assert core.e3b_matmul_tn(*args, need, _lib.stream_ptr()) == 0 and torch.equal(out, first)
+    if need > 0:
+        assert core.e3b_matmul_tn(*args, need - 1, _lib.stream_ptr()) == -1
