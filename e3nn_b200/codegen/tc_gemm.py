@@ -262,7 +262,7 @@ def matmul_gemm_spec(k: int, n: int, transpose: bool, scale: float, key: str) ->
     """``out[z, :] = scale * x[z, :] @ W`` with ``W`` row-major ``[k, n]`` (or, transposed, ``g @ W^T``):
     the dense layers of the radial network.  Wide outputs are cut into column tiles of at most 256."""
     if transpose:
-        if n % 32 != 0 or k % 16 != 0 or not (16 <= k <= 256):
+        if n % 32 != 0 or k % 32 != 0 or not (32 <= k <= 256):
             return None
         g = Group(0, k, 1)
         g.cases.append("vals[0] = xi[q][0];")
@@ -274,7 +274,7 @@ def matmul_gemm_spec(k: int, n: int, transpose: bool, scale: float, key: str) ->
         groups = [g]
         d_in, d_out = n, k
     else:
-        if k % 32 != 0 or n % 16 != 0:
+        if k % 32 != 0 or n % 32 != 0:
             return None
         groups = []
         col = 0
@@ -561,47 +561,38 @@ for (int q = 0; q < {qn}; ++q) {{{{
                     for (int j = 0; j < 16; ++j) orow[(w0 + j) * DIM + kq] = __uint_as_float(r[j]);
                     }"""
         if g.plain:
-            def block(cols: int) -> str:      # (16 columns: the last block of the last group, the store stops at the row's end)
-                ld = "tc::tmem_ld32" if cols == 32 else "tc::tmem_ld16"
-                return f"""uint8_t* buf = se + (stores & 1) * 4096;
-if (lane == 0) tc::bulk_wait_read<1>();      // the store before the last has read this buffer
-__syncwarp();
-uint32_t r[{cols}];
-{ld}(tbase + wb, r);
-if (nparts == 1) tc::tmem_ld_wait();
-for (int p = 1; p < nparts; ++p) {{   // further partial accumulators: summed here in fp32
-    uint32_t q[{cols}];
-    {ld}(tbase + part_off(p) + wb, q);
-    tc::tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < {cols}; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(q[j]));
-}}
-#pragma unroll
-for (int c = 0; c < {cols // 4}; ++c)
-    *reinterpret_cast<float4*>(buf + lane * 128 + ((c ^ (lane & 7)) << 4)) =
-        make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]), __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
-tc::fence_proxy_async_smem();
-__syncwarp();
-if (lane == 0) {{
-    if (row0 < Z) tc::tma_store_2d(tmap_out, OUT_OFF + wb, static_cast<int32_t>(row0), buf);
-    tc::bulk_commit();
-}}
-++stores;"""
-            full = g.n // 32 * 32
+            assert g.n % 32 == 0
             EPILOGUE = f"""            // 32 columns at a time: registers -> one of this warp's two buffers (rows of 128 bytes, 16-byte pieces
             // XOR-swizzled by row) -> a bulk tensor store of 32 x 32, which runs while the next block is read.  With
             // the warps' own loads and stores in its place the epilogue was the limit of the 64 -> 1472 layer: 6.86 million
             // rows (40 GB written) 11.3 -> 7.5 ms, 429,000 rows 644 -> 487 us.
             const int64_t row0 = t * ZT + warp * 32;
             uint8_t* se = reinterpret_cast<uint8_t*>(sE) + warp * 8192;
-            for (int wb = 0; wb < {full}; wb += 32) {{
-{_indent(block(32), 16)}
-            }}"""
-            if g.n % 32:
-                EPILOGUE += f"""
-            {{
-                const int wb = {full};
-{_indent(block(16), 16)}
+            for (int wb = 0; wb < N; wb += 32) {{
+                uint8_t* buf = se + (stores & 1) * 4096;
+                if (lane == 0) tc::bulk_wait_read<1>();      // the store before the last has read this buffer
+                __syncwarp();
+                uint32_t r[32];
+                tc::tmem_ld32(tbase + wb, r);
+                if (nparts == 1) tc::tmem_ld_wait();
+                for (int p = 1; p < nparts; ++p) {{   // further partial accumulators: summed here in fp32
+                    uint32_t q[32];
+                    tc::tmem_ld32(tbase + part_off(p) + wb, q);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(q[j]));
+                }}
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<float4*>(buf + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+                        make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]), __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
+                tc::fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {{
+                    if (row0 < Z) tc::tma_store_2d(tmap_out, OUT_OFF + wb, static_cast<int32_t>(row0), buf);
+                    tc::bulk_commit();
+                }}
+                ++stores;
             }}"""
         elif g.staged_epilogue():
             EPILOGUE = f"""            // 64 columns at a time: registers -> this warp's staging tile (16-byte chunks XOR-swizzled by row,

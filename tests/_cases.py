@@ -1,7 +1,7 @@
 """Layouts used by the GPU property tests (seeded, so they can be pre-built without a GPU)."""
 import random
 
-from e3nn_b200 import layouts, o3
+from e3nn_b200 import _lib, layouts, nn, o3
 
 
 def random_conv_layouts(n=4, seed=0):
@@ -53,6 +53,8 @@ def prebuild():
         for mode in ("tf32", "tf32x3"):
             pb._build_tp(o3.FullyConnectedTensorProduct(*layout, math_mode=mode)._vjp_module(0))
     pb._build_linear(o3.Linear("64x0e+64x1o+64x2e+64x3o", "256x0e+64x1o+64x2e+64x3o", math_mode="tf32x3"))   # Linear -> Gate
+    for gs in nn.FullyConnectedNet([64, 96], math_mode="tf32x3").layer0._tc_specs():      # one column group of 96
+        _lib.tc_gemm_module(gs)
     pb._build_linear(o3.Linear("16x0e+8x1o+4x2e", "8x0e+8x1o+4x2e"))
     pb._build_linear(o3.Linear("64x0e+32x1o+32x2e", "32x0e+64x1o+32x2e"))
     for mode in ("fp32", "tf32x3", "tf32"):

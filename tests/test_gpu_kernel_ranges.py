@@ -194,3 +194,24 @@ def test_dense_layer_weight_gradient(rows, m, n, offset):
     assert core.e3b_matmul_tn(*args, need, _lib.stream_ptr()) == 0 and torch.equal(out, first)
     if need > 0:
         assert core.e3b_matmul_tn(*args, need - 1, _lib.stream_ptr()) == -1
+
+
+# ----------------------------------------------------------------------------- dense layers on tensor cores
+@pytest.mark.parametrize("rows", [1, 33, 127, 1000])
+@pytest.mark.parametrize("width", [96, 1472])
+def test_dense_layer_tiles(width, rows):
+    """128-row tiles whose output leaves in boxes of 32 x 32: the last box ends with the rows.  The output lies between guard
+    rows that must keep their values.  Bound: 4e-5 x RMS, the split-operand bound of this path."""
+    from e3nn_b200 import _lib
+
+    g = torch.Generator().manual_seed(rows)
+    layer = bnn.FullyConnectedNet([64, width], math_mode="tf32x3").layer0
+    w = torch.randn(64, width, generator=g)
+    for transpose, gs in enumerate(layer._tc_specs()):
+        a, b = (w, layer._scale()) if not transpose else (w.t(), layer._scale())
+        x = torch.randn(rows, a.shape[0], generator=g)
+        buf = torch.full((rows + 2, a.shape[1]), 7.0, device=DEV)
+        _lib.tc_gemm_module(gs).run(x.to(DEV), None, w.to(DEV), buf[1 : rows + 1], 2)
+        e3nn_b200.check_status()
+        assert torch.all(buf[0] == 7.0) and torch.all(buf[-1] == 7.0)
+        assert rel_err(buf[1 : rows + 1].cpu(), b * (x.double() @ a.double())) < 4e-5
