@@ -23,6 +23,7 @@ namespace {
 
 constexpr int kMaxBasis = 16;
 constexpr int kEmbedWarps = 8;
+constexpr int kLaneWarps = 4;
 
 enum Act { kSilu = 0, kTanh = 1, kRelu = 2, kIdentity = 3 };
 
@@ -236,8 +237,8 @@ __device__ __forceinline__ void halve(float* v, int lane) {
     }
 }
 
-// GP: position gradient (grad_vec is read too); GW: partial weight gradients, partial[block][nb * H] (without w_scale).
-template <int H2, int NB, bool GP, bool GW>
+// Partial weight gradients, partial[block][nb * H] (without w_scale), and with GP the position gradient (grad_vec is read too).
+template <int H2, int NB, bool GP>
 __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
         const float* __restrict__ pos, const int64_t* __restrict__ src, const int64_t* __restrict__ dst,
         const float* __restrict__ shift, const float* __restrict__ w0, const float* __restrict__ grad_h,
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
     __shared__ float s_basis[kEmbedWarps][32][kMaxBasis + 1];
     __shared__ float s_cot[GP ? kEmbedWarps : 1][32][kMaxBasis + 1];
     __shared__ float s_env[kEmbedWarps][32];     // envelope value of the batch's edges
-    __shared__ float s_gw[GW ? NB * 32 * H2 : 1];
+    __shared__ float s_gw[NB * 32 * H2];
     __shared__ float s_genv[kEmbedWarps][32];    // cotangent of the envelope
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = sp.nb;
@@ -256,13 +257,11 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
     for (int k = 0; k < NB; ++k)
 #pragma unroll
         for (int j = 0; j < H2; ++j) w[k][j] = k < nb ? w0[k * H + lane + 32 * j] * w_scale : 0.0f;
-    float gw[GW ? NB : 1][GW ? H2 : 1];
-    if (GW) {
+    float gw[NB][H2];
 #pragma unroll
-        for (int k = 0; k < NB; ++k)
+    for (int k = 0; k < NB; ++k)
 #pragma unroll
-            for (int j = 0; j < H2; ++j) gw[GW ? k : 0][GW ? j : 0] = 0.0f;
-    }
+        for (int j = 0; j < H2; ++j) gw[k][j] = 0.0f;
     const int64_t batches = (num_edges + 31) / 32;
     for (int64_t b = static_cast<int64_t>(blockIdx.x) * kEmbedWarps + warp; b < batches;
          b += static_cast<int64_t>(gridDim.x) * kEmbedWarps) {
@@ -317,11 +316,9 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
 #pragma unroll
                     for (int k = 0; k < NB; ++k) cot[k] = fmaf(w[k][j], dpre, cot[k]);
                 }
-                if (GW) {
 #pragma unroll
-                    for (int k = 0; k < NB; ++k)
-                        if (k < nb) gw[GW ? k : 0][GW ? j : 0] = fmaf(s_basis[warp][i][k], dpre, gw[GW ? k : 0][GW ? j : 0]);
-                }
+                for (int k = 0; k < NB; ++k)
+                    if (k < nb) gw[k][j] = fmaf(s_basis[warp][i][k], dpre, gw[k][j]);
             }
             if (!GP) continue;
             if (NB == 16) {
@@ -359,21 +356,19 @@ __global__ void __launch_bounds__(kEmbedWarps * 32) radial_embed_bwd_kernel(
         }
         __syncwarp();
     }
-    if (GW) {
-        for (int q = 0; q < kEmbedWarps; ++q) {
-            if (warp == q) {
+    for (int q = 0; q < kEmbedWarps; ++q) {
+        if (warp == q) {
 #pragma unroll
-                for (int k = 0; k < NB; ++k)
+            for (int k = 0; k < NB; ++k)
 #pragma unroll
-                    for (int j = 0; j < H2; ++j) {
-                        float* at = s_gw + (k * H + lane + 32 * j);
-                        *at = (q > 0 ? *at : 0.0f) + gw[GW ? k : 0][GW ? j : 0];
-                    }
-            }
-            __syncthreads();
+                for (int j = 0; j < H2; ++j) {
+                    float* at = s_gw + (k * H + lane + 32 * j);
+                    *at = (q > 0 ? *at : 0.0f) + gw[k][j];
+                }
         }
-        for (int c = threadIdx.x; c < nb * H; c += kEmbedWarps * 32) partial[static_cast<int64_t>(blockIdx.x) * nb * H + c] = s_gw[c];
+        __syncthreads();
     }
+    for (int c = threadIdx.x; c < nb * H; c += kEmbedWarps * 32) partial[static_cast<int64_t>(blockIdx.x) * nb * H + c] = s_gw[c];
 }
 
 // grad_w0[c] = w_scale * sum over the blocks of partial[block][c]: 32 columns a block, 32 warps over the rows.
@@ -392,6 +387,108 @@ __global__ void __launch_bounds__(1024) radial_embed_weight_sum_kernel(const flo
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0 && blockIdx.x * 32 + warp < cols) grad_w0[blockIdx.x * 32 + warp] = w_scale * v;
+}
+
+// Position gradient alone, one lane per edge from start to end: the basis and its cotangent stay in the lane's registers,
+// the layer's weights are read from shared memory by all lanes at once, and 32 hidden units of the 32 cotangent rows are
+// transposed through shared memory at a time.  About 80 instructions an edge; with the hidden units across the lanes (the
+// kernel above, which the weight gradient needs) every edge reads the basis from shared memory and reduces its cotangent
+// over the lanes, about 330.  Neighbouring lanes with the same destination are summed before the atomic additions.
+// 6.86 million edges 2.2 -> 1.64 ms, 105,000 edges 48 -> 36 us, 6,600 edges 22 -> 15 us (64 hidden units, silu).
+template <int NB, int ACT>
+__global__ void __launch_bounds__(kLaneWarps * 32) radial_embed_bwd_pos_kernel(
+        const float* __restrict__ pos, const int64_t* __restrict__ src, const int64_t* __restrict__ dst,
+        const float* __restrict__ shift, const float* __restrict__ w0, const float* __restrict__ grad_h,
+        const float* __restrict__ grad_vec, int64_t num_edges, int64_t num_nodes, RadialSpec sp, int hidden, float w_scale,
+        float act_scale, float* __restrict__ grad_pos, int* __restrict__ status) {
+    __shared__ __align__(16) float s_w[128 * NB];               // [unit][k], scaled
+    __shared__ float s_gh[kLaneWarps][32][33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = sp.nb;
+    for (int i = threadIdx.x; i < hidden * NB; i += kLaneWarps * 32) {
+        const int j = i / NB, k = i % NB;
+        s_w[i] = k < nb ? w0[k * hidden + j] * w_scale : 0.0f;
+    }
+    __syncthreads();
+    float(*gh)[33] = s_gh[warp];
+    const int64_t batches = (num_edges + 31) / 32;
+    for (int64_t b = static_cast<int64_t>(blockIdx.x) * kLaneWarps + warp; b < batches; b += static_cast<int64_t>(gridDim.x) * kLaneWarps) {
+        const int64_t e = b * 32 + lane;
+        const int count = static_cast<int>(num_edges - b * 32 < 32 ? num_edges - b * 32 : 32);
+        const bool live = lane < count;
+        EdgeGeom g;
+        g.vx = g.vy = g.vz = 0.0f; g.r = 0.0; g.s = g.d = -1;
+        float basis[kMaxBasis], dbasis[kMaxBasis], env = 1.0f, denv = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kMaxBasis; ++k) basis[k] = dbasis[k] = 0.0f;
+        if (live) {
+            g = edge_geom(pos, src, dst, shift, e, num_nodes, status);
+            radial_basis(sp, g.r, basis, dbasis);
+            radial_envelope(sp, g.r, env, denv);
+        }
+        const float scale = env * act_scale;
+        float cot[NB], genv = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NB; ++k) cot[k] = 0.0f;
+        for (int j0 = 0; j0 < hidden; j0 += 32) {
+            const float* rows = grad_h + b * 32 * hidden + j0 + lane;
+#pragma unroll 16
+            for (int i = 0; i < 32; ++i) gh[i][lane] = i < count ? __ldg(rows + static_cast<int64_t>(i) * hidden) : 0.0f;
+            __syncwarp();
+#pragma unroll 1
+            for (int j = 0; j < 32; j += 8) {
+                // eight units in accumulators of their own (rounding as in a tree)
+                float part[NB];
+#pragma unroll
+                for (int k = 0; k < NB; ++k) part[k] = 0.0f;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float4* wq = reinterpret_cast<const float4*>(s_w + (j0 + j + u) * NB);
+                    float w[NB], pre = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < NB; k += 4) {
+                        const float4 t = wq[k / 4];
+                        w[k] = t.x; w[k + 1] = t.y; w[k + 2] = t.z; w[k + 3] = t.w;
+                    }
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) pre = fmaf(basis[k], w[k], pre);
+                    const float gv = gh[lane][j + u];
+                    if (sp.envelope) genv = fmaf(gv * act_scale, act_fwd(ACT, pre), genv);
+                    const float dpre = gv * scale * act_grad(ACT, pre);
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) part[k] = fmaf(w[k], dpre, part[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < NB; ++k) cot[k] += part[k];
+            }
+            __syncwarp();
+        }
+        float gx = 0.0f, gy = 0.0f, gz = 0.0f;
+        if (live) {
+            double dr = sp.envelope ? static_cast<double>(genv) * denv : 0.0;
+#pragma unroll
+            for (int k = 0; k < NB; ++k)
+                if (k < nb) dr += static_cast<double>(cot[k]) * dbasis[k];
+            if (grad_vec) { gx = grad_vec[e * 3]; gy = grad_vec[e * 3 + 1]; gz = grad_vec[e * 3 + 2]; }
+            if (g.r > 0.0) {
+                const double f = dr / g.r;
+                gx += static_cast<float>(f * g.vx); gy += static_cast<float>(f * g.vy); gz += static_cast<float>(f * g.vz);
+            }
+            atomicAdd(grad_pos + g.s * 3, gx); atomicAdd(grad_pos + g.s * 3 + 1, gy); atomicAdd(grad_pos + g.s * 3 + 2, gz);
+        }
+        // runs of lanes with one destination: the first lane of a run adds the run's sum
+        const long long before = __shfl_up_sync(0xffffffffu, static_cast<long long>(g.d), 1);
+        const bool head = lane == 0 || before != g.d;
+        const unsigned heads = __ballot_sync(0xffffffffu, head);
+        const int end = (lane < 31 && (heads >> (lane + 1)) != 0u) ? lane + __ffs(heads >> (lane + 1)) : 32;   // first lane past the run
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float ux = __shfl_down_sync(0xffffffffu, gx, o), uy = __shfl_down_sync(0xffffffffu, gy, o), uz = __shfl_down_sync(0xffffffffu, gz, o);
+            if (lane + o < end) { gx += ux; gy += uy; gz += uz; }
+        }
+        if (head && live) {
+            atomicAdd(grad_pos + g.d * 3, -gx); atomicAdd(grad_pos + g.d * 3 + 1, -gy); atomicAdd(grad_pos + g.d * 3 + 2, -gz);
+        }
+    }
 }
 
 int check_embed_args(int64_t num_edges, int64_t num_nodes, int num_basis, int hidden, int act) {
@@ -477,13 +574,30 @@ int embed_bwd(const float* pos, const int64_t* edge_src, const int64_t* edge_dst
     if (grad_w0 && (!scratch || scratch_bytes < static_cast<int64_t>(sizeof(float)) * grid * cols))
         return fail(E3B_ERR_ARG, "radial_embed_bwd: scratch too small");
     float* partial = static_cast<float*>(scratch);
-#define E3B_LAUNCH(H2, NBP, GP, GW)                                                                                          \
-    radial_embed_bwd_kernel<H2, NBP, GP, GW><<<grid, threads, 0, s>>>(pos, edge_src, edge_dst, shift, w0, grad_h, grad_edge_vec, \
-                                                                      num_edges, num_nodes, sp, w_scale, act_scale, act, grad_pos, partial, status)
+    if (!grad_w0) {
+        const int64_t want = ceil_div(ceil_div(num_edges, 32), kLaneWarps), cap = static_cast<int64_t>(kNumSMs) * 16;
+        const int blocks = static_cast<int>(want < cap ? want : cap);
+#define E3B_LAUNCH(NBP, ACT)                                                                                                 \
+    radial_embed_bwd_pos_kernel<NBP, ACT><<<blocks, kLaneWarps * 32, 0, s>>>(pos, edge_src, edge_dst, shift, w0, grad_h, grad_edge_vec, \
+                                                                             num_edges, num_nodes, sp, hidden, w_scale, act_scale, grad_pos, status)
+#define E3B_LAUNCH_ACT(ACT)                                                                                                  \
+    if (num_basis <= 8) { E3B_LAUNCH(8, ACT); } else { E3B_LAUNCH(16, ACT); }
+        switch (act) {
+            case kSilu: E3B_LAUNCH_ACT(kSilu) break;
+            case kTanh: E3B_LAUNCH_ACT(kTanh) break;
+            case kRelu: E3B_LAUNCH_ACT(kRelu) break;
+            default: E3B_LAUNCH_ACT(kIdentity) break;
+        }
+#undef E3B_LAUNCH
+#undef E3B_LAUNCH_ACT
+        return check_launch("radial_embed_bwd");
+    }
+#define E3B_LAUNCH(H2, NBP, GP)                                                                                              \
+    radial_embed_bwd_kernel<H2, NBP, GP><<<grid, threads, 0, s>>>(pos, edge_src, edge_dst, shift, w0, grad_h, grad_edge_vec,   \
+                                                                  num_edges, num_nodes, sp, w_scale, act_scale, act, grad_pos, partial, status)
 #define E3B_LAUNCH_G(H2, NBP)                                                                                                \
-    if (!grad_w0) E3B_LAUNCH(H2, NBP, true, false);                                                                          \
-    else if (grad_pos) E3B_LAUNCH(H2, NBP, true, true);                                                                      \
-    else E3B_LAUNCH(H2, NBP, false, true)
+    if (grad_pos) E3B_LAUNCH(H2, NBP, true);                                                                                 \
+    else E3B_LAUNCH(H2, NBP, false)
 #define E3B_LAUNCH_H(H2)                                                                                                     \
     if (num_basis <= 8) { E3B_LAUNCH_G(H2, 8); } else { E3B_LAUNCH_G(H2, 16); }
     switch (hidden / 32) {
@@ -495,7 +609,7 @@ int embed_bwd(const float* pos, const int64_t* edge_src, const int64_t* edge_dst
 #undef E3B_LAUNCH
 #undef E3B_LAUNCH_G
 #undef E3B_LAUNCH_H
-    if (grad_w0) radial_embed_weight_sum_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, grid, cols, w_scale, grad_w0);
+    radial_embed_weight_sum_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, grid, cols, w_scale, grad_w0);
     return check_launch("radial_embed_bwd");
 }
 }  // namespace
