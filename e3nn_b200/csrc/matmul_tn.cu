@@ -1,12 +1,12 @@
 // out[m, n] = scale * sum_z x[z, m] g[z, n] in fp32: the weight gradient of a dense layer (many rows z, a narrow x).
 //
 // Bound by the FP32 pipe: 64 x 1472 entries over 429,000 rows are 81 GFLOP, 1.1 ms at 148 x 128 multiply-adds a clock, while
-// the rows are 2.6 GB, 0.4 ms.  A block owns 64 x 128 entries, 8 x 8 a thread, which read 4 x 16 bytes of shared memory for 32
+// the rows are 2.6 GB, 0.4 ms.  A block owns 64 x 256 entries, 8 x 16 a thread, which read 6 x 16 bytes of shared memory for 64
 // packed multiply-adds (FFMA2: half the issue slots); rows arrive by cp.async four stages ahead.  The rows are split over
-// whole waves of three blocks per SM, at most 2,048 rows a block, and a second kernel adds the partial matrices in a fixed
-// order: the error stays below that of the library's fp32 product, which sums longer runs (429,000 rows: 8.4e-7 against 1.7e-6).
-// Against that product, 64 x 1472: 5,000 rows 51 -> 39 us, 15,600 127 -> 76, 105,000 500 -> 419, 429,000 1690 -> 1609.  FFMA in
-// place of FFMA2 is 5 - 10 % slower, two blocks with accumulators per 64 rows (3.5e-7) 25 %.
+// whole waves, at most 2,048 rows a block, and a second kernel adds the partial matrices in a fixed order: the error stays
+// below that of the library's fp32 product, which sums longer runs (429,000 rows: 8.1e-7 against 1.7e-6).
+// Against that product, 64 x 1472: 5,000 rows 51 -> 35 us, 15,600 127 -> 71, 105,000 500 -> 404, 429,000 1690 -> 1582.  With
+// 8 x 8 a thread 39, 76, 419 and 1609 us; FFMA in place of FFMA2 is 5 - 10 % slower than that.
 #include "common.cuh"
 
 #include <algorithm>
@@ -14,10 +14,11 @@
 namespace e3b {
 namespace {
 
-constexpr int kTnM = 64, kTnN = 128, kTnRows = 16, kTnStages = 4, kTnThreads = 128;
-constexpr int kTnBlocks = 3;              // blocks an SM holds
+constexpr int kTnM = 64, kTnRows = 16, kTnStages = 4, kTnThreads = 128;
 constexpr int64_t kTnMostRows = 2048;     // rows of a block, up to eight waves
-constexpr int kTnStageFloats = kTnRows * (kTnM + kTnN);
+
+template <int TN>
+__host__ __device__ constexpr int tn_stage_floats() { return kTnRows * (kTnM + TN); }
 
 template <int BYTES>
 __device__ __forceinline__ void tn_copy(float* dst, const float* src, bool live) {
@@ -26,11 +27,11 @@ __device__ __forceinline__ void tn_copy(float* dst, const float* src, bool live)
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(live ? 4 : 0) : "memory");
 }
 
-// VEC: widths are multiples of 4 and both bases 16-byte aligned
-template <bool VEC>
+// TN: columns of a block, 128 or 256.  VEC: widths are multiples of 4 and both bases 16-byte aligned
+template <int TN, bool VEC>
 __device__ __forceinline__ void tn_fetch(float* sx, float* sg, const float* __restrict__ x, const float* __restrict__ g, int64_t z0,
                                          int64_t z_end, int m0, int n0, int M, int N) {
-    constexpr int V = VEC ? 4 : 1, QX = kTnM / V, QG = kTnN / V;
+    constexpr int V = VEC ? 4 : 1, QX = kTnM / V, QG = TN / V;
 #pragma unroll 4
     for (int i = threadIdx.x; i < kTnRows * QX; i += kTnThreads) {
         const int r = i / QX, c = (i % QX) * V;
@@ -41,27 +42,28 @@ __device__ __forceinline__ void tn_fetch(float* sx, float* sg, const float* __re
     for (int i = threadIdx.x; i < kTnRows * QG; i += kTnThreads) {
         const int r = i / QG, c = (i % QG) * V;
         const bool live = z0 + r < z_end && n0 + c < N;
-        tn_copy<4 * V>(sg + r * kTnN + c, live ? g + (z0 + r) * N + n0 + c : g, live);
+        tn_copy<4 * V>(sg + r * TN + c, live ? g + (z0 + r) * N + n0 + c : g, live);
     }
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(kTnThreads, kTnBlocks) matmul_tn_kernel(const float* __restrict__ x, const float* __restrict__ g, int64_t Z, int M,
+template <int TN, bool VEC>
+__global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kernel(const float* __restrict__ x, const float* __restrict__ g, int64_t Z, int M,
                                                                   int N, int64_t rows_per_split, float scale, float* __restrict__ out) {
     extern __shared__ __align__(16) float smem[];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int n0 = blockIdx.x * kTnN, m0 = blockIdx.y * kTnM;
+    constexpr int NP = TN / 32;             // pairs of columns a thread owns: 4 columns of every 64
+    const int n0 = blockIdx.x * TN, m0 = blockIdx.y * kTnM;
     const int64_t z_begin = static_cast<int64_t>(blockIdx.z) * rows_per_split;
     const int64_t z_end = z_begin + rows_per_split < Z ? z_begin + rows_per_split : Z;
     const int64_t steps = (z_end - z_begin + kTnRows - 1) / kTnRows;
-    float2 acc[8][4];
+    float2 acc[8][NP];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+        for (int j = 0; j < NP; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
     auto fetch = [&](int64_t step) {
-        float* s = smem + (step % kTnStages) * kTnStageFloats;
-        if (step < steps) tn_fetch<VEC>(s, s + kTnRows * kTnM, x, g, z_begin + step * kTnRows, z_end, m0, n0, M, N);
+        float* s = smem + (step % kTnStages) * tn_stage_floats<TN>();
+        if (step < steps) tn_fetch<TN, VEC>(s, s + kTnRows * kTnM, x, g, z_begin + step * kTnRows, z_end, m0, n0, M, N);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     for (int s = 0; s < kTnStages - 1; ++s) fetch(s);
@@ -69,20 +71,24 @@ __global__ void __launch_bounds__(kTnThreads, kTnBlocks) matmul_tn_kernel(const 
         asm volatile("cp.async.wait_group %0;" ::"n"(kTnStages - 2) : "memory");
         __syncthreads();            // this stage has landed for everyone; the stage fetched next is free
         fetch(step + kTnStages - 1);
-        const float* sx = smem + (step % kTnStages) * kTnStageFloats;
+        const float* sx = smem + (step % kTnStages) * tn_stage_floats<TN>();
         const float* sg = sx + kTnRows * kTnM;
 #pragma unroll
         for (int k = 0; k < kTnRows; ++k) {
             const float4 a0 = *reinterpret_cast<const float4*>(sx + k * kTnM + ty * 4);
             const float4 a1 = *reinterpret_cast<const float4*>(sx + k * kTnM + 32 + ty * 4);
-            const float4 b0 = *reinterpret_cast<const float4*>(sg + k * kTnN + tx * 4);
-            const float4 b1 = *reinterpret_cast<const float4*>(sg + k * kTnN + 64 + tx * 4);
             const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float2 b[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
+            float2 b[NP];
+#pragma unroll
+            for (int j = 0; j < NP / 2; ++j) {
+                const float4 v = *reinterpret_cast<const float4*>(sg + k * TN + 64 * j + tx * 4);
+                b[2 * j] = make_float2(v.x, v.y);
+                b[2 * j + 1] = make_float2(v.z, v.w);
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
+                for (int j = 0; j < NP; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
         }
     }
     float* o = out + static_cast<int64_t>(blockIdx.z) * M * N;
@@ -91,7 +97,7 @@ __global__ void __launch_bounds__(kTnThreads, kTnBlocks) matmul_tn_kernel(const 
         const int m = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < NP; ++j) {
             const int n = n0 + (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
             if (n < N) o[static_cast<int64_t>(m) * N + n] = scale * acc[i][j].x;
             if (n + 1 < N) o[static_cast<int64_t>(m) * N + n + 1] = scale * acc[i][j].y;
@@ -109,14 +115,18 @@ __global__ void __launch_bounds__(256) matmul_tn_sum_kernel(const float* __restr
     out[i] = scale * v;
 }
 
-struct TnPlan { int64_t rows; int splits, tiles_m, tiles_n; };
+struct TnPlan { int64_t rows; int splits, tiles_m, tiles_n, tn; };
 
 TnPlan tn_plan(int64_t Z, int M, int N) {
     TnPlan p;
     p.tiles_m = (M + kTnM - 1) / kTnM;
-    p.tiles_n = (N + kTnN - 1) / kTnN;
+    // 256 columns a block (a third more multiply-adds per byte of shared memory) unless they leave
+    // more than an eighth of the work to padding
+    const int n128 = (N + 127) / 128, n256 = (N + 255) / 256;
+    p.tn = 16 * n256 <= 9 * n128 ? 256 : 128;
+    p.tiles_n = p.tn == 256 ? n256 : n128;
     const int64_t tiles = static_cast<int64_t>(p.tiles_m) * p.tiles_n, chunks = ceil_div(Z, 4 * kTnRows);
-    int64_t wave = kTnBlocks * kNumSMs / tiles;      // splits that fill the chip once
+    int64_t wave = (p.tn == 256 ? 2 : 3) * kNumSMs / tiles;      // splits that fill the chip once
     wave = wave < 1 ? 1 : wave;
     const int64_t splits = std::min(chunks, wave * std::min<int64_t>(8, ceil_div(Z, wave * kTnMostRows)));   // (the partials stay small)
     p.rows = ceil_div(chunks, splits) * 4 * kTnRows;
@@ -152,8 +162,9 @@ extern "C" int e3b_matmul_tn(const float* x, const float* g, int64_t rows, int m
         return fail(E3B_ERR_ARG, "matmul_tn: scratch too small");
     const bool vec = m % 4 == 0 && n % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
     const dim3 grid(p.tiles_n, p.tiles_m, p.splits);
-    constexpr int smem = kTnStages * kTnStageFloats * static_cast<int>(sizeof(float));
-    auto kernel = vec ? matmul_tn_kernel<true> : matmul_tn_kernel<false>;
+    const int smem = kTnStages * static_cast<int>(sizeof(float)) * (p.tn == 256 ? tn_stage_floats<256>() : tn_stage_floats<128>());
+    auto kernel = p.tn == 256 ? (vec ? matmul_tn_kernel<256, true> : matmul_tn_kernel<256, false>)
+                              : (vec ? matmul_tn_kernel<128, true> : matmul_tn_kernel<128, false>);
     E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     float* to = p.splits > 1 ? static_cast<float*>(scratch) : out;
     kernel<<<grid, kTnThreads, smem, s>>>(x, g, rows, m, n, p.rows, p.splits > 1 ? 1.0f : scale, to);
