@@ -211,6 +211,7 @@ def core() -> ctypes.CDLL:
                                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
         lib.e3b_gate_fwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]
         lib.e3b_gate_fwd_channels.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]
+        lib.e3b_gate_bwd_channels.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]
         lib.e3b_gate_bwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]
         lib.e3b_selftest_bounded_wait.argtypes = [c_void_p, ctypes.c_uint, c_void_p]
         lib.e3b_selftest_bounded_wait.restype = c_int
@@ -218,7 +219,7 @@ def core() -> ctypes.CDLL:
                      "e3b_dense_bwd_x_supported", "e3b_fill_columns",
                      "e3b_radial_embed_fwd", "e3b_radial_embed_bwd", "e3b_radial_embed_bwd_all", "e3b_matmul_tn", "e3b_neighbor_count", "e3b_neighbor_fill",
                      "e3b_neighbor_count_rows", "e3b_neighbor_fill_rows",
-                     "e3b_gate_fwd", "e3b_gate_fwd_channels", "e3b_gate_bwd"):
+                     "e3b_gate_fwd", "e3b_gate_fwd_channels", "e3b_gate_bwd", "e3b_gate_bwd_channels"):
             getattr(lib, name).restype = c_int
         _core = lib
     return _core

@@ -69,9 +69,16 @@ def channel_tables(out_tbl: torch.Tensor, out_cst: torch.Tensor):
     return torch.tensor(rows, dtype=torch.int32).reshape(-1, 5), torch.tensor(csts, dtype=torch.float32)
 
 
+def covers_inputs(ch_tbl: torch.Tensor, din: int) -> bool:
+    """Whether every input column belongs to exactly one channel (as a component or as its gate): the gradient by channels
+    then writes every column once."""
+    cols = [c for src, n, gate, _, _ in ch_tbl.tolist() for c in list(range(src, src + n)) + ([gate] if gate >= 0 else [])]
+    return sorted(cols) == list(range(din))
+
+
 class _GateFunction(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, out_tbl, out_cst, in_tbl, in_cst, dout, ch_tbl=None, ch_cst=None):
+    def forward(ctx, x, out_tbl, out_cst, in_tbl, in_cst, dout, ch_tbl=None, ch_cst=None, ch_covers=False):
         rows, din = x.shape
         out = torch.empty(rows, dout, dtype=torch.float32, device=x.device)
         with torch.cuda.device(x.device):
@@ -82,21 +89,26 @@ class _GateFunction(torch.autograd.Function):
                 rc = _lib.core().e3b_gate_fwd(_lib._ptr(x), _lib._ptr(out_tbl), _lib._ptr(out_cst), _lib._ptr(out), rows, din,
                                               dout, _lib.stream_ptr())
         _lib.check(rc, "e3b_gate_fwd")
-        ctx.save_for_backward(x, in_tbl, in_cst)
+        ctx.by_channels = ch_covers and ch_tbl is not None
+        ctx.save_for_backward(x, *((ch_tbl, ch_cst) if ctx.by_channels else (in_tbl, in_cst)))
         ctx.dout = dout
         return out
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_out):
-        x, in_tbl, in_cst = ctx.saved_tensors
+        x, tbl, cst = ctx.saved_tensors
         rows, din = x.shape
         gx = torch.empty_like(x)
         with torch.cuda.device(x.device):
-            rc = _lib.core().e3b_gate_bwd(_lib._ptr(x), _lib._ptr(grad_out.contiguous()), _lib._ptr(in_tbl), _lib._ptr(in_cst),
-                                          _lib._ptr(gx), rows, din, ctx.dout, _lib.stream_ptr())
+            grad_out = grad_out.contiguous()
+            args = (_lib._ptr(x), _lib._ptr(grad_out), _lib._ptr(tbl), _lib._ptr(cst), _lib._ptr(gx), rows, din, ctx.dout)
+            if ctx.by_channels:
+                rc = _lib.core().e3b_gate_bwd_channels(*args, tbl.shape[0], _lib.stream_ptr())
+            else:
+                rc = _lib.core().e3b_gate_bwd(*args, _lib.stream_ptr())
         _lib.check(rc, "e3b_gate_bwd")
-        return gx, None, None, None, None, None, None, None
+        return gx, None, None, None, None, None, None, None, None
 
 
 class Gate(torch.nn.Module):
@@ -172,6 +184,7 @@ class Gate(torch.nn.Module):
         ch_tbl, ch_cst = channel_tables(self._out_tbl, self._out_cst)
         self.register_buffer("_ch_tbl", ch_tbl, persistent=False)
         self.register_buffer("_ch_cst", ch_cst, persistent=False)
+        self._ch_covers = covers_inputs(ch_tbl, din)
 
     def __repr__(self) -> str:
         return f"{self.__class__.__name__} ({self.irreps_in} -> {self.irreps_out})"
@@ -187,5 +200,6 @@ class Gate(torch.nn.Module):
         for name in ("_out_cst", "_in_cst", "_ch_cst"):
             _lib.require_operand(getattr(self, name), x, f"Gate.{name} (move the module with .to(device))")
         out = _GateFunction.apply(x, self._out_tbl, self._out_cst, self._in_tbl, self._in_cst, self.irreps_out.dim,
-                                  self._ch_tbl if self._ch_tbl.shape[0] > 0 else None, self._ch_cst)
+                                  self._ch_tbl if self._ch_tbl.shape[0] > 0 else None, self._ch_cst,
+                                  getattr(self, "_ch_covers", False))
         return out.reshape(*lead, self.irreps_out.dim)

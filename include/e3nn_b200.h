@@ -201,6 +201,10 @@ int e3b_gate_fwd(const float* x, const int32_t* out_table, const float* out_cons
  * a gate is evaluated once per channel instead of once per gated component. */
 int e3b_gate_fwd_channels(const float* x, const int32_t* channel_table, const float* channel_const, float* out,
                           int64_t rows, int din, int dout, int num_channels, void* stream);
+/* e3b_gate_bwd_channels: the gradient from the table of e3b_gate_fwd_channels, when every input column belongs to exactly one
+ * channel (as a component or as its gate). */
+int e3b_gate_bwd_channels(const float* x, const float* grad_out, const int32_t* channel_table, const float* channel_const,
+                          float* grad_x, int64_t rows, int din, int dout, int num_channels, void* stream);
 int e3b_gate_bwd(const float* x, const float* grad_out, const int32_t* in_table, const float* in_const, float* grad_x,
                  int64_t rows, int din, int dout, void* stream);
 

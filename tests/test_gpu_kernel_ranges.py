@@ -215,3 +215,30 @@ def test_dense_layer_tiles(width, rows):
         e3nn_b200.check_status()
         assert torch.all(buf[0] == 7.0) and torch.all(buf[-1] == 7.0)
         assert rel_err(buf[1 : rows + 1].cpu(), b * (x.double() @ a.double())) < 4e-5
+
+
+# ----------------------------------------------------------------------------- Gate by channels
+@pytest.mark.parametrize("rows", [1, 2, 333])
+@pytest.mark.parametrize("scalars,gates,gated", [("5x0e", "3x0e+2x0e+4x0e+1x0e", "3x1o+2x2e+4x3o+1x4e"), ("", "70x0e", "70x1o"), ("300x0e", "", "")])
+def test_gate_channels(scalars, gates, gated, rows):
+    """One to nine components a channel, more channels than a block has threads, gates only, scalars only; the gradient by
+    channels against the one by columns (the same formula: differences of the last bit) and the forward against fp64."""
+    from e3nn_b200 import _lib
+
+    silu, sig = torch.nn.functional.silu, torch.sigmoid
+    gate = bnn.Gate(scalars, [silu] * len(o3.Irreps(scalars)), gates, [sig] * len(o3.Irreps(gates)), gated).to(DEV)
+    assert gate._ch_covers
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, gate.irreps_in.dim, generator=g).to(DEV).requires_grad_(True)
+    go = torch.randn(rows, gate.irreps_out.dim, generator=g).to(DEV)
+    out = gate(x)
+    (got,) = torch.autograd.grad(out, x, go)
+    by_columns = torch.empty_like(x)
+    rc = _lib.core().e3b_gate_bwd(_lib._ptr(x), _lib._ptr(go), _lib._ptr(gate._in_tbl), _lib._ptr(gate._in_cst), _lib._ptr(by_columns), rows,
+                                  x.shape[1], go.shape[1], _lib.stream_ptr())
+    assert rc == 0
+    assert rel_err(got.cpu(), by_columns.cpu().double()) < 1e-6
+    t, c, x64 = gate._out_tbl.cpu().long(), gate._out_cst.cpu().double(), x.detach().cpu().double()
+    f = lambda act, v: torch.where(act == 0, silu(v), torch.sigmoid(v))      # noqa: E731
+    ref = torch.where(t[:, 1] < 0, c * f(t[:, 2], x64[:, t[:, 0]]), x64[:, t[:, 0]] * c * f(t[:, 2], x64[:, t[:, 1].clamp_min(0)]))
+    assert rel_err(out.detach().cpu(), ref) < 1e-5
