@@ -8,6 +8,8 @@ is its offset.
 """
 from __future__ import annotations
 
+import struct
+from itertools import chain
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -18,8 +20,11 @@ from ._wigner import wigner_3j_numpy
 MAGIC = 0x65336250
 
 
+_FLOAT, _INT = struct.Struct("<f"), struct.Struct("<i")
+
+
 def _f2i(v: float) -> int:
-    return int(np.float32(v).view(np.int32))
+    return _INT.unpack(_FLOAT.pack(v))[0]
 
 
 class _Builder:
@@ -54,8 +59,7 @@ class _Builder:
 
     def add_group(self, out_off: int, mul_out: int, dim3: int, kents: Sequence[Tuple[int, int, int, int]], w_stride: int = 1):
         start = len(self.kent) // 4
-        for k in kents:
-            self.kent += list(k)
+        self.kent += chain.from_iterable(kents)
         self.groups.append([out_off, mul_out, dim3, len(kents), start, w_stride])
         self.max_k = max(self.max_k, len(kents))
 
@@ -104,9 +108,9 @@ class _Builder:
             d1max, d3max = max(d1max, d1), max(d3max, d3)
             ki = jj = 0
             if p["x2off"] >= 0:
-                c = p["c"]
-                ki = segments([[(j, float(c[i, j, k])) for j in range(d2) if c[i, j, k] != 0.0] for k in range(d3) for i in range(d1)])
-                jj = segments([[(i * d3 + k, float(c[i, j, k])) for i in range(d1) for k in range(d3) if c[i, j, k] != 0.0] for j in range(d2)])
+                c = p["c"].tolist()
+                ki = segments([[(j, c[i][j][k]) for j in range(d2) if c[i][j][k] != 0.0] for k in range(d3) for i in range(d1)])
+                jj = segments([[(i * d3 + k, c[i][j][k]) for i in range(d1) for k in range(d3) if c[i][j][k] != 0.0] for j in range(d2)])
             rows.append([d1, d2, d3, p["su"], p["sw"], ki, jj, p["x1off"], p["m1"], p["x2off"], p["m2"], p["out_off"], p["mo"],
                          p["wbase"], p["sv"], _f2i(p.get("coef", 0.0))])
         chunks, groups = [], []
@@ -162,14 +166,10 @@ def uvw_plan(spec, instruction_ids: Optional[Sequence[int]] = None) -> Tuple[np.
                 continue
             (m1, ir1), (m2, ir2) = i1[ins.i_in1], i2[ins.i_in2]
             c = wigner_3j_numpy(ir1.l, ir2.l, ir_out.l) * ins.path_weight
-            per_k = []
-            for k in range(ir_out.dim):
-                per_k.append([(i, j, float(c[i, j, k])) for i in range(ir1.dim) for j in range(ir2.dim) if c[i, j, k] != 0.0])
-            pid = b.add_path(per_k)
-            for u in range(m1):
-                for v in range(m2):
-                    kents.append((pid, o1[ins.i_in1] + u * ir1.dim, o2[ins.i_in2] + v * ir2.dim,
-                                  woffs[n] + (u * m2 + v) * mul_out))
+            cl, x1off, x2off, d1, d2 = c.tolist(), o1[ins.i_in1], o2[ins.i_in2], ir1.dim, ir2.dim
+            pid = b.add_path([[(i, j, cl[i][j][k]) for i in range(d1) for j in range(d2) if cl[i][j][k] != 0.0]
+                              for k in range(ir_out.dim)])
+            kents += [(pid, x1off + u * d1, x2off + v * d2, woffs[n] + (u * m2 + v) * mul_out) for u in range(m1) for v in range(m2)]
             whole.append(b.add_whole_path(x1off=o1[ins.i_in1], m1=m1, d1=ir1.dim, x2off=o2[ins.i_in2], m2=m2, d2=ir2.dim,
                                           out_off=oo[out_idx], mo=mul_out, d3=ir_out.dim, wbase=woffs[n], su=m2 * mul_out, sv=mul_out,
                                           sw=1, c=c))
