@@ -113,7 +113,23 @@ class Group:
     def smem_bytes(self) -> int:
         return self.resident_bytes() + self.nstage() * self.stage_bytes() + self.extra_bytes() + 1024 + 1024
 
+    producers: int = 0         # producer warps (Linear and its transpose), for work()
+
     def work(self) -> int:
+        if self.producers:
+            # Linear: microseconds of a 128-row tile, the longer of the producers' chunks and the epilogue, fitted to each
+            # group timed alone (conv Linear 6336 -> 1024, its transpose, 1024 -> 1216 and its transpose; within 20 %).  Against
+            # a split by the sum below: 6336 -> 1024 transposed, 262,144 rows 3.49 -> 3.04 ms, 16,384 rows 236 -> 202 us;
+            # 1024 -> 1216, 100,000 rows 409 -> 356 us, its transpose 448 -> 387 us.
+            chunk = (1.0 if self.dim == 7 else 0.9) if self.producers > 8 else 1.2
+            if self.staged_epilogue():
+                epilogue = 3.3 + 0.0042 * self.n
+            elif self.swap:
+                epilogue = 2.1 + (0.009 if self.dim == 3 else 0.013) * self.n
+            else:
+                epilogue = (2.5 if self.dim == 3 else 1.6) + 0.0265 * self.n
+            tile = max(chunk * len(self.chunks), epilogue) * (1.5 if self.nstage() == 2 else 1.0)
+            return max(1, int(100000 * tile / self.zt))
         # per 128-row tile: the producers' chunks plus the epilogue (tensor-memory loads and stores of N columns per
         # row; the dominant term of short-K groups)
         per_tile = sum(40 + self.case_cost[c.case] * max(1, -(-self.zt // PRODUCER_WARPS)) for c in self.chunks)
@@ -249,6 +265,7 @@ def linear_gemm_spec(irreps_in: Irreps, irreps_out: Irreps, instructions, transp
     for g in out:
         g.has_y = False
         g.aligned_out = dst.dim % 4 == 0 and g.out_off % 4 == 0
+        g.producers = 8 if transpose else 16
         g.swap = transpose and g.dim in SWAP_DIMS and g.n % 128 == 0 and not g.staged_epilogue()
     if any(g.nstage() < 2 for g in out):
         return None
