@@ -1168,18 +1168,20 @@ static bool rows_plan(const Part2& P) {
 // A plan couples a second operand in all of its paths (a product) or in none (a Linear).
 static bool coupled_plan(const Part2& P) { return P.h[2] > 0 && P.chunk(0)[3] >= 0; }
 
-// pass: 0 every group, 1 the groups of scalars, 2 the others.
+// pass: 0 every group, 1 the groups of scalars, 2 the others.  Scalar groups with Gate go out one launch each, in plan order: a
+// gated scalar then finds the gates of an earlier irrep written (blocks of one grid have no order among them).
 template <bool COUPLED, bool GATE>
 static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
                            float* out, int64_t Z, int accumulate, const DenseGateEpilogue& ep, int pass, cudaStream_t s, bool* done) {
     const Part2 P(plan_host);
+    const int most = GATE && pass == 1 ? 1 : kMaxGroups;
     int g0 = 0;
     while (g0 < P.n_groups()) {
         RowsLaunch L;
         L.n = 0;
         int64_t blocks = 0;
         size_t floats = 0;
-        for (; g0 < P.n_groups() && L.n < kMaxGroups; ++g0) {
+        for (; g0 < P.n_groups() && L.n < most; ++g0) {
             const int32_t* g = P.group(g0);
             if (g[1] == 0 || g[4] == 0 || (pass == 1 && g[2] != 1) || (pass == 2 && g[2] == 1)) continue;
             // the narrowest tile that holds the group's channels in one pass, so that the coupled operand is built once

@@ -8,7 +8,8 @@ scalar irreps (plain scalars and gates) first, the gated irreps after them; only
 round trip through memory.  The result equals ``gate(lin(x))``.
 
 The fused kernels are forward passes.  When a gradient is required (the Gate's gradient needs the Linear's output
-row), with biases, or for Linear outputs no path writes, the two modules run one after the other.
+row), with biases, for Linear outputs no path writes, or when a gated irrep is itself a scalar (it would read its gate in
+the launch that writes it), the two modules run one after the other.
 
 ``fuse``: ``True`` runs the fused kernels whenever they apply, ``False`` never, ``"auto"`` (default) only where they
 are the faster choice.  Today that is nowhere: the fused pair moves 46 % fewer bytes, but both Linear kernels are
@@ -61,6 +62,7 @@ class LinearGate(torch.nn.Module):
         needs_grad = torch.is_grad_enabled() and (features.requires_grad or any(p.requires_grad for p in lin.parameters()))
         return (not needs_grad and lin.internal_weights and lin.bias_numel == 0 and not lin._unwritten
                 and lin.weight_numel > 0 and features.dtype == torch.float32
+                and not any(mul > 0 and ir.l == 0 for mul, ir in self.gate.irreps_gated)
                 and (lin._precision == 0 or lin._tc_fwd is not None))
 
     def forward(self, features: torch.Tensor) -> torch.Tensor:

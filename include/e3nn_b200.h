@@ -233,7 +233,8 @@ int e3b_dense_fwd(const int32_t* plan_host, const int32_t* plan_dev, const float
  *   kind 0 scalar:  out[z, dst]    = const * act(y)        kind 2 gate: gates[z, slot] = const * act(y)
  *   kind 1 gated:   out[z, dst]    = y * gates[z, slot]    kind 3: no output depends on the column.
  * gates [rows, n_slots] is written and read by this call (the only extra traffic: the gate scalars, once each way);
- * out [rows, dout] is the Gate's output row.  Scalar irreps are launched before the gated ones on `stream`.
+ * out [rows, dout] is the Gate's output row.  Scalar irreps are launched before the others on `stream`, one launch each in the
+ * order of the plan: a gated irrep that is itself a scalar must come after the irrep of its gates, in a block of its own.
  * Activation codes as in e3b_gate_fwd.
  */
 int e3b_dense_fwd_gate(const int32_t* plan_host, const int32_t* plan_dev, const float* x, const float* weight,

@@ -46,7 +46,8 @@ int e3b_tc_gemm_fwd(const float* x1, const float* x2, const float* weight, float
  * {kind, destination column, activation, gate slot} and gate_const [dout] per column of that row: kind 0 scalar:
  * out[z, dst] = const * act(y); kind 2 gate: gates[z, slot] = const * act(y); kind 1 component k of a gated channel
  * (entry of its component 0): out[z, dst + k] = y * gates[z, slot]; kind 3 unused.  gates [Z, n_slots], out
- * [Z, dout_final] (the Gate's output row).  Activation codes of e3b_gate_fwd.  Two launches on `stream`.
+ * [Z, dout_final] (the Gate's output row).  Activation codes of e3b_gate_fwd.  Two launches on `stream`, scalar columns in the
+ * first: a gated channel must not be a scalar itself.
  */
 int e3b_tc_gemm_fwd_gate(const float* x1, const float* weight, const int32_t* gate_table, const float* gate_const,
                          float* gates, int n_slots, float* out, int dout_final, int64_t Z, int precision, void* scratch,

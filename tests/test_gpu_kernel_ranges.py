@@ -242,3 +242,40 @@ def test_gate_channels(scalars, gates, gated, rows):
     f = lambda act, v: torch.where(act == 0, silu(v), torch.sigmoid(v))      # noqa: E731
     ref = torch.where(t[:, 1] < 0, c * f(t[:, 2], x64[:, t[:, 0]]), x64[:, t[:, 0]] * c * f(t[:, 2], x64[:, t[:, 1].clamp_min(0)]))
     assert rel_err(out.detach().cpu(), ref) < 1e-5
+
+
+# ----------------------------------------------------------------------------- Gate as the Linear's epilogue: gated scalars
+GATED_SCALARS = [
+    # gate arguments, the Linear's output irreps, whether every gate stands in an irrep before the scalars it gates
+    (("16x0e", ["silu"], "8x0o", ["tanh"], "8x0e"), "8x0o+24x0e", True),
+    (("16x0e", ["silu"], "8x0e+4x0e", ["sigmoid", "tanh"], "8x0e+4x1o"), "16x0e+12x0e+8x0e+4x1o", True),
+    (("16x0e", ["silu"], "8x0e", ["sigmoid"], "8x0e"), "32x0e", False),
+    (("16x0e", ["silu"], "8x0e", ["sigmoid"], "8x0o"), "8x0o+24x0e", False),
+]
+
+
+@pytest.mark.parametrize("rows", [1, 5000])
+@pytest.mark.parametrize("args,irreps,ordered", GATED_SCALARS)
+def test_linear_gate_gated_scalars(args, irreps, ordered, rows):
+    """The module against the fp64 oracle; where the gates' irreps come first, the fused entry point too, from gate slots that
+    held NaN.  1e-5 x RMS, the fp32 parity bound of this path."""
+    from e3nn_b200 import _lib
+
+    f = {"silu": torch.nn.functional.silu, "tanh": torch.tanh, "sigmoid": torch.sigmoid}
+    gate = bnn.Gate(args[0], [f[a] for a in args[1]], args[2], [f[a] for a in args[3]], args[4])
+    lin = o3.Linear("24x0e+12x0o+8x1o", irreps)
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, lin.irreps_in.dim, generator=g)
+    ref = orc.gate(*args, orc.linear(str(lin.irreps_in), str(lin.irreps_out), x.double(), lin.weight.detach().double()))
+    pair = bnn.LinearGate(lin, gate, fuse=True).to(DEV)
+    xd = x.to(DEV)
+    with torch.no_grad():
+        assert rel_err(pair(xd).cpu(), ref) < 1e-5
+    if ordered:
+        gates = torch.full((rows, pair.n_slots), float("nan"), device=DEV)
+        out = torch.full((rows, gate.irreps_out.dim), float("nan"), device=DEV)
+        rc = _lib.core().e3b_dense_fwd_gate(lin._plan_host.ctypes.data, _lib._ptr(lin._plan_on(xd.device, False)), _lib._ptr(xd),
+                                            _lib._ptr(lin.weight.detach()), _lib._ptr(pair._fuse_tbl), _lib._ptr(pair._fuse_cst),
+                                            _lib._ptr(gates), pair.n_slots, _lib._ptr(out), out.shape[1], rows, _lib.stream_ptr())
+        assert rc == 0
+        assert rel_err(out.cpu(), ref) < 1e-5

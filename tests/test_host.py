@@ -273,3 +273,18 @@ def test_cta_split_is_proportional_and_bounded():
             assert _lib._tc_gemm_max_ctas is None
         assert _lib._tc_gemm_max_ctas == 100
     assert _lib._tc_gemm_max_ctas is None
+
+
+@pytest.mark.parametrize("mode", ["fp32", "tf32x3"])
+@pytest.mark.parametrize("gates,gated,fuses", [("64x0o", "64x0e", False), ("64x0e", "64x0o", False), ("64x0e", "32x0e+32x1o", False),
+                                               ("64x0e", "0x0e+64x1o", True)])
+def test_linear_gate_does_not_fuse_gated_scalars(mode, gates, gated, fuses):
+    """The fused kernels write the gates in the launch of the scalar columns, which has no order among its blocks: a gated
+    scalar would read its gate there."""
+    from e3nn_b200 import nn as bnn
+
+    gate = bnn.Gate("64x0e", [torch.tanh], gates, [torch.tanh], gated)
+    lin = o3.Linear(gate.irreps_in, gate.irreps_in, math_mode=mode)
+    pair = bnn.LinearGate(lin, gate, fuse=True)
+    with torch.no_grad():
+        assert pair.fusable(torch.zeros(1, lin.irreps_in.dim)) == fuses
