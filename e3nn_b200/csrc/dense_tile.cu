@@ -1165,9 +1165,21 @@ static bool rows_plan(const Part2& P) {
     return true;
 }
 
+// Whether the tile of every group that has work fits a block's shared memory.
+template <typename ShapeOf>
+static bool all_groups_fit(const Part2& P, const ShapeOf& shape_of) {
+    for (int n = 0; n < P.n_groups(); ++n) {
+        const int32_t* g = P.group(n);
+        if (g[1] != 0 && g[4] != 0 && shape_of(g).floats * sizeof(float) > static_cast<size_t>(kMaxShared)) return false;
+    }
+    return true;
+}
+
 // A plan couples a second operand in all of its paths (a product) or in none (a Linear).
 static bool coupled_plan(const Part2& P) { return P.h[2] > 0 && P.chunk(0)[3] >= 0; }
 
+// Launches go out up to kMaxGroups groups at a time.  *done = false: nothing was launched, because a group needs more shared
+// memory than a block can have (a very wide second operand).
 // pass: 0 every group, 1 the groups of scalars, 2 the others.  Scalar groups with Gate go out one launch each, in plan order: a
 // gated scalar then finds the gates of an earlier irrep written (blocks of one grid have no order among them).
 template <bool COUPLED, bool GATE>
@@ -1175,6 +1187,11 @@ static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, co
                            float* out, int64_t Z, int accumulate, const DenseGateEpilogue& ep, int pass, cudaStream_t s, bool* done) {
     const Part2 P(plan_host);
     const int most = GATE && pass == 1 ? 1 : kMaxGroups;
+    // the narrowest tile that holds the group's channels in one pass, so that the coupled operand is built once
+    auto threads_a_row = [](const int32_t* g) { return g[1] <= 32 ? 4 : g[1] <= 64 ? 8 : 16; };
+    auto shape_of = [&](const int32_t* g) { return fwd_shape<COUPLED>(g[2], threads_a_row(g), P.d1max(), plan_host[2]); };
+    *done = all_groups_fit(P, shape_of);
+    if (!*done) return E3B_OK;
     int g0 = 0;
     while (g0 < P.n_groups()) {
         RowsLaunch L;
@@ -1184,9 +1201,8 @@ static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, co
         for (; g0 < P.n_groups() && L.n < most; ++g0) {
             const int32_t* g = P.group(g0);
             if (g[1] == 0 || g[4] == 0 || (pass == 1 && g[2] != 1) || (pass == 2 && g[2] == 1)) continue;
-            // the narrowest tile that holds the group's channels in one pass, so that the coupled operand is built once
-            const int tx = g[1] <= 32 ? 4 : g[1] <= 64 ? 8 : 16;
-            const FwdShape shape = fwd_shape<COUPLED>(g[2], tx, P.d1max(), plan_host[2]);
+            const int tx = threads_a_row(g);
+            const FwdShape shape = shape_of(g);
             L.first_block[L.n] = static_cast<int>(blocks);
             L.group[L.n] = static_cast<int16_t>(g0);
             L.shape[L.n] = static_cast<int16_t>(tx);
@@ -1198,21 +1214,23 @@ static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, co
         if (L.n == 0) continue;
         L.first_block[L.n] = static_cast<int>(blocks);
         const size_t bytes = floats * sizeof(float);
-        if (bytes > static_cast<size_t>(kMaxShared)) return E3B_OK;      // a very wide second operand: *done stays false
         auto kernel = dense_rows_fwd_kernel<COUPLED, GATE>;
         E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
         kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, weight, out, Z, accumulate, L, ep);
         if (int rc = check_launch("e3b_dense_fwd")) return rc;
-        *done = true;
     }
-    *done = true;
     return E3B_OK;
 }
 
+// As launch_rows_fwd, for the weight gradient.
 template <bool COUPLED>
 static int launch_rows_wgrad(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* gout,
                              float* grad_w, int64_t Z, cudaStream_t s, bool* done) {
     const Part2 P(plan_host);
+    auto channels_of = [](const int32_t* g) { return g[1] <= 32 ? 32 : g[1] <= 64 ? 64 : 128; };
+    auto shape_of = [&](const int32_t* g) { return wgrad_shape<COUPLED>(g[2], channels_of(g), P.d1max(), plan_host[2]); };
+    *done = all_groups_fit(P, shape_of);
+    if (!*done) return E3B_OK;
     int g0 = 0;
     while (g0 < P.n_groups()) {
         RowsLaunch L;
@@ -1222,8 +1240,8 @@ static int launch_rows_wgrad(const int32_t* plan_host, const int32_t* plan_dev, 
         for (; g0 < P.n_groups() && L.n < kMaxGroups; ++g0) {
             const int32_t* g = P.group(g0);
             if (g[1] == 0 || g[4] == 0) continue;
-            const int bw = g[1] <= 32 ? 32 : g[1] <= 64 ? 64 : 128;
-            const FwdShape shape = wgrad_shape<COUPLED>(g[2], bw, P.d1max(), plan_host[2]);
+            const int bw = channels_of(g);
+            const FwdShape shape = shape_of(g);
             L.group[L.n] = static_cast<int16_t>(g0);
             L.shape[L.n] = static_cast<int16_t>(bw);
             parts[L.n] = ceil_div(g[4], 4096 / bw / kKC) * ceil_div(g[1], bw);
@@ -1235,7 +1253,6 @@ static int launch_rows_wgrad(const int32_t* plan_host, const int32_t* plan_dev, 
         }
         if (L.n == 0) continue;
         const size_t bytes = floats * sizeof(float);
-        if (bytes > static_cast<size_t>(kMaxShared)) return E3B_OK;
         // one wave of resident blocks over all groups, in proportion to their rows x components
         const int64_t resident = kNumSMs * std::max<int64_t>(1, std::min<int64_t>(4, kMaxShared / static_cast<int64_t>(bytes + 1024)));
         for (int n = 0; n < L.n; ++n) {
@@ -1250,9 +1267,7 @@ static int launch_rows_wgrad(const int32_t* plan_host, const int32_t* plan_dev, 
         E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
         kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, gout, grad_w, Z, L);
         if (int rc = check_launch("e3b_dense_bwd_w")) return rc;
-        *done = true;
     }
-    *done = true;
     return E3B_OK;
 }
 

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 import e3nn_b200
-from conftest import rel_err
+from conftest import fp32_bound, rel_err
 from e3nn_b200 import layouts
 from e3nn_b200 import nn as bnn
 from e3nn_b200 import o3
@@ -82,6 +82,34 @@ def test_fp32_product_tiles(layout, rows):
     for n, leaf in enumerate((xd, yd)):
         other = tp(xd if n == 0 else xd.detach(), yd if n == 1 else yd.detach(), tp.weight.detach())
         assert rel_err(torch.autograd.grad(other, leaf, go.to(DEV))[0].cpu(), ref_g[n]) < 1e-5
+
+
+@pytest.mark.parametrize("tail", ["2x3o", "2x0e"])
+def test_fp32_product_many_outputs_wide_second_operand(tail):
+    """33 output irreps (32 go out in one launch) and a second operand of 1,280 columns: with the l = 3 irrep last, the first 32
+    fit a block's shared memory and the last does not.  Outputs start from NaN.  Bound: 1e-5 x RMS, or 1.5 times the distance of
+    plain fp32 arithmetic on the host where that is larger (sums of up to 5,280 terms)."""
+    rows = 40
+    g = torch.Generator().manual_seed(5)
+    outs = "+".join(["2x0e"] * 32 + [tail])
+    ins = [(i, j, k, "uvw", True) for k, l in enumerate([0] * 32 + [3 if tail == "2x3o" else 0])
+           for i, j in [(0, 0), (3, 3), (0, 3), (3, 0)] if (l == 3) == (i != j)]
+    tp = o3.TensorProduct("2x0e+2x1o+2x2e+2x3o", "80x0e+80x1o+80x2e+80x3o", outs, ins)
+    x, y = torch.randn(rows, tp.irreps_in1.dim, generator=g), torch.randn(rows, tp.irreps_in2.dim, generator=g)
+    go = torch.randn(rows, tp.irreps_out.dim, generator=g)
+    want = []
+    for dtype in (torch.float64, torch.float32):
+        leaves = [t.detach().to(dtype).requires_grad_(True) for t in (x, y, tp.weight)]
+        ref = orc.tensor_product(*(str(i) for i in (tp.irreps_in1, tp.irreps_in2, tp.irreps_out)), ins, *leaves, True)
+        want.append([ref.detach()] + list(torch.autograd.grad(ref, leaves, go.to(dtype))))
+    tp = tp.to(DEV)
+    xd, yd = x.to(DEV).requires_grad_(True), y.to(DEV).requires_grad_(True)
+    out = torch.full((rows, tp.irreps_out.dim), float("nan"), device=DEV)
+    with torch.no_grad():
+        tp._uvw_run(xd, yd, tp.weight, out, False)
+    got = [out] + list(torch.autograd.grad(tp(xd, yd), [xd, yd, tp.weight], go.to(DEV)))
+    for a, r64, r32 in zip(got, *want):
+        assert rel_err(a.cpu(), r64) < fp32_bound(rel_err(r32, r64))
 
 
 @pytest.mark.parametrize("rows", [1, 257])
