@@ -22,7 +22,7 @@ from .. import _lib, layouts
 from ..message_passing import conv_uvu
 from ..o3 import Irreps, Linear
 from ._edge_embed import edge_embed
-from ._fc import FullyConnectedNet, bessel
+from ._fc import FullyConnectedNet, _Layer, bessel
 
 
 def radius_graph_pbc(pos: torch.Tensor, box: float, cutoff: float) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
@@ -121,14 +121,18 @@ class InteractionBlock(torch.nn.Module):
 
     def _embeds(self, pos, edge_src, edge_dst, shift) -> bool:
         """Whether a training step (gradient of the first radial layer's weights wanted) may use the fused edge embedding:
-        operands in the one form that kernel reads, no gradient w.r.t. the shifts, and no hooks on the modules it stands for."""
+        operands in the one form that kernel reads, no gradient w.r.t. the shifts, and the modules and the method it stands for
+        are this package's own, without hooks."""
         E, dev = edge_src.numel(), pos.device
         w0 = self.fc.layer0.weight
-        return (pos.dim() == 2 and pos.shape[1] == 3 and edge_src.shape == edge_dst.shape == (E,)
+        return (type(self.fc) is FullyConnectedNet and type(self.fc.layer0) is _Layer
+                and type(self).edge_weights is InteractionBlock.edge_weights and "edge_weights" not in self.__dict__
+                and pos.dim() == 2 and pos.shape[1] == 3 and edge_src.shape == edge_dst.shape == (E,)
                 and edge_src.dtype == edge_dst.dtype == torch.int64 and edge_src.device == edge_dst.device == dev
                 and w0.device == dev and w0.dtype == torch.float32
                 and (shift is None or (shift.shape == (E, 3) and shift.dtype == torch.float32 and shift.device == dev
                                        and not shift.requires_grad))
+                and not torch.nn.modules.module._has_any_global_hook()
                 and not any(hooks for m in (self.fc, self.fc.layer0)
                             for hooks in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks, m._backward_pre_hooks)))
 

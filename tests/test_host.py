@@ -288,3 +288,41 @@ def test_linear_gate_does_not_fuse_gated_scalars(mode, gates, gated, fuses):
     pair = bnn.LinearGate(lin, gate, fuse=True)
     with torch.no_grad():
         assert pair.fusable(torch.zeros(1, lin.irreps_in.dim)) == fuses
+
+
+def test_interaction_block_embeds_only_in_place_of_its_own_modules():
+    """The fused edge embedding of a training step stands for ``edge_weights`` and the radial network's first layer: with either
+    replaced, or hooks in the way, the step runs them."""
+    from e3nn_b200 import nn as bnn
+
+    class OtherNet(bnn.FullyConnectedNet):
+        pass
+
+    class OtherBlock(bnn.InteractionBlock):
+        def edge_weights(self, edge_vec):
+            return 2.0 * super().edge_weights(edge_vec)
+
+    def block(cls=bnn.InteractionBlock):
+        return cls("8x0e+8x1o", 1, hidden=32)
+
+    pos, idx = torch.zeros(4, 3), torch.zeros(6, dtype=torch.int64)
+    embeds = lambda b: b._embeds(pos, idx, idx, None)      # noqa: E731
+    assert embeds(block()) and not embeds(block(OtherBlock))
+    b = block()
+    b.edge_weights = lambda vec: vec
+    assert not embeds(b)
+    b = block()
+    b.fc = OtherNet(b.fc.hs, torch.nn.functional.silu)
+    assert not embeds(b)
+    b = block()
+    torch.nn.utils.parametrize.register_parametrization(b.fc.layer0, "weight", torch.nn.Identity())
+    assert not embeds(b)
+    b = block()
+    b.fc.layer0.register_forward_hook(lambda *a: None)
+    assert not embeds(b)
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    try:
+        assert not embeds(block())
+    finally:
+        handle.remove()
+    assert embeds(block())
