@@ -255,8 +255,10 @@ __global__ void __launch_bounds__(kThreads) dense_tile_fwd_kernel(const int32_t*
     }
 }
 
-// Columns of a tile: the narrowest that holds the group's channels in one pass, so that the coupled operand is built once.
-inline int columns_for(int mo) { return mo <= 16 ? 16 : mo <= 32 ? 32 : mo <= 64 ? 64 : 128; }
+// Columns of a tile: the narrowest that holds the group's channels in one pass, so that the coupled operand is built once;
+// at most 64 where one row's components would not fit the rows of a wider tile (l = 16 and up).
+constexpr int kMostDim = 64;
+inline int columns_for(int mo, int d3) { return mo <= 16 ? 16 : mo <= 32 ? 32 : (mo <= 64 || d3 > tile_rows(128)) ? 64 : 128; }
 
 // ---------------------------------------------------------------------------------------------- weight gradient, any irrep
 // grad_W_p[u, v, w] += sum_{z, k} A[z, k, u] grad_out[z, w, k]: a block owns the K entries of up to 128 / 64 / 32 channels
@@ -1302,8 +1304,8 @@ int launch_dense_tile_fwd(const int32_t* plan_host, const int32_t* plan_dev, con
         for (; g0 < P.n_groups() && L.n < kMaxGroups; ++g0) {
             const int32_t* g = P.group(g0);
             if (g[1] == 0 || g[4] == 0) continue;
-            const int bn = columns_for(g[1]), bm = tile_rows(bn);
-            if (g[2] > bm) return fail(E3B_ERR_UNSUPPORTED, "dense_fwd: irrep dimension %d too large", g[2]);
+            const int bn = columns_for(g[1], g[2]), bm = tile_rows(bn);
+            if (g[2] > kMostDim) return fail(E3B_ERR_UNSUPPORTED, "dense_fwd: irrep dimension %d too large", g[2]);
             L.first_block[L.n] = static_cast<int>(blocks);
             L.group[L.n] = static_cast<int16_t>(g0);
             L.bn[L.n] = static_cast<int16_t>(bn);

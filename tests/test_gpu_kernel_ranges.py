@@ -113,9 +113,11 @@ def test_fp32_product_many_outputs_wide_second_operand(tail):
 
 
 @pytest.mark.parametrize("rows", [1, 257])
-@pytest.mark.parametrize("irreps", [("1x0e+40x1o+3x2e", "200x0e+2x0e+17x1o"), ("70x0e+9x4e", "9x4e+16x0e+5x1o"), ("64x0e+64x3o", "32x0e+64x3o")])
+@pytest.mark.parametrize("irreps", [("1x0e+40x1o+3x2e", "200x0e+2x0e+17x1o"), ("70x0e+9x4e", "9x4e+16x0e+5x1o"), ("64x0e+64x3o", "32x0e+64x3o"),
+                                    ("40x16e+3x31o+2x0e", "70x16e+130x31o+5x0e")])
 def test_fp32_linear_tiles(irreps, rows):
-    """Forward, transposed (two outputs of different width from one input, an input nothing reads) and weight gradient."""
+    """Forward, transposed (two outputs of different width from one input, an input nothing reads) and weight gradient; the
+    last layout has more components than a tile of 128 columns has rows, up to the largest irrep taken."""
     g = torch.Generator().manual_seed(rows)
     lin = o3.Linear(*irreps)
     x, go = torch.randn(rows, lin.irreps_in.dim, generator=g), torch.randn(rows, lin.irreps_out.dim, generator=g)
