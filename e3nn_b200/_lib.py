@@ -63,14 +63,23 @@ def require_cuda(*tensors: torch.Tensor) -> None:
 # (CSR builder), 2 = a source / edge index out of range (the access was skipped), 3 = a bounded wait on an mbarrier gave
 # up (the kernel returned early, its output is incomplete).  One word per device lives for the life of the process, in
 # pinned host memory that the device addresses directly: a kernel writes it only when something is wrong, the next call
-# of any op on that device looks at it (no synchronisation) and raises; `check_status` synchronises and raises.  A code
-# stays until it is raised once.  (With the word in device memory a copy and an event followed every launch: nine copies
+# of any op on that device looks at it (no synchronisation while it is 0) and raises; `check_status` synchronises and raises.
+# A code stays until it is raised once: the word is cleared when the device is idle, because a launch that has reported one
+# bad index may still be running and report more.  (With the word in device memory a copy and an event followed every launch: nine copies
 # and 0.1 ms of host time in a molecular-dynamics step.)
 class _DeviceStatus:
     def __init__(self, device: torch.device):
         self.device = device
         self.word = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.value = c_int32.from_address(self.word.data_ptr())
+        self.lock = threading.Lock()
+
+    def take(self) -> int:
+        """Wait for the device, return the word and clear it."""
+        with self.lock:
+            torch.cuda.synchronize(self.device)
+            code, self.value.value = self.value.value, 0
+        return code
 
 
 _status: Dict[int, _DeviceStatus] = {}
@@ -107,12 +116,13 @@ def status_after_launch(device: torch.device) -> None:
 
 
 def poll_status(device: torch.device, what: str = "an earlier e3nn_b200 kernel") -> None:
-    """Raise if an earlier launch on `device` has reported a condition.  Never waits."""
+    """Raise if an earlier launch on `device` has reported a condition.  Waits only when there is one to raise."""
     st = _status.get(device.index if device.index is not None else torch.cuda.current_device())
     if st is None or st.value.value == 0 or torch.cuda.is_current_stream_capturing():
         return
-    code, st.value.value = st.value.value, 0
-    _raise_status(code, what)
+    code = st.take()
+    if code != 0:      # (another thread may have raised it)
+        _raise_status(code, what)
 
 
 def last_status_code(device: Optional[torch.device] = None) -> int:
@@ -126,9 +136,8 @@ def last_status_code(device: Optional[torch.device] = None) -> int:
 def check_status(device: Optional[torch.device] = None, what: str = "e3nn_b200 kernels") -> None:
     """Synchronise `device` and raise if any launch since the last check reported a condition."""
     dev = device if device is not None else torch.device("cuda", torch.cuda.current_device())
-    code = last_status_code(dev)
+    code = _device_status(dev).take()
     if code != 0:
-        _device_status(dev).value.value = 0
         _raise_status(code, what)
 
 

@@ -34,11 +34,29 @@ def test_status_is_raised_by_the_next_call_without_a_sync():
     word = _lib.status_word(dev)
     assert _lib.core().e3b_selftest_bounded_wait(_lib._ptr(word), 200, _lib.stream_ptr()) == 0
     _lib.status_after_launch(dev)
-    torch.cuda.synchronize()                      # the read-back has landed; poll_status itself never waits
+    torch.cuda.synchronize()                      # the kernel has written the word; poll_status looks at it without waiting
     lin = o3.Linear("8x0e+8x1o", "8x0e+8x1o").to(dev)
     with pytest.raises(e3nn_b200.E3BError):
         lin(torch.randn(4, 32, device=dev))
     lin(torch.randn(4, 32, device=dev))           # cleared
+    e3nn_b200.check_status()
+
+
+def test_one_launch_with_many_bad_indices_raises_once():
+    dev = torch.device("cuda", 0)
+    e3nn_b200.check_status()
+    tp = layouts.conv_tensor_product("8x0e+8x1o+8x2e", "0e+1o+2e", layouts.ALL_L2)
+    N, E = 1000, 400_000
+    rowptr = torch.arange(N + 1, device=dev) * (E // N)
+    lin, x = o3.Linear("8x0e+8x1o", "8x0e+8x1o").to(dev), torch.randn(4, 32, device=dev)
+    lin(x)
+    e3nn_b200.conv_uvu(tp, torch.randn(N, tp.irreps_in1.dim, device=dev), torch.randn(E, 3, device=dev),
+                       torch.full((E,), N, device=dev), rowptr, torch.randn(E, tp.weight_numel, device=dev), edge_attr_is_vector=True)
+    with pytest.raises(IndexError):
+        for _ in range(100_000):                  # until the first of the reports is seen, with the kernel still running
+            lin(x)
+    torch.cuda.synchronize()
+    lin(x)                                        # the launch's other reports are not raised again
     e3nn_b200.check_status()
 
 
