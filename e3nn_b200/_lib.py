@@ -198,7 +198,10 @@ def core() -> ctypes.CDLL:
                                            c_int, c_int64, c_void_p]
         lib.e3b_dense_bwd_w.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p]
         lib.e3b_dense_bwd_x.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p]
+        lib.e3b_dense_bwd_x_ordered.argtypes = lib.e3b_dense_bwd_x.argtypes[:-1] + [c_void_p, c_int64, c_void_p]
         lib.e3b_dense_bwd_x_supported.argtypes = [c_void_p]
+        lib.e3b_dense_bwd_x_scratch_bytes.argtypes = [c_void_p, c_int64]
+        lib.e3b_dense_bwd_x_scratch_bytes.restype = c_int64
         lib.e3b_fill_columns.argtypes = [c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
         spec = [c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_float, c_int]
         lib.e3b_radial_embed_fwd.argtypes = [c_void_p] * 5 + [c_int64, c_int64] + spec + [c_void_p, c_void_p, c_void_p, c_void_p]
@@ -225,7 +228,7 @@ def core() -> ctypes.CDLL:
         lib.e3b_selftest_bounded_wait.argtypes = [c_void_p, ctypes.c_uint, c_void_p]
         lib.e3b_selftest_bounded_wait.restype = c_int
         for name in ("e3b_sh_fwd", "e3b_sh_bwd", "e3b_csr_from_dst", "e3b_dense_fwd", "e3b_dense_fwd_gate", "e3b_dense_bwd_w", "e3b_dense_bwd_x",
-                     "e3b_dense_bwd_x_supported", "e3b_fill_columns",
+                     "e3b_dense_bwd_x_ordered", "e3b_dense_bwd_x_supported", "e3b_fill_columns",
                      "e3b_radial_embed_fwd", "e3b_radial_embed_bwd", "e3b_radial_embed_bwd_all", "e3b_matmul_tn", "e3b_neighbor_count", "e3b_neighbor_fill",
                      "e3b_neighbor_count_rows", "e3b_neighbor_fill_rows",
                      "e3b_gate_fwd", "e3b_gate_fwd_channels", "e3b_gate_bwd", "e3b_gate_bwd_channels"):

@@ -911,12 +911,14 @@ __global__ void __launch_bounds__(kThreads, 4) dense_rows_wgrad_kernel(const int
 //     grad_x1[z, u, i] += sum_k T_p[z, k, i] Q[z, u, k]
 //     M[z, i, k]       = sum_u x1[z, u, i] Q[z, u, k],   grad_x2[z, v, j] += sum_{i, k} C_ijk M[z, i, k]
 // A block owns one input irrep's 32 channels for 32 rows; a thread owns one row and 8 channels for every k and i, so
-// the sums over k stay in its registers, and the sums over u cross 4 lanes.
+// the sums over k stay in its registers, and the sums over u cross 4 lanes.  Its share of grad_x2 goes to a partial of its
+// own; a second kernel adds the partials in a fixed order.
 constexpr int kBxZ = 32, kBxU = 8;
 
 struct BwdXLaunch {
     int n;
     int first_block[kMaxGroups + 1];
+    int first_part[kMaxGroups];          // of all blocks of 32 channels of the first operand, the group's first
     int16_t group[kMaxGroups];
 };
 
@@ -1049,7 +1051,8 @@ __device__ __forceinline__ void bwd_x_step(const Part2& P, const BwdXStep& s, co
 template <int D1, bool NEED1, bool NEED2>
 __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, const float* __restrict__ x1, const float* __restrict__ x2,
                                             const float* __restrict__ W, const float* __restrict__ gout, float* __restrict__ g1,
-                                            float* __restrict__ g2, int64_t Z, int block, const BwdXShared& S) {
+                                            float* __restrict__ g2, float* __restrict__ partial, int64_t Z, int block, int first_part,
+                                            const BwdXShared& S) {
     const int x1off = in[0], m1 = in[1], ublocks = (m1 + 31) / 32;
     const int64_t z0 = static_cast<int64_t>(block / ublocks) * kBxZ;
     const int u0 = (block % ublocks) * 32, nu = min(32, m1 - u0);
@@ -1107,7 +1110,11 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
         for (int r = 0; r < 8; ++r) {
             const int zl = warp * 8 + r;
             if (z0 + zl >= Z) break;
-            for (int e = lane; e < d2row; e += 32) atomicAdd(g2 + (z0 + zl) * d2row + e, S.g2[zl * S.ld2 + e]);
+            float* o = (partial ? partial + (first_part + block % ublocks) * Z * d2row : g2) + (z0 + zl) * d2row;
+            for (int e = lane; e < d2row; e += 32) {
+                if (partial) o[e] = S.g2[zl * S.ld2 + e];
+                else atomicAdd(o + e, S.g2[zl * S.ld2 + e]);
+            }
         }
     }
 }
@@ -1116,7 +1123,8 @@ template <bool NEED1, bool NEED2>
 __global__ void __launch_bounds__(kThreads, 3) dense_tile_bwd_x_kernel(const int32_t* __restrict__ plan, const float* __restrict__ x1,
                                                                        const float* __restrict__ x2, const float* __restrict__ W,
                                                                        const float* __restrict__ gout, float* __restrict__ g1,
-                                                                       float* __restrict__ g2, int64_t Z, int g_floats, BwdXLaunch L) {
+                                                                       float* __restrict__ g2, float* __restrict__ partial, int64_t Z,
+                                                                       int g_floats, BwdXLaunch L) {
     extern __shared__ __align__(16) float smem[];
     const Part2 P(plan);
     BwdXShared S;
@@ -1134,14 +1142,37 @@ __global__ void __launch_bounds__(kThreads, 3) dense_tile_bwd_x_kernel(const int
     const int32_t* in = P.in_group(L.group[s]);
     const int block = static_cast<int>(blockIdx.x) - L.first_block[s];
     switch (in[2]) {
-        case 1: bwd_x_block<1, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, Z, block, S); break;
-        case 3: bwd_x_block<3, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, Z, block, S); break;
-        case 5: bwd_x_block<5, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, Z, block, S); break;
-        default: bwd_x_block<7, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, Z, block, S); break;
+        case 1: bwd_x_block<1, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
+        case 3: bwd_x_block<3, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
+        case 5: bwd_x_block<5, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
+        default: bwd_x_block<7, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
     }
 }
 
+// out[i] = sum of partial[0..parts)[i], i < count.
+__global__ void __launch_bounds__(256) dense_bwd_x_sum_kernel(const float* __restrict__ partial, int parts, int64_t count, float* __restrict__ out) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    float v = 0.0f;
+#pragma unroll 4
+    for (int p = 0; p < parts; ++p) v += partial[p * count + i];
+    out[i] = v;
+}
+
 constexpr int kMaxShared = 227 * 1024;
+
+// Blocks of 32 channels of the first operand, each with a partial of grad_x2.
+inline int bwd_x_parts(const Part2& P) {
+    int parts = 0;
+    for (int g = 0; g < P.n_in(); ++g) parts += (P.in_group(g)[1] + 31) / 32;
+    return parts;
+}
+
+// Rows whose partials are held at a time: at most 128 MB of them, at least 16 row tiles.
+inline int64_t bwd_x_slab(const int32_t* plan, int parts, int64_t rows) {
+    const int64_t fit = (int64_t{128} << 20) / (static_cast<int64_t>(sizeof(float)) * parts * std::max(plan[2], 1)) / kBxZ * kBxZ;
+    return std::min<int64_t>(rows, std::max<int64_t>(fit, 16 * kBxZ));
+}
 
 // Floats of one cotangent buffer of dense_tile_bwd_x_kernel; the two together later hold the grad_x1 tile.
 inline int bwd_x_g_floats(int d1max, int d3max) {
@@ -1378,10 +1409,10 @@ int launch_dense_tile_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, c
 
 template <bool NEED1, bool NEED2>
 static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
-                        const float* gout, float* g1, float* g2, int64_t Z, cudaStream_t s) {
+                        const float* gout, float* g1, float* g2, float* partial, int64_t Z, cudaStream_t s) {
     const Part2 P(plan_host);
     const size_t bytes = bwd_x_shared(plan_host, P.d1max(), P.d3max(), NEED2);
-    int g0 = 0;
+    int g0 = 0, part = 0;
     while (g0 < P.n_in()) {
         BwdXLaunch L;
         L.n = 0;
@@ -1389,7 +1420,9 @@ static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const
         for (; g0 < P.n_in() && L.n < kMaxGroups; ++g0) {
             const int32_t* in = P.in_group(g0);
             L.first_block[L.n] = static_cast<int>(blocks);
+            L.first_part[L.n] = part;
             L.group[L.n] = static_cast<int16_t>(g0);
+            part += (in[1] + 31) / 32;
             blocks += ceil_div(Z, kBxZ) * ceil_div(in[1], 32);
             if (too_many_blocks(blocks)) return fail(E3B_ERR_ARG, "dense_bwd_x: too many rows");
             ++L.n;
@@ -1397,7 +1430,7 @@ static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const
         L.first_block[L.n] = static_cast<int>(blocks);
         auto kernel = dense_tile_bwd_x_kernel<NEED1, NEED2>;
         E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
-        kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, weight, gout, g1, g2, Z,
+        kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, weight, gout, g1, g2, partial, Z,
                                                                       bwd_x_g_floats(P.d1max(), P.d3max()), L);
         if (int rc = check_launch("e3b_dense_bwd_x")) return rc;
     }
@@ -1413,19 +1446,61 @@ extern "C" int e3b_dense_bwd_x_supported(const int32_t* plan_host) {
     return P.n_in() > 0 && P.d1max() <= 7 && P.d3max() <= 7 && bwd_x_shared(plan_host, P.d1max(), P.d3max(), true) <= static_cast<size_t>(kMaxShared);
 }
 
-extern "C" int e3b_dense_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
-                               const float* grad_out, float* grad_x1, float* grad_x2, int64_t num_rows, void* stream) {
-    using namespace e3b;
+namespace e3b {
+// partial: nullptr (grad_x2 by atomics) or bwd_x_parts() x rows x d2 floats (grad_x2 itself when there is one part).
+static int bwd_x_rows(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight, const float* gout,
+                      float* g1, float* g2, float* partial, int64_t Z, cudaStream_t s) {
+    if (g1 && g2) return launch_bwd_x<true, true>(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, partial, Z, s);
+    if (g1) return launch_bwd_x<true, false>(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, partial, Z, s);
+    return launch_bwd_x<false, true>(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, partial, Z, s);
+}
+
+static int bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight, const float* gout,
+                 float* g1, float* g2, int64_t Z, bool ordered, void* scratch, int64_t scratch_bytes, void* stream) {
     if (!plan_host || plan_host[0] != kDenseMagic) return fail(E3B_ERR_ARG, "dense_bwd_x: bad plan");
-    if (num_rows < 0) return fail(E3B_ERR_ARG, "dense_bwd_x: negative row count");
-    if (num_rows == 0 || (!grad_x1 && !grad_x2)) return E3B_OK;
-    if (!plan_dev || !x1 || !x2 || !weight || !grad_out) return fail(E3B_ERR_ARG, "dense_bwd_x: null pointer");
+    if (Z < 0) return fail(E3B_ERR_ARG, "dense_bwd_x: negative row count");
+    if (Z == 0 || (!g1 && !g2)) return E3B_OK;
+    if (!plan_dev || !x1 || !x2 || !weight || !gout) return fail(E3B_ERR_ARG, "dense_bwd_x: null pointer");
     if (!e3b_dense_bwd_x_supported(plan_host)) return fail(E3B_ERR_UNSUPPORTED, "dense_bwd_x: irreps above l = 3 or too wide");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Part2 P(plan_host);
-    if (grad_x1 && !P.covers_x1()) E3B_CUDA_TRY(cudaMemsetAsync(grad_x1, 0, sizeof(float) * num_rows * plan_host[1], s));
-    if (grad_x2) E3B_CUDA_TRY(cudaMemsetAsync(grad_x2, 0, sizeof(float) * num_rows * plan_host[2], s));
-    if (grad_x1 && grad_x2) return launch_bwd_x<true, true>(plan_host, plan_dev, x1, x2, weight, grad_out, grad_x1, grad_x2, num_rows, s);
-    if (grad_x1) return launch_bwd_x<true, false>(plan_host, plan_dev, x1, x2, weight, grad_out, grad_x1, grad_x2, num_rows, s);
-    return launch_bwd_x<false, true>(plan_host, plan_dev, x1, x2, weight, grad_out, grad_x1, grad_x2, num_rows, s);
+    const int64_t d1 = plan_host[1], d2 = plan_host[2], dout = plan_host[3];
+    const int parts = bwd_x_parts(P);
+    if (g1 && !P.covers_x1()) E3B_CUDA_TRY(cudaMemsetAsync(g1, 0, sizeof(float) * Z * d1, s));
+    if (!g2 || parts == 1) return bwd_x_rows(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, g2, Z, s);
+    if (!ordered) {
+        E3B_CUDA_TRY(cudaMemsetAsync(g2, 0, sizeof(float) * Z * d2, s));
+        return bwd_x_rows(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, nullptr, Z, s);
+    }
+    const int64_t slab = bwd_x_slab(plan_host, parts, Z);
+    if (!scratch || scratch_bytes < static_cast<int64_t>(sizeof(float)) * parts * slab * d2) return fail(E3B_ERR_ARG, "dense_bwd_x: scratch too small");
+    float* partial = static_cast<float*>(scratch);
+    for (int64_t z = 0; z < Z; z += slab) {
+        const int64_t n = std::min(slab, Z - z), count = n * d2;
+        if (int rc = bwd_x_rows(plan_host, plan_dev, x1 + z * d1, x2 + z * d2, weight, gout + z * dout, g1 ? g1 + z * d1 : nullptr, g2 + z * d2,
+                                partial, n, s))
+            return rc;
+        dense_bwd_x_sum_kernel<<<static_cast<unsigned>(ceil_div(count, 256)), 256, 0, s>>>(partial, parts, count, g2 + z * d2);
+        if (int rc = check_launch("e3b_dense_bwd_x")) return rc;
+    }
+    return E3B_OK;
+}
+}  // namespace e3b
+
+extern "C" int64_t e3b_dense_bwd_x_scratch_bytes(const int32_t* plan_host, int64_t num_rows) {
+    using namespace e3b;
+    if (!e3b_dense_bwd_x_supported(plan_host) || num_rows <= 0) return 0;
+    const int parts = bwd_x_parts(Part2(plan_host));
+    return parts == 1 ? 0 : static_cast<int64_t>(sizeof(float)) * parts * bwd_x_slab(plan_host, parts, num_rows) * plan_host[2];
+}
+
+extern "C" int e3b_dense_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
+                               const float* grad_out, float* grad_x1, float* grad_x2, int64_t num_rows, void* stream) {
+    return e3b::bwd_x(plan_host, plan_dev, x1, x2, weight, grad_out, grad_x1, grad_x2, num_rows, false, nullptr, 0, stream);
+}
+
+extern "C" int e3b_dense_bwd_x_ordered(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
+                                       const float* grad_out, float* grad_x1, float* grad_x2, int64_t num_rows, void* scratch,
+                                       int64_t scratch_bytes, void* stream) {
+    return e3b::bwd_x(plan_host, plan_dev, x1, x2, weight, grad_out, grad_x1, grad_x2, num_rows, true, scratch, scratch_bytes, stream);
 }

@@ -60,7 +60,7 @@ class _UvuFunction(torch.autograd.Function):
 
 class _UvwFunction(torch.autograd.Function):
     """Weight-shared or per-row 'uvw' paths: forward on the engine the module's ``math_mode`` selects; gradients
-    w.r.t. the two operands by ``e3b_dense_bwd_x``, or as two derived 'uvw' products of the cotangent
+    w.r.t. the two operands by ``e3b_dense_bwd_x_ordered``, or as two derived 'uvw' products of the cotangent
     (``TensorProduct._vjp_module``: per-row weights, l > 3, a tensor-core mode's first operand alone), w.r.t. shared weights by ``e3b_dense_bwd_w``, w.r.t. per-row weights by ``TensorProduct._uvw_row_weight_grad``."""
 
     @staticmethod
@@ -85,10 +85,12 @@ class _UvwFunction(torch.autograd.Function):
             if tp._uvw_bwd_x_ok() and (need2 or (need1 and tp.math_mode == "fp32")):
                 g1 = torch.empty_like(x1) if need1 else None
                 g2 = torch.empty_like(x2) if need2 else None
+                core, plan = _lib.core(), tp._plan_host.ctypes.data
+                scratch = torch.empty(core.e3b_dense_bwd_x_scratch_bytes(plan, x1.shape[0]) if need2 else 0, dtype=torch.uint8, device=g.device)
                 with torch.cuda.device(g.device):
-                    rc = _lib.core().e3b_dense_bwd_x(tp._plan_host.ctypes.data, _lib._ptr(tp._plan_on(g.device)), _lib._ptr(x1),
-                                                     _lib._ptr(x2), _lib._ptr(w), _lib._ptr(g), _lib._ptr(g1), _lib._ptr(g2),
-                                                     x1.shape[0], _lib.stream_ptr())
+                    rc = core.e3b_dense_bwd_x_ordered(plan, _lib._ptr(tp._plan_on(g.device)), _lib._ptr(x1), _lib._ptr(x2), _lib._ptr(w),
+                                                      _lib._ptr(g), _lib._ptr(g1), _lib._ptr(g2), x1.shape[0], _lib._ptr(scratch),
+                                                      scratch.numel(), _lib.stream_ptr())
                 _lib.check(rc, "e3b_dense_bwd_x")
                 need1 = need2 = False
             if need1:
@@ -439,7 +441,7 @@ class TensorProduct(torch.nn.Module):
         return out
 
     def _uvw_bwd_x_ok(self) -> bool:
-        """Whether ``e3b_dense_bwd_x`` covers the 'uvw' paths (shared weights, l <= 3)."""
+        """Whether ``e3b_dense_bwd_x_ordered`` covers the 'uvw' paths (shared weights, l <= 3)."""
         if not hasattr(self, "_bwd_x_ok"):
             self._bwd_x_ok = bool(self.shared_weights and _lib.core().e3b_dense_bwd_x_supported(self._plan_host.ctypes.data))
         return self._bwd_x_ok

@@ -84,6 +84,25 @@ def test_fp32_product_tiles(layout, rows):
         assert rel_err(torch.autograd.grad(other, leaf, go.to(DEV))[0].cpu(), ref_g[n]) < 1e-5
 
 
+@pytest.mark.parametrize("layout,rows", [(("65x0e+33x1o+32x2e", "1x0e+1x1o+1x2e", "32x0e+32x1o+32x2e"), 4000),      # 6 blocks of channels
+                                         (("320x0e+64x1o", "300x0e+60x1o", "2x0e"), 6000),                      # 12, rows in two turns
+                                         (("32x0e", "1x0e+1x1o", "8x0e+8x1o"), 100)])                           # one: no partials
+def test_fp32_product_second_operand_gradient_repeats(layout, rows):
+    """Bit for bit: the same on every call, and for a row whatever rows stand beside it."""
+    g = torch.Generator().manual_seed(rows)
+    tp = o3.FullyConnectedTensorProduct(*layout).to(DEV)
+    x, y, go = (torch.randn(rows, d, generator=g).to(DEV) for d in (tp.irreps_in1.dim, tp.irreps_in2.dim, tp.irreps_out.dim))
+
+    def grad(sl):
+        leaf = y[sl].clone().requires_grad_(True)
+        return torch.autograd.grad(tp(x[sl], leaf), leaf, go[sl])[0]
+
+    first = grad(slice(None))
+    assert torch.equal(grad(slice(rows - 70, None)), first[rows - 70 :])
+    for _ in range(5):
+        assert torch.equal(grad(slice(None)), first)
+
+
 @pytest.mark.parametrize("tail", ["2x3o", "2x0e"])
 def test_fp32_product_many_outputs_wide_second_operand(tail):
     """33 output irreps (32 go out in one launch) and a second operand of 1,280 columns: with the l = 3 irrep last, the first 32
