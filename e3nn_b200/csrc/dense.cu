@@ -11,7 +11,7 @@
 // the tensor-core mode lives in uvw_tc.cu.
 //
 // Plan layout (int32 words, floats bit-cast), built by e3nn_b200/o3/_dense_plan.py:
-//   [0] magic 0x65336250  [1] d1  [2] d2  [3] dout  [4] n_groups  [5] n_paths  [6] total words
+//   [0] magic 0x65336251 (0x65336250: no second part)  [1] d1  [2] d2  [3] dout  [4] n_groups  [5] n_paths  [6] total words
 //   [7] off_groups [8] off_kent [9] off_pathk [10] off_cg   [11] max K over groups
 //   groups  : n_groups x 6 : out_off, mul_out, dim3, K, kent_start, w_stride
 //   kent    : sum K   x 4 : path, x1off, x2off (-1: factor 1), wbase
@@ -264,11 +264,11 @@ extern "C" int e3b_dense_fwd(const int32_t* plan_host, const int32_t* plan_dev, 
                              const float* weight, int64_t weight_row_stride, float* out, int64_t num_rows,
                              int accumulate, void* stream) {
     using namespace e3b;
-    if (!plan_host || plan_host[0] != kDenseMagic) return fail(E3B_ERR_ARG, "dense_fwd: bad plan");
+    if (!any_plan(plan_host)) return fail(E3B_ERR_ARG, "dense_fwd: bad plan");
     if (num_rows < 0) return fail(E3B_ERR_ARG, "dense_fwd: negative row count");
     if (num_rows == 0) return E3B_OK;
     if (!plan_dev || !x1 || !out || !weight) return fail(E3B_ERR_ARG, "dense_fwd: null pointer");
-    if (weight_row_stride == 0)
+    if (weight_row_stride == 0 && whole_plan(plan_host))
         return launch_dense_tile_fwd(plan_host, plan_dev, x1, x2, weight, out, num_rows, accumulate, static_cast<cudaStream_t>(stream));
     const DenseGateEpilogue none{nullptr, nullptr, nullptr, nullptr, 0, 0};
     return launch_dense_groups(plan_host, plan_dev, x1, x2, weight, weight_row_stride, out, num_rows, accumulate, none, 0,
@@ -279,7 +279,7 @@ extern "C" int e3b_dense_fwd_gate(const int32_t* plan_host, const int32_t* plan_
                                   const int32_t* gate_table, const float* gate_const, float* gates, int n_slots,
                                   float* out, int dout, int64_t num_rows, void* stream) {
     using namespace e3b;
-    if (!plan_host || plan_host[0] != kDenseMagic) return fail(E3B_ERR_ARG, "dense_fwd_gate: bad plan");
+    if (!any_plan(plan_host)) return fail(E3B_ERR_ARG, "dense_fwd_gate: bad plan");
     if (num_rows < 0 || n_slots < 0 || dout < 0) return fail(E3B_ERR_ARG, "dense_fwd_gate: negative size");
     if (num_rows == 0) return E3B_OK;
     if (!plan_dev || !x || !weight || !gate_table || !gate_const || !out || (n_slots > 0 && !gates))
@@ -287,7 +287,8 @@ extern "C" int e3b_dense_fwd_gate(const int32_t* plan_host, const int32_t* plan_
     const DenseGateEpilogue ep{gate_table, gate_const, gates, out, n_slots, dout};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     bool done = false;
-    if (int rc = launch_dense_rows_gate(plan_host, plan_dev, x, weight, ep, num_rows, s, &done)) return rc;
+    if (whole_plan(plan_host))
+        if (int rc = launch_dense_rows_gate(plan_host, plan_dev, x, weight, ep, num_rows, s, &done)) return rc;
     if (done) return E3B_OK;
     // scalars and gates first: the launches of the gated irreps read the activated gates of the same rows
     if (int rc = launch_dense_groups(plan_host, plan_dev, x, nullptr, weight, 0, out, num_rows, 0, ep, 1, s)) return rc;
@@ -297,7 +298,7 @@ extern "C" int e3b_dense_fwd_gate(const int32_t* plan_host, const int32_t* plan_
 extern "C" int e3b_dense_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2,
                                const float* grad_out, float* grad_weight, int64_t num_rows, void* stream) {
     using namespace e3b;
-    if (!plan_host || plan_host[0] != kDenseMagic) return fail(E3B_ERR_ARG, "dense_bwd_w: bad plan");
+    if (!whole_plan(plan_host)) return fail(E3B_ERR_ARG, "dense_bwd_w: bad plan (one without its second part has to be built again)");
     if (num_rows < 0) return fail(E3B_ERR_ARG, "dense_bwd_w: negative row count");
     if (num_rows == 0) return E3B_OK;
     if (!plan_dev || !x1 || !grad_out || !grad_weight) return fail(E3B_ERR_ARG, "dense_bwd_w: null pointer");

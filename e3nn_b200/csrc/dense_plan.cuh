@@ -6,7 +6,11 @@
 
 namespace e3b {
 
-constexpr int kDenseMagic = 0x65336250;
+constexpr int kDenseMagic = 0x65336251;          // a plan with both parts
+constexpr int kDenseMagicFirst = 0x65336250;     // the first part alone, as plans were before there was a second
+
+inline bool whole_plan(const int32_t* plan) { return plan && plan[0] == kDenseMagic; }
+inline bool any_plan(const int32_t* plan) { return plan && (plan[0] == kDenseMagic || plan[0] == kDenseMagicFirst); }
 
 // Gate applied where the contraction's result is still in registers (Linear followed by Gate).  Column c of the
 // contraction's output row is described by tbl[4 c ..] = {kind, destination column, activation, gate slot} and

@@ -1441,7 +1441,7 @@ static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const
 
 extern "C" int e3b_dense_bwd_x_supported(const int32_t* plan_host) {
     using namespace e3b;
-    if (!plan_host || plan_host[0] != kDenseMagic) return 0;
+    if (!whole_plan(plan_host)) return 0;
     const Part2 P(plan_host);
     return P.n_in() > 0 && P.d1max() <= 7 && P.d3max() <= 7 && bwd_x_shared(plan_host, P.d1max(), P.d3max(), true) <= static_cast<size_t>(kMaxShared);
 }
@@ -1457,7 +1457,7 @@ static int bwd_x_rows(const int32_t* plan_host, const int32_t* plan_dev, const f
 
 static int bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight, const float* gout,
                  float* g1, float* g2, int64_t Z, bool ordered, void* scratch, int64_t scratch_bytes, void* stream) {
-    if (!plan_host || plan_host[0] != kDenseMagic) return fail(E3B_ERR_ARG, "dense_bwd_x: bad plan");
+    if (!whole_plan(plan_host)) return fail(E3B_ERR_ARG, "dense_bwd_x: bad plan (one without its second part has to be built again)");
     if (Z < 0) return fail(E3B_ERR_ARG, "dense_bwd_x: negative row count");
     if (Z == 0 || (!g1 && !g2)) return E3B_OK;
     if (!plan_dev || !x1 || !x2 || !weight || !gout) return fail(E3B_ERR_ARG, "dense_bwd_x: null pointer");

@@ -17,7 +17,7 @@ import numpy as np
 from ._irreps import Irreps
 from ._wigner import wigner_3j_numpy
 
-MAGIC = 0x65336250
+MAGIC = 0x65336251          # (..50: plans of the first part alone)
 
 
 _FLOAT, _INT = struct.Struct("<f"), struct.Struct("<i")

@@ -17,7 +17,7 @@ import hashlib
 
 from .. import _lib
 from ..codegen import tc_gemm
-from ._dense_plan import linear_plan
+from ._dense_plan import MAGIC, linear_plan
 from ._irreps import Irreps
 from ._spec import LinearInstruction, normalize_linear_instructions
 
@@ -135,17 +135,7 @@ class Linear(torch.nn.Module):
         live = [ins for ins in self.instructions if 0 not in ins.path_shape]
         self.weight_numel = sum(prod(ins.path_shape) for ins in live if ins.i_in != -1)
         self.bias_numel = sum(prod(ins.path_shape) for ins in live if ins.i_in == -1)
-        # the flat weight vector skips empty instructions, exactly as the reference's code generator does
-        packed = [ins if 0 not in ins.path_shape else ins._replace(path_shape=(0, 0)) for ins in self.instructions]
-        self._plan_host, written = linear_plan(irreps_in, irreps_out, packed, transpose=False)
-        self._plan_t_host, read = linear_plan(irreps_in, irreps_out, packed, transpose=True)
-        self._reads_all = all(i in read for i, (mul, ir) in enumerate(irreps_in) if mul * ir.dim > 0)
-        self._plan_dev = {}
-        # tensor-core modules (None when the multiplicities do not fit the 32-wide K chunks / 16-wide N)
-        tag = hashlib.sha1(repr((str(irreps_in), str(irreps_out), [(i.i_in, i.i_out, i.path_shape, repr(i.path_weight))
-                                                                      for i in packed])).encode()).hexdigest()[:14]
-        self._tc_fwd = tc_gemm.linear_gemm_spec(irreps_in, irreps_out, packed, False, "lin" + tag + "f")
-        self._tc_bwd = tc_gemm.linear_gemm_spec(irreps_in, irreps_out, packed, True, "lin" + tag + "t")
+        written = self._plan()
         offs = irreps_out.offsets()
         bias_out = [ins.i_out for ins in self.instructions if ins.i_in == -1 and 0 not in ins.path_shape]
         self._unwritten = [
@@ -180,6 +170,27 @@ class Linear(torch.nn.Module):
         for i, ins in enumerate(self.instructions):
             offset = sum(prod(p.path_shape) for p in self.instructions[:i])
             self.weight_index_slices.append(LinearSlices(slice(offset, offset + prod(ins.path_shape), None), ins.path_shape))
+
+    def _plan(self) -> List[int]:
+        """Dense plans and tensor-core modules of the instructions; returns the output irreps written."""
+        irreps_in, irreps_out = self.irreps_in, self.irreps_out
+        # the flat weight vector skips empty instructions, exactly as the reference's code generator does
+        packed = [ins if 0 not in ins.path_shape else ins._replace(path_shape=(0, 0)) for ins in self.instructions]
+        self._plan_host, written = linear_plan(irreps_in, irreps_out, packed, transpose=False)
+        self._plan_t_host, read = linear_plan(irreps_in, irreps_out, packed, transpose=True)
+        self._reads_all = all(i in read for i, (mul, ir) in enumerate(irreps_in) if mul * ir.dim > 0)
+        self._plan_dev = {}
+        # tensor-core modules (None when the multiplicities do not fit the 32-wide K chunks / 16-wide N)
+        tag = hashlib.sha1(repr((str(irreps_in), str(irreps_out), [(i.i_in, i.i_out, i.path_shape, repr(i.path_weight))
+                                                                      for i in packed])).encode()).hexdigest()[:14]
+        self._tc_fwd = tc_gemm.linear_gemm_spec(irreps_in, irreps_out, packed, False, "lin" + tag + "f")
+        self._tc_bwd = tc_gemm.linear_gemm_spec(irreps_in, irreps_out, packed, True, "lin" + tag + "t")
+        return written
+
+    def __setstate__(self, state) -> None:
+        super().__setstate__(state)
+        if int(self._plan_host[0]) != MAGIC:      # saved with a plan of another form
+            self._plan()
 
     def __repr__(self) -> str:
         return f"{self.__class__.__name__}({self.irreps_in} -> {self.irreps_out} | {self.weight_numel} weights)"

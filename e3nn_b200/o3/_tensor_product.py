@@ -23,7 +23,7 @@ import warnings
 import torch
 
 from .. import _lib
-from ._dense_plan import uvw_plan
+from ._dense_plan import MAGIC, uvw_plan
 from ._irreps import Irreps
 from ._spec import SUPPORTED_MODES, Instruction, TPSpec, normalize_tp_instructions
 
@@ -221,6 +221,14 @@ class TensorProduct(torch.nn.Module):
         self._plan_dev = {}
         if self._uvw_ids:
             self._plan_host, self._uvw_written = uvw_plan(self._spec)
+
+    def __setstate__(self, state) -> None:
+        super().__setstate__(state)
+        if self._plan_host is not None and int(self._plan_host[0]) != MAGIC:      # saved with a plan of another form
+            self._plan_host, self._uvw_written = uvw_plan(self._spec)
+            self._plan_dev = {}
+            for name in ("_tcg_spec", "_tc_ok", "_bwd_x_ok"):
+                self.__dict__.pop(name, None)
 
     def __repr__(self) -> str:
         npath = sum(prod(i.path_shape) for i in self.instructions)

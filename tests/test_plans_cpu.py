@@ -15,7 +15,7 @@ def _i2f(v: int) -> float:
 
 def run_plan(plan: np.ndarray, x1: np.ndarray, x2, W: np.ndarray, accumulate_into=None) -> np.ndarray:
     """out[z, out_off + w * dim3 + k] (+)= sum_K A[z, k, K] * W[wbase(K) + w * wstride], A from the CG triples."""
-    assert plan[0] == MAGIC
+    assert plan[0] in (MAGIC, 0x65336250)
     d1, d2, dout, n_groups = (int(v) for v in plan[1:5])
     off_groups, off_kent, off_pathk, off_cg = (int(v) for v in plan[7:11])
     assert x1.shape[1] == d1 and (x2 is None or x2.shape[1] == d2)
@@ -100,6 +100,41 @@ def test_linear_plan_rejects_nothing_it_accepts_in_forward():
     # empty instruction lists and zero-multiplicity irreps build (degenerate) plans
     plan, written = linear_plan(o3.Irreps("0x0e+2x1o"), o3.Irreps("3x1o"), o3.Linear("0x0e+2x1o", "3x1o").instructions)
     assert written == [0] and int(plan[4]) == 1
+
+
+def _first_part(plan: np.ndarray) -> np.ndarray:
+    """The plan as it was before there was a second part."""
+    old = plan[: int(plan[10]) + _cg_words(plan)].copy()
+    old[0], old[6] = 0x65336250, len(old)
+    return old
+
+
+def _cg_words(plan: np.ndarray) -> int:
+    paths = [int(plan[int(plan[9]) + p]) for p in range(int(plan[5]))] + [int(plan[10])]
+    return max([3 * int(plan[a] + plan[a + 1]) for p, q in zip(paths, paths[1:]) for a in range(p, q, 2)], default=0)
+
+
+def test_plans_without_a_second_part():
+    """Modules saved with such plans get new ones when they are loaded; the entry points that need the second part refuse."""
+    import pickle
+
+    from e3nn_b200 import _lib
+
+    tp, lin = o3.FullyConnectedTensorProduct("3x0e+2x1o", "1x0e+1x1o", "2x0e+3x1o"), o3.Linear("3x0e+2x1o", "4x0e+2x1o")
+    written, plans = tp._uvw_written, (tp._plan_host, lin._plan_host, lin._plan_t_host)
+    tp._plan_host, lin._plan_host, lin._plan_t_host = (_first_part(p) for p in plans)
+    del lin._reads_all
+    x1, x2 = np.random.randn(4, tp.irreps_in1.dim), np.random.randn(4, tp.irreps_in2.dim)
+    w = tp.weight.detach().double().numpy()
+    assert np.array_equal(run_plan(tp._plan_host, x1, x2, w), run_plan(plans[0], x1, x2, w))
+    tp2, lin2 = (pickle.loads(pickle.dumps(m)) for m in (tp, lin))
+    for got, want in zip((tp2._plan_host, lin2._plan_host, lin2._plan_t_host), plans):
+        assert np.array_equal(got, want)
+    assert lin2._reads_all and tp2._uvw_written == written
+    core, host = _lib.core(), tp._plan_host.ctypes.data
+    assert core.e3b_dense_bwd_x_supported(host) == 0 and core.e3b_dense_bwd_x_supported(plans[0].ctypes.data) == 1
+    assert core.e3b_dense_bwd_w(host, None, None, None, None, None, 5, None) == -1
+    assert core.e3b_dense_bwd_x(host, None, None, None, None, None, None, None, 5, None) == -1
 
 
 # ----------------------------------------------------------------------------- planner of the post-coupling 'uvw' kernel
