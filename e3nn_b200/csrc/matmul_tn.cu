@@ -3,8 +3,9 @@
 // Bound by the FP32 pipe: 64 x 1472 entries over 429,000 rows are 81 GFLOP, 1.1 ms at 148 x 128 multiply-adds a clock, while
 // the rows are 2.6 GB, 0.4 ms.  A block owns 64 x 256 entries, 8 x 16 a thread, which read 6 x 16 bytes of shared memory for 64
 // packed multiply-adds (FFMA2: half the issue slots); rows arrive by cp.async four stages ahead.  The rows are split over
-// whole waves, at most 2,048 rows a block, and a second kernel adds the partial matrices in a fixed order: the error stays
-// below that of the library's fp32 product, which sums longer runs (429,000 rows: 8.1e-7 against 1.7e-6).
+// whole waves, up to eight; a block sums 2,048 rows at a time in registers and adds the runs in its partial matrix, and a
+// second kernel adds the partial matrices, all in a fixed order: the error stays below that of the library's fp32 product,
+// which sums longer runs (429,000 rows: 8.1e-7 against 1.7e-6).
 // Against that product, 64 x 1472: 5,000 rows 51 -> 35 us, 15,600 127 -> 71, 105,000 500 -> 404, 429,000 1690 -> 1582.  With
 // 8 x 8 a thread 39, 76, 419 and 1609 us; FFMA in place of FFMA2 is 5 - 10 % slower than that.
 #include "common.cuh"
@@ -15,7 +16,7 @@ namespace e3b {
 namespace {
 
 constexpr int kTnM = 64, kTnRows = 16, kTnStages = 4, kTnThreads = 128;
-constexpr int64_t kTnMostRows = 2048;     // rows of a block, up to eight waves
+constexpr int64_t kTnMostRows = 2048;     // rows summed in registers
 
 template <int TN>
 __host__ __device__ constexpr int tn_stage_floats() { return kTnRows * (kTnM + TN); }
@@ -66,6 +67,22 @@ __global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kerne
         if (step < steps) tn_fetch<TN, VEC>(s, s + kTnRows * kTnM, x, g, z_begin + step * kTnRows, z_end, m0, n0, M, N);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // this run's sums into the block's own entries of `out`, which hold the runs before
+    float* o = out + static_cast<int64_t>(blockIdx.z) * M * N;
+    auto flush = [&](bool first) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int m = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
+#pragma unroll
+            for (int j = 0; j < NP; ++j) {
+                const int n = n0 + (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
+                float* p = o + static_cast<int64_t>(m) * N + n;
+                if (m < M && n < N) p[0] = first ? scale * acc[i][j].x : fmaf(scale, acc[i][j].x, p[0]);
+                if (m < M && n + 1 < N) p[1] = first ? scale * acc[i][j].y : fmaf(scale, acc[i][j].y, p[1]);
+                acc[i][j] = make_float2(0.0f, 0.0f);
+            }
+        }
+    };
     for (int s = 0; s < kTnStages - 1; ++s) fetch(s);
     for (int64_t step = 0; step < steps; ++step) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kTnStages - 2) : "memory");
@@ -90,18 +107,7 @@ __global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kerne
 #pragma unroll
                 for (int j = 0; j < NP; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
         }
-    }
-    float* o = out + static_cast<int64_t>(blockIdx.z) * M * N;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < NP; ++j) {
-            const int n = n0 + (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
-            if (n < N) o[static_cast<int64_t>(m) * N + n] = scale * acc[i][j].x;
-            if (n + 1 < N) o[static_cast<int64_t>(m) * N + n + 1] = scale * acc[i][j].y;
-        }
+        if (step + 1 == steps || (step + 1) % (kTnMostRows / kTnRows) == 0) flush(step < kTnMostRows / kTnRows);
     }
 }
 

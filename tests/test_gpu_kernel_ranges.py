@@ -245,6 +245,26 @@ def test_dense_layer_weight_gradient(rows, m, n, offset):
         assert core.e3b_matmul_tn(*args, need - 1, _lib.stream_ptr()) == -1
 
 
+def test_dense_layer_weight_gradient_past_eight_waves():
+    """Blocks of 16,384 rows, summed 2,048 at a time.  Bound: twice the random walk of such a run's roundings, 0.3 x 2^-24 x
+    sqrt(2048) of the sums' size (0.3: the mean rounding error of a sum that grows to its last size)."""
+    from e3nn_b200 import _lib
+
+    rows, m, n = 131_072, 2048, 2048
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x, go = torch.randn(rows, m, generator=g, device=DEV), torch.randn(rows, n, generator=g, device=DEV)
+    core, out = _lib.core(), torch.empty(m, n, device=DEV)
+    scratch = torch.empty(core.e3b_matmul_tn_scratch_bytes(rows, m, n), dtype=torch.uint8, device=DEV)
+    assert scratch.numel() == 8 * m * n * 4
+    assert core.e3b_matmul_tn(_lib._ptr(x), _lib._ptr(go), rows, m, n, 0.5, _lib._ptr(out), _lib._ptr(scratch), scratch.numel(),
+                              _lib.stream_ptr()) == 0
+    ref = torch.zeros(m, n, dtype=torch.float64, device=DEV)
+    for z in range(0, rows, 16_384):
+        ref += 0.5 * (x[z : z + 16_384].double().t() @ go[z : z + 16_384].double())
+    err = ((out.double() - ref).norm() / ref.norm()).item()
+    assert err < 2.0**-24 * (4 + 0.6 * 2048**0.5), err
+
+
 # ----------------------------------------------------------------------------- dense layers on tensor cores
 @pytest.mark.parametrize("rows", [1, 33, 127, 1000])
 @pytest.mark.parametrize("width", [96, 1472])
