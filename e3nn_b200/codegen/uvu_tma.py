@@ -230,16 +230,16 @@ __device__ __forceinline__ void v2_team_sync(int team) {{
 // loads) nor the source look-up is on the path of the lane that issues the copies.  Permuted lists took the direct-load
 // kernels before: 150,001 edges, 11 paths, forward 328 -> 130 us, gradients 440 -> 208 us and 297 -> 254 us.
 struct V2Ids {{
-    int64_t* edge;
-    int64_t* src;      // -1: outside [0, num_src)
+    int64_t* edge;     // 0 where the permutation's entry is outside [0, num_edges)
+    int64_t* src;      // -1: that, or a source outside [0, num_src): reported, and the slot is skipped
     __device__ __forceinline__ void load(const int64_t* __restrict__ perm, const int64_t* __restrict__ edge_src, int64_t first,
                                          int64_t e_lo, int64_t e_hi, int64_t num_edges, int64_t num_src, int lane,
                                          int* __restrict__ status) const {{
         const int64_t ee = first + lane;
         if (ee >= e_hi) return;
-        int64_t id = perm ? perm[ee] : ee;
-        if (id < 0 || id >= num_edges) {{ atomicExch(status, 2); id = 0; }}
-        int64_t s = edge_src[id];
+        int64_t id = perm ? perm[ee] : ee, s = -1;
+        if (id >= 0 && id < num_edges) s = edge_src[id];
+        else id = 0;
         if (s < 0 || s >= num_src) {{ atomicExch(status, 2); s = -1; }}
         edge[(ee - e_lo) & 63] = id;
         src[(ee - e_lo) & 63] = s;
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kV2Threads, 1) conv_fwd_tma_kernel(const float
     int64_t e = e_lo;
     int64_t issue = e;          // next slot to stage (leader lane only)
     bool ok = true;
-    // stage slot `issue` (a source out of range has been reported: row 0 is read in its place)
+    // stage slot `issue` (a slot that will be skipped stages row 0)
     auto stage_next = [&](int s) {{
         const int at = static_cast<int>((issue - e_lo) & 63);
         const int64_t sidx = ids.src[at];
@@ -345,7 +345,9 @@ __global__ void __launch_bounds__(kV2Threads, 1) conv_fwd_tma_kernel(const float
             float Y[kD2];
 #pragma unroll
             for (int j = 0; j < kD2; ++j) Y[j] = ybuf[slot * kV2YStride + j];
-{switch([p[1] for p in parts], 12)}
+            if (ids.src[it & 63u] >= 0) {{
+{switch([p[1] for p in parts], 16)}
+            }}
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&empty[s]);
             if (leader && it > 0 && issue < e_hi) {{

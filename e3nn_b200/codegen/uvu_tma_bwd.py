@@ -179,7 +179,7 @@ constexpr int kB2SmemBytes = kB2Teams * kB2RingBytes + kB2Teams * 2 * kB2Depth *
 // One lane per edge: sum the warps' partial grad_Y of a finished batch, apply the harmonics Jacobian, store.
 __device__ __forceinline__ void b2_batch_finish(const float* __restrict__ vec, float* __restrict__ grad_vec, const V2Ids& ids, uint32_t it0,
                                                 int count, const float* dybuf, int lane) {{
-    if (lane < count) {{
+    if (lane < count && ids.src[(it0 + lane) & 63u] >= 0) {{
         const int64_t ee = ids.edge[(it0 + lane) & 63u];
         float gY[kD2];
 #pragma unroll
@@ -291,7 +291,9 @@ __global__ void __launch_bounds__(kB2Threads, 1) conv_bwd_tma_kernel(const float
 #pragma unroll
             for (int j = 0; j < kD2; ++j) Y[j] = ybuf[slot * kB2YStride + j];
 {_indent(dy_decl, 12)}
-{switch([b[1] for b in bodies], 12)}
+            if (ids.src[it & 63u] >= 0) {{
+{switch([b[1] for b in bodies], 16)}
+            }}
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&empty[s]);
             if (leader && it > 0 && issue < e_hi) {{

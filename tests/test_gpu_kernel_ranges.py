@@ -186,6 +186,49 @@ def test_conv_pipelined_permuted_edges(layout, nodes, edges):
         assert rel_err(a.cpu(), b.cpu().double()) < 2e-5
 
 
+@pytest.mark.parametrize("layout", ["cfg3_11", "cfg5_23"])
+@pytest.mark.parametrize("bad", ["source", "perm", "perm_negative"])
+def test_conv_pipelined_skips_a_bad_index(layout, bad):
+    """One slot with a source or a permutation entry out of range: reported, and every other edge and row is what it is without
+    that edge, bit for bit (its weights set to zero give the same sums); 1e-6 x RMS for the atomic node-feature gradient."""
+    g = torch.Generator().manual_seed(3)
+    tp, nodes, edges, slot = layouts.bench_conv_tp(layout), 50, 1500, 777
+    dst, src = torch.randint(0, nodes, (edges,), generator=g), torch.randint(0, nodes, (edges,), generator=g).to(DEV)
+    perm, rowptr = e3nn_b200.csr_from_dst(dst.to(DEV), nodes)
+    lost = int(perm[slot])
+    assert lost != 0
+    x, vec, w = (torch.randn(*s, generator=g).to(DEV) for s in ((nodes, tp.irreps_in1.dim), (edges, 3), (edges, tp.weight_numel)))
+    go = torch.randn(nodes, tp.irreps_out.dim, generator=g).to(DEV)
+
+    def call(src, perm, w):
+        leaves = [t.clone().requires_grad_(True) for t in (x, vec, w)]
+        out = e3nn_b200.conv_uvu(tp, leaves[0], leaves[1], src, rowptr, leaves[2], perm=perm, scale=0.5, edge_attr_is_vector=True)
+        return [out.detach()] + list(torch.autograd.grad(out, leaves, go))
+
+    w_without = w.clone()
+    w_without[lost] = 0.0
+    want = call(src, perm, w_without)
+    e3nn_b200.check_status()
+    bad_src, bad_perm = src.clone(), perm.clone()
+    if bad == "source":
+        bad_src[lost] = nodes
+    else:
+        bad_perm[slot] = edges if bad == "perm" else -1
+    from e3nn_b200 import _lib
+
+    poll, _lib.poll_status = _lib.poll_status, lambda *a: None      # (the report of the forward pass would be raised in the backward)
+    try:
+        got = call(bad_src, bad_perm, w)
+    finally:
+        _lib.poll_status = poll
+    with pytest.raises(IndexError):
+        e3nn_b200.check_status()
+    rest = torch.arange(edges, device=DEV) != lost
+    assert torch.equal(got[0], want[0])
+    assert torch.equal(got[2][rest], want[2][rest]) and torch.equal(got[3][rest], want[3][rest])
+    assert rel_err(got[1].cpu(), want[1].cpu().double()) < 1e-6
+
+
 # ----------------------------------------------------------------------------- edge embedding: gradient of its weights
 @pytest.mark.parametrize("edges", [1, 33, 4001])
 @pytest.mark.parametrize("act,hidden,nb,with_pos", [("silu", 64, 8, False), ("tanh", 32, 5, True), ("relu", 128, 16, True), ("silu", 96, 9, False)])
