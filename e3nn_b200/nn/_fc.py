@@ -4,9 +4,9 @@
 ``[h_in, h_out]`` ~ N(0,1), every layer divided by sqrt(h_in), hidden layers followed by the
 activation rescaled to unit second moment, ``e3nn/math/_normalize_activation.py:9-57``) and ``bessel``
 mirrors ``e3nn/math/_bessel.py:6-37``.  With ``math_mode='tf32x3'`` the layers whose widths fit
-(h_in % 32 == 0, h_out % 16 == 0: the 64 -> weight_numel layer) run on the tcgen05 kernel of
-``codegen/tc_gemm.py`` with hi/lo-split tf32 operands, forward and input gradient; other layers and
-``math_mode='fp32'`` are plain dense GEMMs left to cuBLAS through ``torch.matmul`` in fp32.  The
+(h_in and h_out multiples of 32, h_in up to 256: the 64 -> weight_numel layer) run on the tcgen05 kernel of
+``codegen/tc_gemm.py`` with hi/lo-split tf32 operands, forward and input gradient, and on ``csrc/matmul_tn.cu`` for the
+weight gradient; other layers and ``math_mode='fp32'`` are plain dense GEMMs left to cuBLAS through ``torch.matmul`` in fp32.  The
 elementwise parts are torch operators.
 """
 from __future__ import annotations

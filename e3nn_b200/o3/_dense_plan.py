@@ -180,8 +180,8 @@ def uvw_plan(spec, instruction_ids: Optional[Sequence[int]] = None) -> Tuple[np.
 
 def linear_plan(irreps_in: Irreps, irreps_out: Irreps, instructions, transpose: bool = False) -> Tuple[np.ndarray, List[int]]:
     """Plan of a Linear (weight instructions only).  ``transpose``: the map from output
-    cotangents back to input cotangents (same weights, read with a stride); a transposed plan may hold
-    several groups for one target and must be run with ``accumulate`` on zeroed rows."""
+    cotangents back to input cotangents (same weights, read with a stride).  In the first part of a transposed plan a
+    target may have several groups (to be added up); in the second part, which ``e3b_dense_fwd`` runs, it has one."""
     oi, oo = irreps_in.offsets(), irreps_out.offsets()
     woff, offs = 0, []
     for ins in instructions:

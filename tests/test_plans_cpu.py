@@ -1,6 +1,8 @@
-"""Host logic of the weight-shared paths, checked on the CPU: the dense plans (interpreted here in numpy exactly as
-the kernels read them) and the construction of the transposed products that give the operand gradients."""
+"""Host logic of the weight-shared paths, checked on the CPU: the dense plans, interpreted here in numpy as the kernels read
+them (the first part: per-row weights and the Gate epilogue above l = 3; the second part: everything else), and the
+construction of the transposed products that give the operand gradients."""
 import numpy as np
+import pytest
 import torch
 
 from conftest import rel_err
@@ -39,6 +41,80 @@ def run_plan(plan: np.ndarray, x1: np.ndarray, x2, W: np.ndarray, accumulate_int
     return out
 
 
+class SecondPart:
+    """The tables of a plan's second part: forward, weight gradient and operand gradients from whole paths."""
+
+    def __init__(self, plan: np.ndarray):
+        assert plan[0] == MAGIC and len(plan) == plan[6]
+        self.plan = plan
+        h = [int(v) for v in plan[int(plan[-1]) : int(plan[-1]) + 12]]
+        self.d1max, self.d3max, self.covered = h[8], h[9], h[11]
+        rows = lambda n, at, width: plan[at : at + n * width].reshape(n, width).tolist()      # noqa: E731
+        self.groups, self.chunks, self.paths = rows(h[0], h[1], 6), rows(h[2], h[3], 6), rows(h[4], h[5], 16)
+        self.in_groups = rows(h[6], h[7], 5)
+        self.in_paths = plan[h[10] : h[10] + sum(g[4] for g in self.in_groups)].tolist()
+
+    def _segment(self, at: int, n: int):
+        a, b = int(self.plan[at + n]), int(self.plan[at + n + 1])
+        return [(int(self.plan[q]), _i2f(self.plan[q + 1])) for q in range(a, b, 2)]
+
+    def _coupled(self, path, x1, x2, x1off: int, channels: int, x2off: int) -> np.ndarray:
+        """A[z, u, k] of `channels` channels: T[z, k, i] = sum_j C_ijk x2[z, j], A = T x1 (Linear: the coefficient times x1)."""
+        d1, d3 = path[0], path[2]
+        x = x1[:, x1off : x1off + channels * d1].reshape(-1, channels, d1)
+        if x2off < 0:
+            return _i2f(path[15]) * x
+        t = np.zeros((len(x1), d3, d1))
+        for k in range(d3):
+            for i in range(d1):
+                for j, c in self._segment(path[5], k * d1 + i):
+                    t[:, k, i] += c * x2[:, x2off + j]
+        return np.einsum("zki,zui->zuk", t, x)
+
+    def _walk(self, x1, x2):
+        """(group, A of the chunk, flat weight indices [channel, output channel]) of every chunk; T is kept as the kernels do."""
+        for out_off, mo, d3, first, n, _ in self.groups:
+            t_of = None
+            for pid, x1off, channels, x2off, wbase, fresh in self.chunks[first : first + n]:
+                path = self.paths[pid]
+                assert fresh or t_of == (pid, x2off)
+                t_of = (pid, x2off)
+                idx = wbase + path[3] * np.arange(channels)[:, None] + path[4] * np.arange(mo)[None, :]
+                yield (out_off, mo, d3), self._coupled(path, x1, x2, x1off, channels, x2off), idx
+
+    def forward(self, x1, x2, W) -> np.ndarray:
+        out = np.zeros((len(x1), int(self.plan[3])))
+        for (off, mo, d3), a, idx in self._walk(x1, x2):
+            out[:, off : off + mo * d3] += np.einsum("zuk,uw->zwk", a, W[idx]).reshape(len(x1), -1)
+        return out
+
+    def weight_gradient(self, x1, x2, g, numel: int) -> np.ndarray:
+        gw = np.zeros(numel)
+        for (off, mo, d3), a, idx in self._walk(x1, x2):
+            np.add.at(gw, idx, np.einsum("zuk,zwk->uw", a, g[:, off : off + mo * d3].reshape(-1, mo, d3)))
+        return gw
+
+    def operand_gradients(self, x1, x2, W, g):
+        g1, g2 = np.zeros_like(x1), np.zeros_like(x2)
+        for x1off, m1, d1, first, n in self.in_groups:
+            for pid in self.in_paths[first : first + n]:
+                _, d2, d3, su, sw, ki, jj, px1, pm1, x2off, m2, out_off, mo, wbase, sv, _ = path = self.paths[pid]
+                assert (px1, pm1, path[0]) == (x1off, m1, d1)
+                x, gg = x1[:, x1off : x1off + m1 * d1].reshape(-1, m1, d1), g[:, out_off : out_off + mo * d3].reshape(-1, mo, d3)
+                for v in range(m2):
+                    w = W[wbase + v * sv + su * np.arange(m1)[:, None] + sw * np.arange(mo)[None, :]]
+                    q = np.einsum("uw,zwk->zuk", w, gg)
+                    m = np.einsum("zui,zuk->zik", x, q).reshape(len(x1), -1)
+                    for j in range(d2):
+                        for at, c in self._segment(jj, j):
+                            g2[:, x2off + v * d2 + j] += c * m[:, at]
+                    for k in range(d3):
+                        for i in range(d1):
+                            t = sum(c * x2[:, x2off + v * d2 + j] for j, c in self._segment(ki, k * d1 + i))
+                            g1[:, x1off : x1off + m1 * d1].reshape(-1, m1, d1)[:, :, i] += np.reshape(t, (-1, 1)) * q[:, :, k]
+        return g1, g2
+
+
 def _ins(tp):
     return [(i.i_in1, i.i_in2, i.i_out, i.connection_mode, i.has_weight) for i in tp.instructions]
 
@@ -56,6 +132,42 @@ def test_uvw_plan_matches_oracle():
     got = run_plan(tp._plan_host, x1.numpy(), x2.numpy(), w.numpy())
     # the plan stores its coefficients in fp32
     assert rel_err(torch.from_numpy(got), _oracle_tp(tp, x1, x2, w)) < 1e-6
+
+
+@pytest.mark.parametrize("layout", [("3x0e+2x1o+4x2e+1x1e", "2x0e+3x1o+1x2e", "5x0e+2x1o+3x2e+2x1e+1x3o"),
+                                    ("33x0e+65x1o", "1x0e+2x1o", "40x0e+1x1o+2x1e"),          # more than a chunk of channels
+                                    ("2x4e+1x0e+3x5o", "1x4e+2x0e", "2x4e+1x0e+0x1o")])       # an operand block no path leaves
+def test_second_part_of_product_plans(layout):
+    """What the register-tile kernels read: forward and all gradients against autograd through the oracle."""
+    torch.manual_seed(0)
+    tp = o3.FullyConnectedTensorProduct(*layout)
+    x1, x2 = (torch.randn(5, d, dtype=torch.float64, requires_grad=True) for d in (tp.irreps_in1.dim, tp.irreps_in2.dim))
+    w = tp.weight.detach().double().requires_grad_(True)
+    ref = _oracle_tp(tp, x1, x2, w)
+    go = torch.randn_like(ref)
+    want = [ref.detach()] + list(torch.autograd.grad(ref, [w, x1, x2], go))
+    part = SecondPart(tp._plan_host)
+    a, b, ww, g = (t.detach().numpy() for t in (x1, x2, w, go))
+    got = [part.forward(a, b, ww), part.weight_gradient(a, b, g, len(ww)), *part.operand_gradients(a, b, ww, g)]
+    for x, y in zip(got, want):
+        assert rel_err(torch.from_numpy(x), y) < 1e-6        # (the coefficients are fp32)
+    assert bool(part.covered) == all(any(i.i_in1 == n and 0 not in i.path_shape for i in tp.instructions) for n, m in enumerate(tp.irreps_in1) if m.dim > 0)
+
+
+def test_second_part_of_linear_plans():
+    torch.manual_seed(1)
+    lin = o3.Linear("6x0e+4x1o+3x2e+35x0e", "5x0e+2x0e+4x1o+3x1o+3x0o")
+    x = torch.randn(7, lin.irreps_in.dim, dtype=torch.float64, requires_grad=True)
+    w = lin.weight.detach().double().requires_grad_(True)
+    ref = orc.linear(str(lin.irreps_in), str(lin.irreps_out), x, w)
+    go = torch.randn_like(ref)
+    gx, gw = torch.autograd.grad(ref, [x, w], go)
+    forward, back = SecondPart(lin._plan_host), SecondPart(lin._plan_t_host)
+    a, ww, g = (t.detach().numpy() for t in (x, w, go))
+    assert rel_err(torch.from_numpy(forward.forward(a, None, ww)), ref.detach()) < 1e-6
+    assert rel_err(torch.from_numpy(forward.weight_gradient(a, None, g, len(ww))), gw) < 1e-6
+    assert rel_err(torch.from_numpy(back.forward(g, None, ww)), gx) < 1e-6
+    assert not lin._reads_all
 
 
 def test_linear_plans_forward_and_transposed_with_mixed_multiplicities():
