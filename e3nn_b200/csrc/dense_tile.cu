@@ -173,6 +173,14 @@ __device__ __forceinline__ void fwd_tile(const Part2& P, const int32_t* g, const
     // the rows of the tile past nz * d3 are read (and never stored): they must not hold non-finite leftovers
     for (int idx = tid; idx < (BM - tz * d3) * kLda; idx += kThreads) sA[tz * d3 * kLda + idx] = 0.0f;
 
+    // sums of up to 32 entries, over several chunks where the paths have fewer channels, in accumulators of their own: the
+    // rounding error grows with sqrt(32) + sqrt(K / 32)
+    float part[kTM][kTN];
+#pragma unroll
+    for (int i = 0; i < kTM; ++i)
+#pragma unroll
+        for (int j = 0; j < kTN; ++j) part[i][j] = 0.0f;
+    int held = 0;
     for (int c = 0; c < g[4]; ++c) {
         const int32_t* ch = P.chunk(g[3] + c);
         const int32_t* path = P.path(ch[0]);
@@ -186,12 +194,6 @@ __device__ __forceinline__ void fwd_tile(const Part2& P, const int32_t* g, const
         stage_weights<BN>(W + ch[4] + static_cast<int64_t>(c0) * path[4], path[3], path[4], len, cols, sW);
         stage_rows(d1, x1, d1row, ch[1], len, z0, tz, Z, d3, coupled, __int_as_float(path[15]), sT, ldt, sA, kLda);
         __syncthreads();
-        // the chunk's sum in accumulators of its own: the rounding error grows with sqrt(32) + sqrt(K / 32)
-        float part[kTM][kTN];
-#pragma unroll
-        for (int i = 0; i < kTM; ++i)
-#pragma unroll
-            for (int j = 0; j < kTN; ++j) part[i][j] = 0.0f;
         const int kend = (len + 3) & ~3;
 #pragma unroll 1
         for (int kk = 0; kk < kend; kk += 4) {
@@ -211,10 +213,13 @@ __device__ __forceinline__ void fwd_tile(const Part2& P, const int32_t* g, const
                 }
             }
         }
+        held += len;
+        if (c + 1 < g[4] && held + P.chunk(g[3] + c + 1)[2] <= kKC) continue;
+        held = 0;
 #pragma unroll
         for (int i = 0; i < kTM; ++i)
 #pragma unroll
-            for (int j = 0; j < kTN; ++j) acc[i][j] += part[i][j];
+            for (int j = 0; j < kTN; ++j) { acc[i][j] += part[i][j]; part[i][j] = 0.0f; }
     }
     __syncthreads();
     // the tile in output order, then contiguous row segments
@@ -535,6 +540,17 @@ __device__ __forceinline__ void fwd_rows_tile(const Part2& P, const int32_t* g, 
 #pragma unroll
             for (int n = 0; n < 8; ++n) acc[p][k][n] = 0.0f;
 
+    // sums of up to 32 entries, over several chunks where the paths have fewer channels, in accumulators of their own: the
+    // rounding error grows with sqrt(32) + sqrt(K / 32)
+    float part[ZPT][D3][8];
+#pragma unroll
+    for (int p = 0; p < ZPT; ++p)
+#pragma unroll
+        for (int k = 0; k < D3; ++k)
+#pragma unroll
+            for (int n = 0; n < 8; ++n) part[p][k][n] = 0.0f;
+    int held = 0;
+
     if (COUPLED)
         for (int idx = tid; idx < BZ * d2row; idx += kThreads) {
             const int z = idx / d2row, e = idx - z * d2row;
@@ -564,14 +580,6 @@ __device__ __forceinline__ void fwd_rows_tile(const Part2& P, const int32_t* g, 
             __syncthreads();
         }
         const float* w = sW + (c & 1) * kKC * ldw;
-        // the chunk's sum in accumulators of its own: the rounding error grows with sqrt(32) + sqrt(K / 32)
-        float part[ZPT][D3][8];
-#pragma unroll
-        for (int p = 0; p < ZPT; ++p)
-#pragma unroll
-            for (int k = 0; k < D3; ++k)
-#pragma unroll
-                for (int n = 0; n < 8; ++n) part[p][k][n] = 0.0f;
         const int uend = (ch[2] + 3) & ~3;
 #pragma unroll 1
         for (int u = 0; u < uend; u += 4) {
@@ -599,12 +607,18 @@ __device__ __forceinline__ void fwd_rows_tile(const Part2& P, const int32_t* g, 
                         for (int n = 0; n < 8; ++n) part[p][k][n] = fmaf(a[q * D3 + k], wv[q][n], part[p][k][n]);
             }
         }
+        held += ch[2];
+        bool keep = c + 1 < nch && held + P.chunk(g[3] + c + 1)[2] <= kKC;
+        if (!COUPLED && keep) keep = P.path(P.chunk(g[3] + c + 1)[0])[15] == path[15];      // one coefficient
+        if (!keep) {
+            held = 0;
 #pragma unroll
-        for (int p = 0; p < ZPT; ++p)
+            for (int p = 0; p < ZPT; ++p)
 #pragma unroll
-            for (int k = 0; k < D3; ++k)
+                for (int k = 0; k < D3; ++k)
 #pragma unroll
-                for (int n = 0; n < 8; ++n) acc[p][k][n] = fmaf(coef, part[p][k][n], acc[p][k][n]);
+                    for (int n = 0; n < 8; ++n) { acc[p][k][n] = fmaf(coef, part[p][k][n], acc[p][k][n]); part[p][k][n] = 0.0f; }
+        }
         if (!COUPLED) __syncthreads();          // the buffers are fetched into again
     }
     const bool vec = (dout & 3) == 0 && (cols & 3) == 0 && aligned16(out + out_off + c0 * D3) && !accumulate;
@@ -914,6 +928,7 @@ __global__ void __launch_bounds__(kThreads, 4) dense_rows_wgrad_kernel(const int
 // the sums over k stay in its registers, and the sums over u cross 4 lanes.  Its share of grad_x2 goes to a partial of its
 // own; a second kernel adds the partials in a fixed order.
 constexpr int kBxZ = 32, kBxU = 8;
+constexpr int kBxRun = 32;         // additions to an entry of grad_x1 in a register before it is put away
 
 struct BwdXLaunch {
     int n;
@@ -1072,6 +1087,10 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
 
     BwdXStep step{0, 0, 0, P.path(P.in_path(in[3]))};
     bwd_x_fetch(P, step, W, gout, z0, live, u0, nu, S, 0);
+    // wide second operands: the sums so far are put away in grad_x1 now and then, so that the runs of additions stay short
+    int run = 0;
+    bool away = false;
+    float* orow = NEED1 ? g1 + (z0 + min(ty, live - 1)) * d1row + x1off + u0 * D1 : nullptr;
     for (int buf = 0;; buf ^= 1) {
         BwdXStep next = step;
         const bool more = bwd_x_next(P, in, next);
@@ -1088,6 +1107,18 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
         }
         __syncthreads();      // the buffers and the coupling are written again
         if (!more) break;
+        if (NEED1 && (run += step.path[2]) >= kBxRun) {
+#pragma unroll
+            for (int u = 0; u < kBxU; ++u)
+#pragma unroll
+                for (int i = 0; i < D1; ++i) {
+                    float* o = orow + (tx * kBxU + u) * D1 + i;
+                    if (ty < live && tx * kBxU + u < nu) *o = away ? *o + gx[i][u] : gx[i][u];
+                    gx[i][u] = 0.0f;
+                }
+            run = 0;
+            away = true;
+        }
         step = next;
     }
     if (NEED1) {
@@ -1102,7 +1133,7 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
             const int zl = warp * 8 + r;
             if (z0 + zl >= Z) break;
             float* o = g1 + (z0 + zl) * d1row + x1off + u0 * D1;
-            for (int e = lane; e < nu * D1; e += 32) o[e] = S.g[zl * ld + e];
+            for (int e = lane; e < nu * D1; e += 32) o[e] = away ? o[e] + S.g[zl * ld + e] : S.g[zl * ld + e];
         }
     }
     if (NEED2) {

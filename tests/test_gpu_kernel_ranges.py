@@ -131,6 +131,24 @@ def test_fp32_product_many_outputs_wide_second_operand(tail):
         assert rel_err(a.cpu(), r64) < fp32_bound(rel_err(r32, r64))
 
 
+def test_fp32_rounding_of_long_sums_over_narrow_blocks():
+    """Thousands of terms from operand blocks of one and two channels, summed 32 at a time as with wide blocks.  Bound on the
+    2-norm: 1.5 times, in quadrature, three roundings of 2^-24 and the random walks of a run of 32 and of the K / 32 runs, 0.3 x
+    2^-24 x sqrt(n) each (0.3: the mean rounding error of a sum that grows to its last size).  One walk of K steps: 9e-7."""
+    g = torch.Generator().manual_seed(0)
+    tp = o3.FullyConnectedTensorProduct("+".join(["2x0e"] * 33), "80x0e", "4x0e")
+    lin = o3.Linear("+".join(["1x0e"] * 3000), "32x0e")
+    x, y, z = (torch.randn(100, d, generator=g) for d in (tp.irreps_in1.dim, tp.irreps_in2.dim, lin.irreps_in.dim))
+    ins = [(i.i_in1, i.i_in2, i.i_out, i.connection_mode, i.has_weight) for i in tp.instructions]
+    ref = orc.tensor_product(*(str(i) for i in (tp.irreps_in1, tp.irreps_in2, tp.irreps_out)), ins, x.double(), y.double(),
+                             tp.weight.detach().double(), True)
+    ref_lin = orc.linear(str(lin.irreps_in), str(lin.irreps_out), z.double(), lin.weight.detach().double())
+    with torch.no_grad():
+        for got, want, k in ((tp.to(DEV)(x.to(DEV), y.to(DEV)), ref, 5280), (lin.to(DEV)(z.to(DEV)), ref_lin, 3000)):
+            err = ((got.cpu().double() - want).norm() / want.norm()).item()
+            assert err < 1.5 * 2.0**-24 * (9 + 0.09 * (32 + k / 32)) ** 0.5, (k, err)
+
+
 @pytest.mark.parametrize("rows", [1, 257])
 @pytest.mark.parametrize("irreps", [("1x0e+40x1o+3x2e", "200x0e+2x0e+17x1o"), ("70x0e+9x4e", "9x4e+16x0e+5x1o"), ("64x0e+64x3o", "32x0e+64x3o"),
                                     ("40x16e+3x31o+2x0e", "70x16e+130x31o+5x0e")])
