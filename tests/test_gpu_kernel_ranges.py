@@ -208,7 +208,8 @@ def test_conv_pipelined_permuted_edges(layout, nodes, edges):
 @pytest.mark.parametrize("bad", ["source", "perm", "perm_negative"])
 def test_conv_pipelined_skips_a_bad_index(layout, bad):
     """One slot with a source or a permutation entry out of range: reported, and every other edge and row is what it is without
-    that edge, bit for bit (its weights set to zero give the same sums); 1e-6 x RMS for the atomic node-feature gradient."""
+    that edge, bit for bit (its weights set to zero give the same sums).  Bound for the node-feature gradient, whose atomics
+    come in any order: two sums of about 30 edges, a rounding of 2^-24 each (twice that for rows of twice the edges)."""
     g = torch.Generator().manual_seed(3)
     tp, nodes, edges, slot = layouts.bench_conv_tp(layout), 50, 1500, 777
     dst, src = torch.randint(0, nodes, (edges,), generator=g), torch.randint(0, nodes, (edges,), generator=g).to(DEV)
@@ -244,7 +245,7 @@ def test_conv_pipelined_skips_a_bad_index(layout, bad):
     rest = torch.arange(edges, device=DEV) != lost
     assert torch.equal(got[0], want[0])
     assert torch.equal(got[2][rest], want[2][rest]) and torch.equal(got[3][rest], want[3][rest])
-    assert rel_err(got[1].cpu(), want[1].cpu().double()) < 1e-6
+    assert rel_err(got[1].cpu(), want[1].cpu().double()) < 2 * 2 * 30 * 2.0**-24
 
 
 # ----------------------------------------------------------------------------- edge embedding: gradient of its weights
