@@ -1,5 +1,5 @@
-// fp32 CUDA-core evaluation of 'uvw' tensor-product paths with per-row weights, and of the per-irrep Linear with Gate
-// as its epilogue (weight-shared contractions without it: dense_tile.cu).  Table driven (no per-layout code): the host
+// fp32 CUDA-core evaluation of 'uvw' tensor-product paths with per-row weights or a few channels, and of the per-irrep Linear
+// with Gate as its epilogue above l = 3 (other weight-shared contractions: dense_tile.cu).  Table driven (no per-layout code): the host
 // describes the contraction as a "dense plan" and this kernel evaluates, per output irrep ("group"),
 //
 //     out[z, w, k] = sum_K  A[z, k, K] * W[wbase(K) + w * wstride]
@@ -268,7 +268,7 @@ extern "C" int e3b_dense_fwd(const int32_t* plan_host, const int32_t* plan_dev, 
     if (num_rows < 0) return fail(E3B_ERR_ARG, "dense_fwd: negative row count");
     if (num_rows == 0) return E3B_OK;
     if (!plan_dev || !x1 || !out || !weight) return fail(E3B_ERR_ARG, "dense_fwd: null pointer");
-    if (weight_row_stride == 0 && whole_plan(plan_host))
+    if (weight_row_stride == 0 && whole_plan(plan_host) && !few_channels(plan_host))
         return launch_dense_tile_fwd(plan_host, plan_dev, x1, x2, weight, out, num_rows, accumulate, static_cast<cudaStream_t>(stream));
     const DenseGateEpilogue none{nullptr, nullptr, nullptr, nullptr, 0, 0};
     return launch_dense_groups(plan_host, plan_dev, x1, x2, weight, weight_row_stride, out, num_rows, accumulate, none, 0,

@@ -9,8 +9,10 @@
 //     A[z, k, u]   = sum_i T_p[z, k, i] x1[z, u, i]         (Linear: A = c x1, k = i)
 //     out[z, w, k] = sum_{p, v, u} A[z, k, u] W_p[u, v, w]
 //
-// Second part: header of 12 words { n_groups, groups, n_chunks, chunks, n_paths, paths, n_in, in_groups, d1max, d3max,
-// in_paths, covered } (word offsets into the plan), then
+// x1 and x2 are the call's operands, or exchanged (`swapped`: the operand with more channels goes first, see the builder).
+//
+// Second part: header of 14 words { n_groups, groups, n_chunks, chunks, n_paths, paths, n_in, in_groups, d1max, d3max,
+// in_paths, covered, swapped, channels of all chunks } (word offsets into the plan), then
 //   groups    x 6 : out_off, mul_out, dim3, first chunk, chunks, 0
 //   chunks    x 6 : path, x1 offset of its first channel, channels (<= 32), x2 offset or -1, weight base, 1 = T changes
 //   paths     x 16: d1, d2, d3, weight strides over u and w, ki segments, j segments, x1off, m1, x2off, m2, out_off, mo,
@@ -20,6 +22,8 @@
 #include "common.cuh"
 #include "dense_plan.cuh"
 #include "gate_act.cuh"
+
+#include <utility>
 
 namespace e3b {
 namespace {
@@ -44,6 +48,11 @@ struct Part2 {
     __host__ __device__ int d3max() const { return h[9]; }
     __host__ __device__ int in_path(int n) const { return plan[h[10] + n]; }
     __host__ __device__ bool covers_x1() const { return h[11] != 0; }
+    __host__ __device__ bool swapped() const { return h[12] != 0; }
+    __host__ __device__ int d1row() const { return plan[swapped() ? 2 : 1]; }
+    __host__ __device__ int d2row() const { return plan[swapped() ? 1 : 2]; }
+    __host__ __device__ int n_chunks() const { return h[2]; }
+    __host__ __device__ int channels() const { return h[13]; }      // of all chunks
 };
 
 // T[zl][k * d1 + i] of a tile of nz rows (row stride ldt).
@@ -155,7 +164,7 @@ __device__ __forceinline__ void fwd_tile(const Part2& P, const int32_t* g, const
                                          float* smem) {
     constexpr int CX = BN / kTN, LX = CX < 8 ? CX : 8, LY = 32 / LX, WC = CX / LX, RY = kThreads / CX, BM = RY * kTM;
     constexpr int ldw = BN + 4;
-    const int out_off = g[0], mo = g[1], d3 = g[2], d1row = P.plan[1], d2row = P.plan[2], dout = P.plan[3];
+    const int out_off = g[0], mo = g[1], d3 = g[2], d1row = P.d1row(), d2row = P.d2row(), dout = P.plan[3];
     const int col_blocks = (mo + BN - 1) / BN, tz = BM / d3;
     const int64_t z0 = static_cast<int64_t>(tile / col_blocks) * tz;
     const int c0 = (tile % col_blocks) * BN, cols = min(BN, mo - c0);
@@ -284,7 +293,7 @@ __device__ __forceinline__ void bwd_w_block(const Part2& P, const int32_t* g, co
                                             float* smem) {
     constexpr int KB = 4096 / BW, NCH = KB / kKC, lda = KB + 4, ldg = BW + 4;
     constexpr int CX = BW / kTN, LX = 8, LY = 4, WC = CX / LX;
-    const int out_off = g[0], mo = g[1], d3 = g[2], d1row = P.plan[1], d2row = P.plan[2], dout = P.plan[3];
+    const int out_off = g[0], mo = g[1], d3 = g[2], d1row = P.d1row(), d2row = P.d2row(), dout = P.plan[3];
     const int kblocks = (g[4] + NCH - 1) / NCH, wblocks = (mo + BW - 1) / BW, tz = kBwRows / d3, rows = tz * d3;
     const int split = block / (kblocks * wblocks), rest = block % (kblocks * wblocks);
     const int ch0 = (rest / wblocks) * NCH, nch = min(NCH, g[4] - ch0);
@@ -509,7 +518,7 @@ __device__ __forceinline__ void fwd_rows_tile(const Part2& P, const int32_t* g, 
                                               const float* __restrict__ W, float* __restrict__ out, int64_t Z, int tile, int accumulate,
                                               const DenseGateEpilogue& ep, float* smem) {
     constexpr int ZPT = rows_per_thread<D3, TX, COUPLED>(), TZ = kThreads / TX, BZ = TZ * ZPT, BN = 8 * TX, ldw = BN + 4;
-    const int out_off = g[0], mo = g[1], nch = g[4], d1row = P.plan[1], d2row = P.plan[2], dout = P.plan[3];
+    const int out_off = g[0], mo = g[1], nch = g[4], d1row = P.d1row(), d2row = P.d2row(), dout = P.plan[3];
     const int col_blocks = (mo + BN - 1) / BN;
     const int64_t z0 = static_cast<int64_t>(tile / col_blocks) * BZ;
     const int live = static_cast<int>(min(static_cast<int64_t>(BZ), Z - z0));
@@ -747,7 +756,7 @@ __device__ __forceinline__ void wgrad_block(const Part2& P, const int32_t* g, co
                                             float* smem) {
     constexpr int KB = 4096 / BW, NCH = KB / kKC, BZ = wgrad_rows<D3, COUPLED>(), ldg = pad_row(BW * D3), lda = pad_row(KB * D3);
     constexpr int CX = BW / kTN, WC = CX / 8;
-    const int out_off = g[0], mo = g[1], d1row = P.plan[1], d2row = P.plan[2], dout = P.plan[3];
+    const int out_off = g[0], mo = g[1], d1row = P.d1row(), d2row = P.d2row(), dout = P.plan[3];
     const int kblocks = (g[4] + NCH - 1) / NCH, wblocks = (mo + BW - 1) / BW;
     const int split = block / (kblocks * wblocks), rest = block % (kblocks * wblocks);
     const int ch0 = (rest / wblocks) * NCH, nch = min(NCH, g[4] - ch0);
@@ -1071,7 +1080,7 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
     const int x1off = in[0], m1 = in[1], ublocks = (m1 + 31) / 32;
     const int64_t z0 = static_cast<int64_t>(block / ublocks) * kBxZ;
     const int u0 = (block % ublocks) * 32, nu = min(32, m1 - u0);
-    const int d1row = P.plan[1], d2row = P.plan[2];
+    const int d1row = P.d1row(), d2row = P.d2row();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = lane & 3, ty = warp * 8 + (lane >> 2);
     float gx[D1][kBxU];
@@ -1161,7 +1170,7 @@ __global__ void __launch_bounds__(kThreads, 3) dense_tile_bwd_x_kernel(const int
     BwdXShared S;
     S.ldt = (P.d1max() * P.d3max()) | 1;
     S.ldm = S.ldt;
-    S.ld2 = plan[2] | 1;
+    S.ld2 = P.d2row() | 1;
     S.g_floats = g_floats;
     S.g = smem;
     S.w = S.g + 2 * g_floats;
@@ -1200,8 +1209,8 @@ inline int bwd_x_parts(const Part2& P) {
 }
 
 // Rows whose partials are held at a time: at most 128 MB of them, at least 16 row tiles.
-inline int64_t bwd_x_slab(const int32_t* plan, int parts, int64_t rows) {
-    const int64_t fit = (int64_t{128} << 20) / (static_cast<int64_t>(sizeof(float)) * parts * std::max(plan[2], 1)) / kBxZ * kBxZ;
+inline int64_t bwd_x_slab(const Part2& P, int parts, int64_t rows) {
+    const int64_t fit = (int64_t{128} << 20) / (static_cast<int64_t>(sizeof(float)) * parts * std::max(P.d2row(), 1)) / kBxZ * kBxZ;
     return std::min<int64_t>(rows, std::max<int64_t>(fit, 16 * kBxZ));
 }
 
@@ -1210,12 +1219,17 @@ inline int bwd_x_g_floats(int d1max, int d3max) {
     return std::max(kBxZ * pad_row(32 * d3max), ((kBxZ * (32 * d1max + 1) + 1) / 2 + 3) & ~3);
 }
 
-inline size_t bwd_x_shared(const int32_t* plan, int d1max, int d3max, bool need2) {
-    const int ldt = (d1max * d3max) | 1;
-    size_t f = 2 * static_cast<size_t>(bwd_x_g_floats(d1max, d3max)) + 2 * kKC * kLda + kBxZ * ldt;
-    if (need2) f += static_cast<size_t>(kBxZ) * (ldt + (plan[2] | 1));
+inline size_t bwd_x_shared(const Part2& P, bool need2) {
+    const int ldt = (P.d1max() * P.d3max()) | 1;
+    size_t f = 2 * static_cast<size_t>(bwd_x_g_floats(P.d1max(), P.d3max())) + 2 * kKC * kLda + kBxZ * ldt;
+    if (need2) f += static_cast<size_t>(kBxZ) * (ldt + (P.d2row() | 1));
     return f * sizeof(float);
 }
+
+// Under eight channels a chunk the table-driven kernel (dense.cu), whose contraction index runs over all pairs of channels, is
+// the faster one: 10,000 rows of 4 x 4 -> 64 channels, l <= 2, 169 against 187 us, 100,000 rows of 1 x 1 -> 1, 294 against 504;
+// with eight (30,000 rows of 8 x 8 -> 64) 1,313 against 1,051.
+constexpr int64_t kFewChannels = 8;
 
 bool too_many_blocks(int64_t blocks) { return blocks > 2147483647LL; }
 
@@ -1253,7 +1267,7 @@ static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, co
     const int most = GATE && pass == 1 ? 1 : kMaxGroups;
     // the narrowest tile that holds the group's channels in one pass, so that the coupled operand is built once
     auto threads_a_row = [](const int32_t* g) { return g[1] <= 32 ? 4 : g[1] <= 64 ? 8 : 16; };
-    auto shape_of = [&](const int32_t* g) { return fwd_shape<COUPLED>(g[2], threads_a_row(g), P.d1max(), plan_host[2]); };
+    auto shape_of = [&](const int32_t* g) { return fwd_shape<COUPLED>(g[2], threads_a_row(g), P.d1max(), P.d2row()); };
     *done = all_groups_fit(P, shape_of);
     if (!*done) return E3B_OK;
     int g0 = 0;
@@ -1292,7 +1306,7 @@ static int launch_rows_wgrad(const int32_t* plan_host, const int32_t* plan_dev, 
                              float* grad_w, int64_t Z, cudaStream_t s, bool* done) {
     const Part2 P(plan_host);
     auto channels_of = [](const int32_t* g) { return g[1] <= 32 ? 32 : g[1] <= 64 ? 64 : 128; };
-    auto shape_of = [&](const int32_t* g) { return wgrad_shape<COUPLED>(g[2], channels_of(g), P.d1max(), plan_host[2]); };
+    auto shape_of = [&](const int32_t* g) { return wgrad_shape<COUPLED>(g[2], channels_of(g), P.d1max(), P.d2row()); };
     *done = all_groups_fit(P, shape_of);
     if (!*done) return E3B_OK;
     int g0 = 0;
@@ -1346,9 +1360,15 @@ int launch_dense_rows_gate(const int32_t* plan_host, const int32_t* plan_dev, co
     return launch_rows_fwd<false, true>(plan_host, plan_dev, x, nullptr, weight, nullptr, Z, 0, ep, 2, s, done);
 }
 
+bool few_channels(const int32_t* plan_host) {
+    const Part2 P(plan_host);
+    return coupled_plan(P) && P.channels() < kFewChannels * P.n_chunks();
+}
+
 int launch_dense_tile_fwd(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
                           float* out, int64_t Z, int accumulate, cudaStream_t s) {
     const Part2 P(plan_host);
+    if (P.swapped()) std::swap(x1, x2);
     if (rows_plan(P)) {
         bool done = false;
         const DenseGateEpilogue none{nullptr, nullptr, nullptr, nullptr, 0, 0};
@@ -1391,6 +1411,7 @@ int launch_dense_tile_fwd(const int32_t* plan_host, const int32_t* plan_dev, con
 int launch_dense_tile_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* gout,
                             float* grad_w, int64_t Z, cudaStream_t s) {
     const Part2 P(plan_host);
+    if (P.swapped()) std::swap(x1, x2);
     if (rows_plan(P)) {
         bool done = false;
         const int rc = coupled_plan(P) ? launch_rows_wgrad<true>(plan_host, plan_dev, x1, x2, gout, grad_w, Z, s, &done)
@@ -1442,7 +1463,7 @@ template <bool NEED1, bool NEED2>
 static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
                         const float* gout, float* g1, float* g2, float* partial, int64_t Z, cudaStream_t s) {
     const Part2 P(plan_host);
-    const size_t bytes = bwd_x_shared(plan_host, P.d1max(), P.d3max(), NEED2);
+    const size_t bytes = bwd_x_shared(P, NEED2);
     int g0 = 0, part = 0;
     while (g0 < P.n_in()) {
         BwdXLaunch L;
@@ -1474,11 +1495,11 @@ extern "C" int e3b_dense_bwd_x_supported(const int32_t* plan_host) {
     using namespace e3b;
     if (!whole_plan(plan_host)) return 0;
     const Part2 P(plan_host);
-    return P.n_in() > 0 && P.d1max() <= 7 && P.d3max() <= 7 && bwd_x_shared(plan_host, P.d1max(), P.d3max(), true) <= static_cast<size_t>(kMaxShared);
+    return P.n_in() > 0 && P.d1max() <= 7 && P.d3max() <= 7 && bwd_x_shared(P, true) <= static_cast<size_t>(kMaxShared);
 }
 
 namespace e3b {
-// partial: nullptr (grad_x2 by atomics) or bwd_x_parts() x rows x d2 floats (grad_x2 itself when there is one part).
+// Operands in the plan's order.  partial: nullptr (grad_x2 by atomics) or bwd_x_parts() x rows x d2 floats (grad_x2 itself when there is one part).
 static int bwd_x_rows(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight, const float* gout,
                       float* g1, float* g2, float* partial, int64_t Z, cudaStream_t s) {
     if (g1 && g2) return launch_bwd_x<true, true>(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, partial, Z, s);
@@ -1495,7 +1516,11 @@ static int bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float*
     if (!e3b_dense_bwd_x_supported(plan_host)) return fail(E3B_ERR_UNSUPPORTED, "dense_bwd_x: irreps above l = 3 or too wide");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Part2 P(plan_host);
-    const int64_t d1 = plan_host[1], d2 = plan_host[2], dout = plan_host[3];
+    if (P.swapped()) {
+        std::swap(x1, x2);
+        std::swap(g1, g2);
+    }
+    const int64_t d1 = P.d1row(), d2 = P.d2row(), dout = plan_host[3];
     const int parts = bwd_x_parts(P);
     if (g1 && !P.covers_x1()) E3B_CUDA_TRY(cudaMemsetAsync(g1, 0, sizeof(float) * Z * d1, s));
     if (!g2 || parts == 1) return bwd_x_rows(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, g2, Z, s);
@@ -1503,7 +1528,7 @@ static int bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float*
         E3B_CUDA_TRY(cudaMemsetAsync(g2, 0, sizeof(float) * Z * d2, s));
         return bwd_x_rows(plan_host, plan_dev, x1, x2, weight, gout, g1, g2, nullptr, Z, s);
     }
-    const int64_t slab = bwd_x_slab(plan_host, parts, Z);
+    const int64_t slab = bwd_x_slab(P, parts, Z);
     if (!scratch || scratch_bytes < static_cast<int64_t>(sizeof(float)) * parts * slab * d2) return fail(E3B_ERR_ARG, "dense_bwd_x: scratch too small");
     float* partial = static_cast<float*>(scratch);
     for (int64_t z = 0; z < Z; z += slab) {
@@ -1521,8 +1546,9 @@ static int bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float*
 extern "C" int64_t e3b_dense_bwd_x_scratch_bytes(const int32_t* plan_host, int64_t num_rows) {
     using namespace e3b;
     if (!e3b_dense_bwd_x_supported(plan_host) || num_rows <= 0) return 0;
-    const int parts = bwd_x_parts(Part2(plan_host));
-    return parts == 1 ? 0 : static_cast<int64_t>(sizeof(float)) * parts * bwd_x_slab(plan_host, parts, num_rows) * plan_host[2];
+    const Part2 P(plan_host);
+    const int parts = bwd_x_parts(P);
+    return parts == 1 ? 0 : static_cast<int64_t>(sizeof(float)) * parts * bwd_x_slab(P, parts, num_rows) * P.d2row();
 }
 
 extern "C" int e3b_dense_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,

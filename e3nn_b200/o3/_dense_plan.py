@@ -102,8 +102,14 @@ class _Builder:
             words.extend(ends)
             return at
 
+        swapped = self._swaps()
+        if swapped:
+            paths = [dict(p, x1off=p["x2off"], m1=p["m2"], d1=p["d2"], x2off=p["x1off"], m2=p["m1"], d2=p["d1"], su=p["sv"], sv=p["su"],
+                          c=p["c"].transpose(1, 0, 2)) for p in self.wpaths]
+        else:
+            paths = self.wpaths
         rows, d1max, d3max = [], 1, 1
-        for p in self.wpaths:
+        for p in paths:
             d1, d2, d3 = p["d1"], p["d2"], p["d3"]
             d1max, d3max = max(d1max, d1), max(d3max, d3)
             ki = jj = 0
@@ -117,7 +123,7 @@ class _Builder:
         for out_off, mo, d3, members in self.wgroups:
             first = len(chunks)
             for n in members:
-                p = self.wpaths[n]
+                p = paths[n]
                 for v in range(p["m2"]):
                     x2off = p["x2off"] + v * p["d2"] if p["x2off"] >= 0 else -1
                     for u0 in range(0, p["m1"], 32):
@@ -126,7 +132,7 @@ class _Builder:
             groups.append([out_off, mo, d3, first, len(chunks) - first, 0])
         # the paths that leave each block of the first operand (operand gradients of a product)
         blocks = {}
-        for n, p in enumerate(self.wpaths):
+        for n, p in enumerate(paths):
             if p["x2off"] >= 0 and p["m1"] * p["m2"] * p["mo"] > 0:
                 blocks.setdefault((p["x1off"], p["m1"], p["d1"]), []).append(n)
         in_paths = [n for members in blocks.values() for n in members]
@@ -134,7 +140,7 @@ class _Builder:
         for (x1off, m1, d1), members in blocks.items():
             in_groups.append([x1off, m1, d1, at, len(members)])
             at += len(members)
-        covered = sum(m1 * d1 for _, m1, d1 in blocks) == self.d1
+        covered = sum(m1 * d1 for _, m1, d1 in blocks) == (self.d2 if swapped else self.d1)
         offs = []
         for table in (groups, chunks, rows, in_groups):
             offs.append(base + len(words))
@@ -144,8 +150,21 @@ class _Builder:
         words.extend(in_paths)
         header = base + len(words)
         words.extend([len(groups), offs[0], len(chunks), offs[1], len(rows), offs[2], len(in_groups), offs[3], d1max, d3max, offs[4],
-                      int(covered)])
+                      int(covered), int(swapped), sum(c[2] for c in chunks)])
         return words, header
+
+    def _swaps(self) -> bool:
+        """Whether the second part describes a product with its operands exchanged: the kernels take 32 channels of the first
+        operand at a time for every single channel of the second, so the one that gives fewer such chunks goes first (8 x 64
+        channels: 64 chunks of 8 a path, or 16 of 32; 10,000 rows, l <= 2, forward 5.5 -> 0.78 ms, all gradients 18 -> 3.4; 1 x 128
+        -> 32 channels 16 -> 0.22 and 57 -> 0.70 ms), unless that takes an irrep of l > 3 into the first place, where the row
+        kernels do not have it."""
+        paths = [p for p in self.wpaths if p["m1"] * p["m2"] * p["mo"] > 0]
+        if not paths or paths[0]["x2off"] < 0:
+            return False
+        if max(p["d2"] for p in paths) > 7 >= max(p["d1"] for p in paths):
+            return False
+        return sum(p["m1"] * -(-p["m2"] // 32) for p in paths) < sum(p["m2"] * -(-p["m1"] // 32) for p in paths)
 
 
 def uvw_plan(spec, instruction_ids: Optional[Sequence[int]] = None) -> Tuple[np.ndarray, List[int]]:

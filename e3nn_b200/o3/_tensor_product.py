@@ -86,7 +86,7 @@ class _UvwFunction(torch.autograd.Function):
                 g1 = torch.empty_like(x1) if need1 else None
                 g2 = torch.empty_like(x2) if need2 else None
                 core, plan = _lib.core(), tp._plan_host.ctypes.data
-                scratch = torch.empty(core.e3b_dense_bwd_x_scratch_bytes(plan, x1.shape[0]) if need2 else 0, dtype=torch.uint8, device=g.device)
+                scratch = torch.empty(core.e3b_dense_bwd_x_scratch_bytes(plan, x1.shape[0]), dtype=torch.uint8, device=g.device)
                 with torch.cuda.device(g.device):
                     rc = core.e3b_dense_bwd_x_ordered(plan, _lib._ptr(tp._plan_on(g.device)), _lib._ptr(x1), _lib._ptr(x2), _lib._ptr(w),
                                                       _lib._ptr(g), _lib._ptr(g1), _lib._ptr(g2), x1.shape[0], _lib._ptr(scratch),

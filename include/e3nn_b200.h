@@ -257,10 +257,10 @@ int e3b_dense_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, const flo
  * e3nn/o3/_tensor_product/_codegen.py:148-165 for x and y), with the plan of the forward call:
  *   grad_x1[z,u,i] = sum pw W[u,v,w] C_ijk x2[z,v,j] g[z,w,k],   grad_x2[z,v,j] = sum pw W[u,v,w] C_ijk x1[z,u,i] g[z,w,k].
  * Either output may be NULL.  grad_x1 [rows, d1] and grad_x2 [rows, d2] are overwritten (columns no path reads become
- * zero); grad_x2 is summed over blocks of 32 channels of x1's irreps, by float atomics in e3b_dense_bwd_x and in a fixed order
- * in e3b_dense_bwd_x_ordered, which takes e3b_dense_bwd_x_scratch_bytes(plan_host, num_rows) bytes of scratch (at most about
- * 128 MB: more rows are taken in turns; may be NULL when that is 0 or grad_x2 is NULL).
- * e3b_dense_bwd_x_supported(plan_host): 1 when every irrep of the plan has l <= 3 and x2's row fits the kernel's shared
+ * zero); the one of the narrower operand is summed over blocks of 32 channels of the other's irreps, by float atomics in
+ * e3b_dense_bwd_x and in a fixed order in e3b_dense_bwd_x_ordered, which takes e3b_dense_bwd_x_scratch_bytes(plan_host,
+ * num_rows) bytes of scratch (at most about 128 MB: more rows are taken in turns; may be NULL when that is 0).
+ * e3b_dense_bwd_x_supported(plan_host): 1 when every irrep of the plan has l <= 3 and the narrower operand's row fits the kernel's shared
  * memory, else 0 (the caller then evaluates the two transposed products with e3b_dense_fwd).
  */
 int e3b_dense_bwd_x_supported(const int32_t* plan_host);

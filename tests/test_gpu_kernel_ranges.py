@@ -54,6 +54,10 @@ TILE_LAYOUTS = [
     ("65x0e+5x1o+2x2e", "1x0e+1x1o+1x2e", "130x0e+64x1o+1x2e"),    # column blocks of 128 + 2, one output channel
     ("4x3o+7x2e", "3o+2e+1o", "9x0e+33x3o+2x1o"),                  # l = 3 throughout
     ("3x4e+2x0e", "2x1o+4e", "5x4e+2x0e+3x3o"),                    # l = 4: staged without the unrolled irreps, derived products backward
+    ("2x0e+3x1o", "33x0e+9x1o+40x2e", "9x0e+33x1o+5x2e"),          # operands exchanged: the second one's channels are taken by 32
+    ("9x0e+8x1o", "5x0e+12x1o", "8x0e+8x1o"),                      # around eight channels a chunk
+    ("2x0e+1x1o", "3x0e+1x1o", "40x0e+7x1o"),                      # a few channels: the table-driven kernel forward
+    ("1x0e+2x2e", "20x0e+20x4e", "5x0e+6x2e"),                     # l = 4 in the wide operand, which stays second
     ("8x0e+8x1o", "5x0e", "8x0e+8x1o+4x2e"),                       # scalar second operand, an output no path writes
 ]
 
@@ -86,6 +90,7 @@ def test_fp32_product_tiles(layout, rows):
 
 @pytest.mark.parametrize("layout,rows", [(("65x0e+33x1o+32x2e", "1x0e+1x1o+1x2e", "32x0e+32x1o+32x2e"), 4000),      # 6 blocks of channels
                                          (("320x0e+64x1o", "300x0e+60x1o", "2x0e"), 6000),                      # 12, rows in two turns
+                                         (("3x0e+2x1o", "40x0e+70x1o", "8x0e+4x1o"), 1000),                     # operands exchanged, 5
                                          (("32x0e", "1x0e+1x1o", "8x0e+8x1o"), 100)])                           # one: no partials
 def test_fp32_product_second_operand_gradient_repeats(layout, rows):
     """Bit for bit: the same on every call, and for a row whatever rows stand beside it."""
@@ -105,15 +110,15 @@ def test_fp32_product_second_operand_gradient_repeats(layout, rows):
 
 @pytest.mark.parametrize("tail", ["2x3o", "2x0e"])
 def test_fp32_product_many_outputs_wide_second_operand(tail):
-    """33 output irreps (32 go out in one launch) and a second operand of 1,280 columns: with the l = 3 irrep last, the first 32
+    """33 output irreps (32 go out in one launch) and operands of 1,280 columns: with the l = 3 irrep last, the first 32
     fit a block's shared memory and the last does not.  Outputs start from NaN.  Bound: 1e-5 x RMS, or 1.5 times the distance of
-    plain fp32 arithmetic on the host where that is larger (sums of up to 5,280 terms)."""
-    rows = 40
+    plain fp32 arithmetic on the host where that is larger (sums of thousands of terms)."""
+    rows = 12
     g = torch.Generator().manual_seed(5)
     outs = "+".join(["2x0e"] * 32 + [tail])
     ins = [(i, j, k, "uvw", True) for k, l in enumerate([0] * 32 + [3 if tail == "2x3o" else 0])
            for i, j in [(0, 0), (3, 3), (0, 3), (3, 0)] if (l == 3) == (i != j)]
-    tp = o3.TensorProduct("2x0e+2x1o+2x2e+2x3o", "80x0e+80x1o+80x2e+80x3o", outs, ins)
+    tp = o3.TensorProduct("80x0e+80x1o+80x2e+80x3o", "80x0e+80x1o+80x2e+80x3o", outs, ins)
     x, y = torch.randn(rows, tp.irreps_in1.dim, generator=g), torch.randn(rows, tp.irreps_in2.dim, generator=g)
     go = torch.randn(rows, tp.irreps_out.dim, generator=g)
     want = []

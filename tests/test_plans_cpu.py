@@ -47,11 +47,12 @@ class SecondPart:
     def __init__(self, plan: np.ndarray):
         assert plan[0] == MAGIC and len(plan) == plan[6]
         self.plan = plan
-        h = [int(v) for v in plan[int(plan[-1]) : int(plan[-1]) + 12]]
-        self.d1max, self.d3max, self.covered = h[8], h[9], h[11]
+        h = [int(v) for v in plan[int(plan[-1]) : int(plan[-1]) + 14]]
+        self.d1max, self.d3max, self.covered, self.swapped = h[8], h[9], h[11], h[12]
         rows = lambda n, at, width: plan[at : at + n * width].reshape(n, width).tolist()      # noqa: E731
         self.groups, self.chunks, self.paths = rows(h[0], h[1], 6), rows(h[2], h[3], 6), rows(h[4], h[5], 16)
         self.in_groups = rows(h[6], h[7], 5)
+        assert h[13] == sum(c[2] for c in self.chunks)
         self.in_paths = plan[h[10] : h[10] + sum(g[4] for g in self.in_groups)].tolist()
 
     def _segment(self, at: int, n: int):
@@ -73,6 +74,7 @@ class SecondPart:
 
     def _walk(self, x1, x2):
         """(group, A of the chunk, flat weight indices [channel, output channel]) of every chunk; T is kept as the kernels do."""
+        x1, x2 = (x2, x1) if self.swapped else (x1, x2)
         for out_off, mo, d3, first, n, _ in self.groups:
             t_of = None
             for pid, x1off, channels, x2off, wbase, fresh in self.chunks[first : first + n]:
@@ -95,6 +97,8 @@ class SecondPart:
         return gw
 
     def operand_gradients(self, x1, x2, W, g):
+        if self.swapped:
+            x1, x2 = x2, x1
         g1, g2 = np.zeros_like(x1), np.zeros_like(x2)
         for x1off, m1, d1, first, n in self.in_groups:
             for pid in self.in_paths[first : first + n]:
@@ -112,7 +116,7 @@ class SecondPart:
                         for i in range(d1):
                             t = sum(c * x2[:, x2off + v * d2 + j] for j, c in self._segment(ki, k * d1 + i))
                             g1[:, x1off : x1off + m1 * d1].reshape(-1, m1, d1)[:, :, i] += np.reshape(t, (-1, 1)) * q[:, :, k]
-        return g1, g2
+        return (g2, g1) if self.swapped else (g1, g2)
 
 
 def _ins(tp):
@@ -134,10 +138,15 @@ def test_uvw_plan_matches_oracle():
     assert rel_err(torch.from_numpy(got), _oracle_tp(tp, x1, x2, w)) < 1e-6
 
 
-@pytest.mark.parametrize("layout", [("3x0e+2x1o+4x2e+1x1e", "2x0e+3x1o+1x2e", "5x0e+2x1o+3x2e+2x1e+1x3o"),
-                                    ("33x0e+65x1o", "1x0e+2x1o", "40x0e+1x1o+2x1e"),          # more than a chunk of channels
-                                    ("2x4e+1x0e+3x5o", "1x4e+2x0e", "2x4e+1x0e+0x1o")])       # an operand block no path leaves
-def test_second_part_of_product_plans(layout):
+@pytest.mark.parametrize("layout,swapped", [
+    (("3x0e+2x1o+4x2e+1x1e", "2x0e+3x1o+1x2e", "5x0e+2x1o+3x2e+2x1e+1x3o"), False),
+    (("33x0e+65x1o", "1x0e+2x1o", "40x0e+1x1o+2x1e"), False),                   # more than a chunk of channels
+    (("1x0e+2x1o", "33x0e+65x1o", "40x0e+1x1o+2x1e"), True),                    # the second operand's channels taken by 32
+    (("4x0e+4x1o", "4x0e+4x1o", "2x0e+3x1e"), False),                           # as many either way
+    (("1x0e+2x2e", "20x0e+20x4e", "5x0e+6x2e"), False),                         # l = 4 stays second
+    (("1x0e+2x4e", "20x0e+20x4e", "5x0e+6x2e"), True),                          # l = 4 either way
+    (("2x4e+1x0e+3x5o", "1x4e+2x0e", "2x4e+1x0e+0x1o"), False)])                # an operand block no path leaves
+def test_second_part_of_product_plans(layout, swapped):
     """What the register-tile kernels read: forward and all gradients against autograd through the oracle."""
     torch.manual_seed(0)
     tp = o3.FullyConnectedTensorProduct(*layout)
@@ -151,7 +160,10 @@ def test_second_part_of_product_plans(layout):
     got = [part.forward(a, b, ww), part.weight_gradient(a, b, g, len(ww)), *part.operand_gradients(a, b, ww, g)]
     for x, y in zip(got, want):
         assert rel_err(torch.from_numpy(x), y) < 1e-6        # (the coefficients are fp32)
-    assert bool(part.covered) == all(any(i.i_in1 == n and 0 not in i.path_shape for i in tp.instructions) for n, m in enumerate(tp.irreps_in1) if m.dim > 0)
+    assert bool(part.swapped) == swapped
+    first, where = (tp.irreps_in2, "i_in2") if swapped else (tp.irreps_in1, "i_in1")
+    live = {getattr(i, where) for i in tp.instructions if 0 not in i.path_shape}
+    assert bool(part.covered) == all(n in live for n, m in enumerate(first) if m.dim > 0)
 
 
 def test_second_part_of_linear_plans():
