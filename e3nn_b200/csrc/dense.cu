@@ -1,5 +1,6 @@
-// fp32 CUDA-core evaluation of 'uvw' tensor-product paths with per-row weights or a few channels, and of the per-irrep Linear
-// with Gate as its epilogue above l = 3 (other weight-shared contractions: dense_tile.cu).  Table driven (no per-layout code): the host
+// fp32 CUDA-core evaluation of 'uvw' tensor-product paths with per-row weights or a few channels, of the per-irrep Linear
+// with Gate as its epilogue above l = 3 and over many narrow blocks, and of the weight gradient of products whose blocks fill
+// the register tiles badly (other weight-shared contractions: dense_tile.cu).  Table driven (no per-layout code): the host
 // describes the contraction as a "dense plan" and this kernel evaluates, per output irrep ("group"),
 //
 //     out[z, w, k] = sum_K  A[z, k, K] * W[wbase(K) + w * wstride]
@@ -203,6 +204,109 @@ __global__ void __launch_bounds__(kDenseThreads) dense_fwd_kernel(const int32_t*
     }
 }
 
+// Gradient w.r.t. the shared weights of the same plan:
+//
+//     grad_W[wbase(K) + w * wstride] += sum_{z, k}  A[z, k, K] * grad_out[z, out_off + w * dim3 + k]
+//
+// i.e. per group the product A^T G whose summation index is (row, component).  A block owns a
+// kBwKc x kBwWc block of (K, w), keeps its accumulators in registers over all the row tiles it
+// visits (rounding: one partial sum per tile, added to the running sum) and adds them to the zeroed
+// gradient with float atomics at the end.  Per tile it stages the A columns of its K block (same
+// construction as phase 1 of the forward kernel) and the cotangent columns of its w block.
+constexpr int kBwKc = 64;    // contraction entries per block
+constexpr int kBwWc = 128;   // output channels per block
+constexpr int kBwTK = 8;     // contraction entries per thread
+constexpr int kBwTW = 4;     // output channels per thread
+
+__global__ void __launch_bounds__(kDenseThreads) dense_bwd_w_kernel(const int32_t* __restrict__ plan,
+        const float* __restrict__ x1, const float* __restrict__ x2, const float* __restrict__ gout,
+        float* __restrict__ grad_w, int64_t Z, int group, int rows_z, int n_wc) {
+    extern __shared__ __align__(16) float smem[];
+    float* sA = smem;                                          // [r][kk]
+    float* sG = smem + kRowsPerPass * kBwKc;                   // [r][w]
+    int* sWb = reinterpret_cast<int*>(sG + kRowsPerPass * kBwWc);
+    const int d1 = plan[1], d2 = plan[2], dout = plan[3];
+    const int32_t* gp = plan + plan[7] + 6 * group;
+    const DenseGroup g{gp[0], gp[1], gp[2], gp[3], gp[4], gp[5]};
+    const int32_t* pathk_dir = plan + plan[9];
+    const int32_t* cg = plan + plan[10];
+    const int kc0 = (blockIdx.y / n_wc) * kBwKc, wc0 = (blockIdx.y % n_wc) * kBwWc;
+    const int32_t* kent = plan + plan[8] + 4 * (g.kent_start + kc0);
+    const int nk = min(kBwKc, g.K - kc0), nw = min(kBwWc, g.mul_out - wc0);
+    const int RT = rows_z * g.dim3;
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+    if (tid < kBwKc) sWb[tid] = tid < nk ? kent[4 * tid + 3] : 0;
+
+    float acc[kBwTK][kBwTW];
+#pragma unroll
+    for (int i = 0; i < kBwTK; ++i)
+#pragma unroll
+        for (int j = 0; j < kBwTW; ++j) acc[i][j] = 0.0f;
+
+    const int64_t tiles = (Z + rows_z - 1) / rows_z;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t z0 = tile * rows_z;
+        __syncthreads();
+        for (int idx = tid; idx < RT * kBwKc; idx += kDenseThreads) {
+            const int r = idx / kBwKc, kk = idx - r * kBwKc;
+            const int zl = r / g.dim3, k = r - zl * g.dim3;
+            const int64_t z = z0 + zl;
+            float a = 0.0f;
+            if (z < Z && kk < nk) {
+                const int path = kent[4 * kk], x1off = kent[4 * kk + 1], x2off = kent[4 * kk + 2];
+                const int32_t* pk = plan + pathk_dir[path] + 2 * k;
+                const int cstart = pk[0], ccount = pk[1];
+                const float* xr = x1 + z * d1 + x1off;
+                const float* yr = x2off >= 0 ? x2 + z * d2 + x2off : nullptr;
+                for (int c = 0; c < ccount; ++c) {
+                    const int32_t* t = cg + 3 * (cstart + c);
+                    a = fmaf(__int_as_float(t[2]) * xr[t[0]], yr ? yr[t[1]] : 1.0f, a);
+                }
+            }
+            sA[idx] = a;
+        }
+        for (int idx = tid; idx < RT * kBwWc; idx += kDenseThreads) {
+            const int r = idx / kBwWc, w = idx - r * kBwWc;
+            const int zl = r / g.dim3, k = r - zl * g.dim3;
+            const int64_t z = z0 + zl;
+            sG[idx] = (z < Z && w < nw) ? gout[z * dout + g.out_off + (wc0 + w) * g.dim3 + k] : 0.0f;
+        }
+        __syncthreads();
+        float part[kBwTK][kBwTW];
+#pragma unroll
+        for (int i = 0; i < kBwTK; ++i)
+#pragma unroll
+            for (int j = 0; j < kBwTW; ++j) part[i][j] = 0.0f;
+#pragma unroll 4
+        for (int r = 0; r < RT; ++r) {
+            const float4 a0 = *reinterpret_cast<const float4*>(sA + r * kBwKc + ty * kBwTK);
+            const float4 a1 = *reinterpret_cast<const float4*>(sA + r * kBwKc + ty * kBwTK + 4);
+            const float4 gv = *reinterpret_cast<const float4*>(sG + r * kBwWc + tx * kBwTW);
+            const float a[kBwTK] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const float b[kBwTW] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+            for (int i = 0; i < kBwTK; ++i)
+#pragma unroll
+                for (int j = 0; j < kBwTW; ++j) part[i][j] = fmaf(a[i], b[j], part[i][j]);
+        }
+#pragma unroll
+        for (int i = 0; i < kBwTK; ++i)
+#pragma unroll
+            for (int j = 0; j < kBwTW; ++j) acc[i][j] += part[i][j];
+    }
+    __syncthreads();   // sWb (written before the loop) is visible even when this block had no tile
+#pragma unroll
+    for (int i = 0; i < kBwTK; ++i) {
+        const int kk = ty * kBwTK + i;
+        if (kk >= nk) continue;
+#pragma unroll
+        for (int j = 0; j < kBwTW; ++j) {
+            const int w = tx * kBwTW + j;
+            if (w < nw) atomicAdd(grad_w + sWb[kk] + static_cast<int64_t>(wc0 + w) * g.w_stride, acc[i][j]);
+        }
+    }
+}
+
 // out[z, c] (+)= bias[c] over listed column ranges / zero fill of untouched columns.
 __global__ void dense_fill_kernel(float* __restrict__ out, int64_t Z, int dout, int col0, int ncol,
                                   const float* __restrict__ bias /* may be null: zero fill */, int add) {
@@ -298,11 +402,31 @@ extern "C" int e3b_dense_fwd_gate(const int32_t* plan_host, const int32_t* plan_
 extern "C" int e3b_dense_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2,
                                const float* grad_out, float* grad_weight, int64_t num_rows, void* stream) {
     using namespace e3b;
-    if (!whole_plan(plan_host)) return fail(E3B_ERR_ARG, "dense_bwd_w: bad plan (one without its second part has to be built again)");
+    if (!any_plan(plan_host)) return fail(E3B_ERR_ARG, "dense_bwd_w: bad plan");
     if (num_rows < 0) return fail(E3B_ERR_ARG, "dense_bwd_w: negative row count");
     if (num_rows == 0) return E3B_OK;
     if (!plan_dev || !x1 || !grad_out || !grad_weight) return fail(E3B_ERR_ARG, "dense_bwd_w: null pointer");
-    return launch_dense_tile_bwd_w(plan_host, plan_dev, x1, x2, grad_out, grad_weight, num_rows, static_cast<cudaStream_t>(stream));
+    if (whole_plan(plan_host) && !pairs_bwd_w(plan_host, num_rows))
+        return launch_dense_tile_bwd_w(plan_host, plan_dev, x1, x2, grad_out, grad_weight, num_rows, static_cast<cudaStream_t>(stream));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int n_groups = plan_host[4];
+    const int32_t* groups = plan_host + plan_host[7];
+    for (int g = 0; g < n_groups; ++g) {
+        const int mul_out = groups[6 * g + 1], dim_out = groups[6 * g + 2], K = groups[6 * g + 3];
+        if (K == 0 || mul_out == 0) continue;
+        if (dim_out > kRowsPerPass) return fail(E3B_ERR_UNSUPPORTED, "dense_bwd_w: irrep dimension %d too large", dim_out);
+        const int rows_z = kRowsPerPass / dim_out;
+        const int n_kc = (K + kBwKc - 1) / kBwKc, n_wc = (mul_out + kBwWc - 1) / kBwWc;
+        const int64_t tiles = ceil_div(num_rows, rows_z);
+        const int64_t want = std::max<int64_t>(1, (static_cast<int64_t>(kNumSMs) * 3 + n_kc * n_wc - 1) / (n_kc * n_wc));
+        const dim3 grid(static_cast<unsigned>(std::min<int64_t>(tiles, want)), static_cast<unsigned>(n_kc * n_wc));
+        constexpr int smem = static_cast<int>(sizeof(float)) * (kRowsPerPass * (kBwKc + kBwWc) + kBwKc);
+        E3B_CUDA_TRY(cudaFuncSetAttribute(dense_bwd_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        dense_bwd_w_kernel<<<grid, kDenseThreads, smem, s>>>(plan_dev, x1, x2, grad_out, grad_weight, num_rows, g, rows_z, n_wc);
+        int rc = check_launch("e3b_dense_bwd_w");
+        if (rc != E3B_OK) return rc;
+    }
+    return E3B_OK;
 }
 
 extern "C" int e3b_fill_columns(float* out, int64_t num_rows, int row_stride, int col0, int ncol, const float* bias,

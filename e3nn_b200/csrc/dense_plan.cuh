@@ -27,8 +27,9 @@ struct DenseGateEpilogue {
 // The Linear of a plan with Gate as its epilogue on the row kernels; *done = false: the plan has irreps of l > 3.
 int launch_dense_rows_gate(const int32_t* plan_host, const int32_t* plan_dev, const float* x, const float* weight,
                            const DenseGateEpilogue& ep, int64_t num_rows, cudaStream_t s, bool* done);
-// Whether a product has too few channels in its chunks for the register tiles (forward).
+// Whether the table-driven kernels of dense.cu are faster than the register tiles: forward, and for the weight gradient.
 bool few_channels(const int32_t* plan_host);
+bool pairs_bwd_w(const int32_t* plan_host, int64_t num_rows);
 int launch_dense_tile_fwd(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,
                           float* out, int64_t num_rows, int accumulate, cudaStream_t s);
 int launch_dense_tile_bwd_w(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* grad_out,

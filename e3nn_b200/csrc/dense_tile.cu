@@ -1229,7 +1229,10 @@ inline size_t bwd_x_shared(const Part2& P, bool need2) {
 // Under eight channels a chunk the table-driven kernel (dense.cu), whose contraction index runs over all pairs of channels, is
 // the faster one: 10,000 rows of 4 x 4 -> 64 channels, l <= 2, 169 against 187 us, 100,000 rows of 1 x 1 -> 1, 294 against 504;
 // with eight (30,000 rows of 8 x 8 -> 64) 1,313 against 1,051.
+// A Linear goes there when an output has many such chunks, each with its copies and a barrier: 30,000 rows of 300 x 1 channel
+// 648 -> 255 us; a few (4x0e+4x1o) are 17 us on the tiles against 79.
 constexpr int64_t kFewChannels = 8;
+constexpr int kFewChannelsChunks = 24;
 
 bool too_many_blocks(int64_t blocks) { return blocks > 2147483647LL; }
 
@@ -1362,7 +1365,33 @@ int launch_dense_rows_gate(const int32_t* plan_host, const int32_t* plan_dev, co
 
 bool few_channels(const int32_t* plan_host) {
     const Part2 P(plan_host);
-    return coupled_plan(P) && P.channels() < kFewChannels * P.n_chunks();
+    if (P.channels() >= kFewChannels * P.n_chunks()) return false;
+    if (coupled_plan(P)) return true;
+    if (plan_host[4] != P.n_groups()) return false;      // a transposed Linear whose first part adds up groups
+    int most = 0;
+    for (int g = 0; g < P.n_groups(); ++g) most = std::max(most, P.group(g)[4]);
+    return most > kFewChannelsChunks;
+}
+
+// The table-driven kernel contracts 64 pairs of channels and up to 128 output channels a block, however they come about; the
+// register tiles take a chunk of 32 channels for every channel of the second operand, half as fast beyond 64 output channels.
+// Both sides in microseconds a row as measured (l <= 2), and what the table takes to start: 30,000 rows of 4 x 4 -> 4 channels 422
+// (table) and 1,789 us, 8 x 8 -> 64 1,613 / 3,729, 16 x 16 -> 16 5,780 / 7,723, but 16 x 3 -> 16 1,260 / 1,083, 32 x 8 -> 32 5,947 /
+// 3,627 and 32 x 1 -> 32 816 / 270; 2,000 rows: 4 x 4 -> 4 95 / 129, 16 x 16 -> 16 433 / 526, 2 x 2 -> 2 85 / 64.
+bool pairs_bwd_w(const int32_t* plan_host, int64_t num_rows) {
+    const Part2 P(plan_host);
+    if (!coupled_plan(P)) return false;
+    const int32_t* first = plan_host + plan_host[7];
+    double chunks = 0.0, blocks = 0.0;
+    for (int n = 0; n < P.n_groups(); ++n) {
+        const int mo = P.group(n)[1], wide = (mo + 127) / 128;
+        if (first[6 * n + 2] > kBwRows) return false;
+        chunks += P.group(n)[4] * wide * (mo > 64 ? 1.5 : 1.0);
+        blocks += (first[6 * n + 3] + 63) / 64 * wide;
+    }
+    chunks /= std::max(P.n_groups(), 1);
+    blocks /= std::max(P.n_groups(), 1);
+    return static_cast<double>(num_rows) * ((chunks > 12.0 ? 0.0036 : 0.0028) * chunks - 0.0124 * blocks) > 45.0;
 }
 
 int launch_dense_tile_fwd(const int32_t* plan_host, const int32_t* plan_dev, const float* x1, const float* x2, const float* weight,

@@ -215,8 +215,8 @@ int e3b_gate_bwd(const float* x, const float* grad_out, const int32_t* in_table,
  * per-irrep Linear out[z,w,i] = pw sum_u W[u,w] x[z,u,i] (e3nn/o3/_linear.py:445-469).
  * The contraction is described by a "dense plan": int32 words built on the host
  * (layout documented in e3nn_b200/csrc/dense.cu and dense_tile.cu); plan_host is that array in HOST memory,
- * plan_dev a copy in device memory.  Plans of the first part alone (magic 0x65336250) are taken by e3b_dense_fwd and
- * e3b_dense_fwd_gate; the gradients need both parts.  x2 may be NULL for plans that never read it (Linear).
+ * plan_dev a copy in device memory.  Plans of the first part alone (magic 0x65336250) are taken by all but
+ * e3b_dense_bwd_x.  x2 may be NULL for plans that never read it (Linear).
  * weight_row_stride: 0 for shared weights [weight_numel]; otherwise row z reads its own weights at
  * weight + z * weight_row_stride (e3nn's shared_weights=False).
  * accumulate != 0 adds to out instead of overwriting the columns the plan writes; columns no

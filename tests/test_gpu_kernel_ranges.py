@@ -88,6 +88,23 @@ def test_fp32_product_tiles(layout, rows):
         assert rel_err(torch.autograd.grad(other, leaf, go.to(DEV))[0].cpu(), ref_g[n]) < 1e-5
 
 
+@pytest.mark.parametrize("rows", [500, 4000])
+@pytest.mark.parametrize("layout", [("4x0e+4x1o", "4x0e+4x1o", "5x0e+3x1o"), ("9x0e+5x1o", "9x0e+9x1o", "70x0e+130x1o"), ("16x0e+4x2e", "16x0e+4x2e", "9x0e+2x2e")])
+def test_fp32_product_weight_gradient_over_pairs(layout, rows):
+    """Poorly filled chunks: at the larger row counts the weight gradient contracts pairs of channels.  Bound: 1e-5 x RMS, the
+    fp32 parity bound of this path."""
+    g = torch.Generator().manual_seed(rows)
+    tp = o3.FullyConnectedTensorProduct(*layout)
+    x, y, go = (torch.randn(rows, d, generator=g) for d in (tp.irreps_in1.dim, tp.irreps_in2.dim, tp.irreps_out.dim))
+    ins = [(i.i_in1, i.i_in2, i.i_out, i.connection_mode, i.has_weight) for i in tp.instructions]
+    w64 = tp.weight.detach().double().requires_grad_(True)
+    ref = orc.tensor_product(*(str(i) for i in (tp.irreps_in1, tp.irreps_in2, tp.irreps_out)), ins, x.double(), y.double(), w64, True)
+    (want,) = torch.autograd.grad(ref, w64, go.double())
+    tp = tp.to(DEV)
+    (got,) = torch.autograd.grad(tp(x.to(DEV), y.to(DEV)), tp.weight, go.to(DEV))
+    assert rel_err(got.cpu(), want) < 1e-5
+
+
 @pytest.mark.parametrize("layout,rows", [(("65x0e+33x1o+32x2e", "1x0e+1x1o+1x2e", "32x0e+32x1o+32x2e"), 4000),      # 6 blocks of channels
                                          (("320x0e+64x1o", "300x0e+60x1o", "2x0e"), 6000),                      # 12, rows in two turns
                                          (("3x0e+2x1o", "40x0e+70x1o", "8x0e+4x1o"), 1000),                     # operands exchanged, 5
@@ -156,10 +173,11 @@ def test_fp32_rounding_of_long_sums_over_narrow_blocks():
 
 @pytest.mark.parametrize("rows", [1, 257])
 @pytest.mark.parametrize("irreps", [("1x0e+40x1o+3x2e", "200x0e+2x0e+17x1o"), ("70x0e+9x4e", "9x4e+16x0e+5x1o"), ("64x0e+64x3o", "32x0e+64x3o"),
-                                    ("40x16e+3x31o+2x0e", "70x16e+130x31o+5x0e")])
+                                    ("40x16e+3x31o+2x0e", "70x16e+130x31o+5x0e"),
+                                    ("+".join(["1x0e", "2x1o"] * 24), "7x0e+5x1o"), ("+".join(["1x0e", "2x1o"] * 25), "7x0e+5x1o+1x0o")])
 def test_fp32_linear_tiles(irreps, rows):
-    """Forward, transposed (two outputs of different width from one input, an input nothing reads) and weight gradient; the
-    last layout has more components than a tile of 128 columns has rows, up to the largest irrep taken."""
+    """Forward, transposed (two outputs of different width from one input, an input nothing reads) and weight gradient; one
+    layout has more components than a tile of 128 columns has rows, up to the largest irrep taken, two have many narrow blocks."""
     g = torch.Generator().manual_seed(rows)
     lin = o3.Linear(*irreps)
     x, go = torch.randn(rows, lin.irreps_in.dim, generator=g), torch.randn(rows, lin.irreps_out.dim, generator=g)

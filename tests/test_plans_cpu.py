@@ -239,7 +239,7 @@ def _cg_words(plan: np.ndarray) -> int:
 
 
 def test_plans_without_a_second_part():
-    """Modules saved with such plans get new ones when they are loaded; the entry points that need the second part refuse."""
+    """Modules saved with such plans get new ones when they are loaded; the entry point that needs the second part refuses."""
     import pickle
 
     from e3nn_b200 import _lib
@@ -257,7 +257,6 @@ def test_plans_without_a_second_part():
     assert lin2._reads_all and tp2._uvw_written == written
     core, host = _lib.core(), tp._plan_host.ctypes.data
     assert core.e3b_dense_bwd_x_supported(host) == 0 and core.e3b_dense_bwd_x_supported(plans[0].ctypes.data) == 1
-    assert core.e3b_dense_bwd_w(host, None, None, None, None, None, 5, None) == -1
     assert core.e3b_dense_bwd_x(host, None, None, None, None, None, None, None, 5, None) == -1
 
 
