@@ -47,7 +47,8 @@ __device__ __forceinline__ void tn_fetch(float* sx, float* sg, const float* __re
     }
 }
 
-template <int TN, bool VEC>
+// RUNS: a block has more than kTnMostRows rows and adds one run of them after another in its entries of `out`.
+template <int TN, bool VEC, bool RUNS>
 __global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kernel(const float* __restrict__ x, const float* __restrict__ g, int64_t Z, int M,
                                                                   int N, int64_t rows_per_split, float scale, float* __restrict__ out) {
     extern __shared__ __align__(16) float smem[];
@@ -67,47 +68,49 @@ __global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kerne
         if (step < steps) tn_fetch<TN, VEC>(s, s + kTnRows * kTnM, x, g, z_begin + step * kTnRows, z_end, m0, n0, M, N);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // this run's sums into the block's own entries of `out`, which hold the runs before
+    for (int s = 0; s < kTnStages - 1; ++s) fetch(s);
     float* o = out + static_cast<int64_t>(blockIdx.z) * M * N;
-    auto flush = [&](bool first) {
+    constexpr int64_t kRun = kTnMostRows / kTnRows;
+    for (int64_t from = 0, to = 0; to < steps; from = to) {
+        to = RUNS && from + kRun < steps ? from + kRun : steps;
+        for (int64_t step = from; step < to; ++step) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kTnStages - 2) : "memory");
+            __syncthreads();            // this stage has landed for everyone; the stage fetched next is free
+            fetch(step + kTnStages - 1);
+            const float* sx = smem + (step % kTnStages) * tn_stage_floats<TN>();
+            const float* sg = sx + kTnRows * kTnM;
+#pragma unroll
+            for (int k = 0; k < kTnRows; ++k) {
+                const float4 a0 = *reinterpret_cast<const float4*>(sx + k * kTnM + ty * 4);
+                const float4 a1 = *reinterpret_cast<const float4*>(sx + k * kTnM + 32 + ty * 4);
+                const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+                float2 b[NP];
+#pragma unroll
+                for (int j = 0; j < NP / 2; ++j) {
+                    const float4 v = *reinterpret_cast<const float4*>(sg + k * TN + 64 * j + tx * 4);
+                    b[2 * j] = make_float2(v.x, v.y);
+                    b[2 * j + 1] = make_float2(v.z, v.w);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int m = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
+            if (m >= M) continue;
 #pragma unroll
             for (int j = 0; j < NP; ++j) {
                 const int n = n0 + (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
                 float* p = o + static_cast<int64_t>(m) * N + n;
-                if (m < M && n < N) p[0] = first ? scale * acc[i][j].x : fmaf(scale, acc[i][j].x, p[0]);
-                if (m < M && n + 1 < N) p[1] = first ? scale * acc[i][j].y : fmaf(scale, acc[i][j].y, p[1]);
-                acc[i][j] = make_float2(0.0f, 0.0f);
+                const bool add = RUNS && from > 0;
+                if (n < N) p[0] = add ? fmaf(scale, acc[i][j].x, p[0]) : scale * acc[i][j].x;
+                if (n + 1 < N) p[1] = add ? fmaf(scale, acc[i][j].y, p[1]) : scale * acc[i][j].y;
+                if (RUNS) acc[i][j] = make_float2(0.0f, 0.0f);
             }
         }
-    };
-    for (int s = 0; s < kTnStages - 1; ++s) fetch(s);
-    for (int64_t step = 0; step < steps; ++step) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kTnStages - 2) : "memory");
-        __syncthreads();            // this stage has landed for everyone; the stage fetched next is free
-        fetch(step + kTnStages - 1);
-        const float* sx = smem + (step % kTnStages) * tn_stage_floats<TN>();
-        const float* sg = sx + kTnRows * kTnM;
-#pragma unroll
-        for (int k = 0; k < kTnRows; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(sx + k * kTnM + ty * 4);
-            const float4 a1 = *reinterpret_cast<const float4*>(sx + k * kTnM + 32 + ty * 4);
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            float2 b[NP];
-#pragma unroll
-            for (int j = 0; j < NP / 2; ++j) {
-                const float4 v = *reinterpret_cast<const float4*>(sg + k * TN + 64 * j + tx * 4);
-                b[2 * j] = make_float2(v.x, v.y);
-                b[2 * j + 1] = make_float2(v.z, v.w);
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < NP; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
-        }
-        if (step + 1 == steps || (step + 1) % (kTnMostRows / kTnRows) == 0) flush(step < kTnMostRows / kTnRows);
     }
 }
 
@@ -169,8 +172,11 @@ extern "C" int e3b_matmul_tn(const float* x, const float* g, int64_t rows, int m
     const bool vec = m % 4 == 0 && n % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
     const dim3 grid(p.tiles_n, p.tiles_m, p.splits);
     const int smem = kTnStages * static_cast<int>(sizeof(float)) * (p.tn == 256 ? tn_stage_floats<256>() : tn_stage_floats<128>());
-    auto kernel = p.tn == 256 ? (vec ? matmul_tn_kernel<256, true> : matmul_tn_kernel<256, false>)
-                              : (vec ? matmul_tn_kernel<128, true> : matmul_tn_kernel<128, false>);
+    const bool runs = p.rows > kTnMostRows;
+    auto kernel = p.tn == 256 ? (vec ? (runs ? matmul_tn_kernel<256, true, true> : matmul_tn_kernel<256, true, false>)
+                                     : (runs ? matmul_tn_kernel<256, false, true> : matmul_tn_kernel<256, false, false>))
+                              : (vec ? (runs ? matmul_tn_kernel<128, true, true> : matmul_tn_kernel<128, true, false>)
+                                     : (runs ? matmul_tn_kernel<128, false, true> : matmul_tn_kernel<128, false, false>));
     E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     float* to = p.splits > 1 ? static_cast<float*>(scratch) : out;
     kernel<<<grid, kTnThreads, smem, s>>>(x, g, rows, m, n, p.rows, p.splits > 1 ? 1.0f : scale, to);
