@@ -246,7 +246,8 @@ struct V2Ids {{
     }}
 }};
 
-// One lane per edge: harmonics of a batch of <= 32 consecutive slots into shared memory.
+// One lane per edge: harmonics of a batch of <= 32 consecutive slots into shared memory.  A slot to be skipped has none: its
+// message is zero (a test of every edge in the loop over them costs the forward kernel 3 % on 15 paths).
 __device__ __forceinline__ void v2_batch_harmonics(const float* __restrict__ vec, const V2Ids& ids, uint32_t it0, int64_t left, float* ybuf,
                                                    int lane) {{
     if (lane < left) {{
@@ -255,8 +256,9 @@ __device__ __forceinline__ void v2_batch_harmonics(const float* __restrict__ vec
         const float inv = 1.0f / fmaxf(sqrtf(vx * vx + vy * vy + vz * vz), 1e-12f);
         float Y[kD2];
         e3b_sh_fwd<kShLmax>(vx * inv, vy * inv, vz * inv, Y);
+        const bool live = ids.src[(it0 + lane) & 63u] >= 0;
 #pragma unroll
-        for (int j = 0; j < kD2; ++j) ybuf[lane * kV2YStride + j] = Y[j];
+        for (int j = 0; j < kD2; ++j) ybuf[lane * kV2YStride + j] = live ? Y[j] : 0.0f;
     }}
 }}
 
@@ -345,9 +347,7 @@ __global__ void __launch_bounds__(kV2Threads, 1) conv_fwd_tma_kernel(const float
             float Y[kD2];
 #pragma unroll
             for (int j = 0; j < kD2; ++j) Y[j] = ybuf[slot * kV2YStride + j];
-            if (ids.src[it & 63u] >= 0) {{
-{switch([p[1] for p in parts], 16)}
-            }}
+{switch([p[1] for p in parts], 12)}
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&empty[s]);
             if (leader && it > 0 && issue < e_hi) {{
