@@ -69,10 +69,10 @@ __global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kerne
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     for (int s = 0; s < kTnStages - 1; ++s) fetch(s);
-    float* o = out + static_cast<int64_t>(blockIdx.z) * M * N;
     constexpr int64_t kRun = kTnMostRows / kTnRows;
-    for (int64_t from = 0, to = 0; to < steps; from = to) {
-        to = RUNS && from + kRun < steps ? from + kRun : steps;
+    int64_t from = 0;
+    do {
+        const int64_t to = RUNS && from + kRun < steps ? from + kRun : steps;
         for (int64_t step = from; step < to; ++step) {
             asm volatile("cp.async.wait_group %0;" ::"n"(kTnStages - 2) : "memory");
             __syncthreads();            // this stage has landed for everyone; the stage fetched next is free
@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kerne
                     for (int j = 0; j < NP; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
             }
         }
+        float* o = out + static_cast<int64_t>(blockIdx.z) * M * N;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int m = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
@@ -111,7 +112,8 @@ __global__ void __launch_bounds__(kTnThreads, TN == 128 ? 3 : 2) matmul_tn_kerne
                 if (RUNS) acc[i][j] = make_float2(0.0f, 0.0f);
             }
         }
-    }
+        if (RUNS) from = to;
+    } while (RUNS && from < steps);
 }
 
 __global__ void __launch_bounds__(256) matmul_tn_sum_kernel(const float* __restrict__ partial, int splits, int64_t count, float scale,
