@@ -513,7 +513,8 @@ inline size_t fwd_floats(int d1max, int d2row) {
     return w + static_cast<size_t>(BZ) * (pad_row(32 * d1max) + pad_row(32 * D3) + (d1max * D3 | 1) + (d2row | 1));
 }
 
-template <int D3, int TX, bool COUPLED, bool GATE>
+// NARROW: some chunk has fewer than 32 channels.
+template <int D3, int TX, bool COUPLED, bool GATE, bool NARROW>
 __device__ __forceinline__ void fwd_rows_tile(const Part2& P, const int32_t* g, const float* __restrict__ x1, const float* __restrict__ x2,
                                               const float* __restrict__ W, float* __restrict__ out, int64_t Z, int tile, int accumulate,
                                               const DenseGateEpilogue& ep, float* smem) {
@@ -617,7 +618,7 @@ __device__ __forceinline__ void fwd_rows_tile(const Part2& P, const int32_t* g, 
             }
         }
         held += ch[2];
-        bool keep = c + 1 < nch && held + P.chunk(g[3] + c + 1)[2] <= kKC;
+        bool keep = NARROW && c + 1 < nch && held + P.chunk(g[3] + c + 1)[2] <= kKC;
         if (!COUPLED && keep) keep = P.path(P.chunk(g[3] + c + 1)[0])[15] == path[15];      // one coefficient
         if (!keep) {
             held = 0;
@@ -702,13 +703,13 @@ inline FwdShape fwd_shape(int d3, int tx, int d1max, int d2row) {
     }
 }
 
-template <int D3, bool COUPLED, bool GATE>
+template <int D3, bool COUPLED, bool GATE, bool NARROW>
 __device__ __forceinline__ void fwd_rows_tx(int tx, const Part2& P, const int32_t* g, const float* __restrict__ x1, const float* __restrict__ x2,
                                             const float* __restrict__ W, float* __restrict__ out, int64_t Z, int tile, int accumulate,
                                             const DenseGateEpilogue& ep, float* smem) {
-    if (tx == 4) fwd_rows_tile<D3, 4, COUPLED, GATE>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
-    else if (tx == 8) fwd_rows_tile<D3, 8, COUPLED, GATE>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
-    else fwd_rows_tile<D3, 16, COUPLED, GATE>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
+    if (tx == 4) fwd_rows_tile<D3, 4, COUPLED, GATE, NARROW>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
+    else if (tx == 8) fwd_rows_tile<D3, 8, COUPLED, GATE, NARROW>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
+    else fwd_rows_tile<D3, 16, COUPLED, GATE, NARROW>(P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem);
 }
 
 struct RowsLaunch {
@@ -719,7 +720,7 @@ struct RowsLaunch {
     int16_t shape[kMaxGroups];           // forward: threads a row; weight gradient: output channels of a block
 };
 
-template <bool COUPLED, bool GATE>
+template <bool COUPLED, bool GATE, bool NARROW>
 __global__ void __launch_bounds__(kThreads, 3) dense_rows_fwd_kernel(const int32_t* __restrict__ plan, const float* __restrict__ x1,
                                                                      const float* __restrict__ x2, const float* __restrict__ W,
                                                                      float* __restrict__ out, int64_t Z, int accumulate, RowsLaunch L,
@@ -731,10 +732,10 @@ __global__ void __launch_bounds__(kThreads, 3) dense_rows_fwd_kernel(const int32
     const int32_t* g = P.group(L.group[s]);
     const int tile = static_cast<int>(blockIdx.x) - L.first_block[s];
     switch (g[2]) {
-        case 1: fwd_rows_tx<1, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
-        case 3: fwd_rows_tx<3, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
-        case 5: fwd_rows_tx<5, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
-        default: fwd_rows_tx<7, COUPLED, GATE>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+        case 1: fwd_rows_tx<1, COUPLED, GATE, NARROW>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+        case 3: fwd_rows_tx<3, COUPLED, GATE, NARROW>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+        case 5: fwd_rows_tx<5, COUPLED, GATE, NARROW>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
+        default: fwd_rows_tx<7, COUPLED, GATE, NARROW>(L.shape[s], P, g, x1, x2, W, out, Z, tile, accumulate, ep, smem); break;
     }
 }
 
@@ -1268,6 +1269,7 @@ static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, co
                            float* out, int64_t Z, int accumulate, const DenseGateEpilogue& ep, int pass, cudaStream_t s, bool* done) {
     const Part2 P(plan_host);
     const int most = GATE && pass == 1 ? 1 : kMaxGroups;
+    const bool narrow = P.channels() < kKC * P.n_chunks();
     // the narrowest tile that holds the group's channels in one pass, so that the coupled operand is built once
     auto threads_a_row = [](const int32_t* g) { return g[1] <= 32 ? 4 : g[1] <= 64 ? 8 : 16; };
     auto shape_of = [&](const int32_t* g) { return fwd_shape<COUPLED>(g[2], threads_a_row(g), P.d1max(), P.d2row()); };
@@ -1295,7 +1297,7 @@ static int launch_rows_fwd(const int32_t* plan_host, const int32_t* plan_dev, co
         if (L.n == 0) continue;
         L.first_block[L.n] = static_cast<int>(blocks);
         const size_t bytes = floats * sizeof(float);
-        auto kernel = dense_rows_fwd_kernel<COUPLED, GATE>;
+        auto kernel = narrow ? dense_rows_fwd_kernel<COUPLED, GATE, true> : dense_rows_fwd_kernel<COUPLED, GATE, GATE>;
         E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
         kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, weight, out, Z, accumulate, L, ep);
         if (int rc = check_launch("e3b_dense_fwd")) return rc;
