@@ -1073,7 +1073,8 @@ __device__ __forceinline__ void bwd_x_step(const Part2& P, const BwdXStep& s, co
     }
 }
 
-template <int D1, bool NEED1, bool NEED2>
+// RUNS: some block of the first operand takes more than kBxRun additions (put away in between).
+template <int D1, bool NEED1, bool NEED2, bool RUNS>
 __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, const float* __restrict__ x1, const float* __restrict__ x2,
                                             const float* __restrict__ W, const float* __restrict__ gout, float* __restrict__ g1,
                                             float* __restrict__ g2, float* __restrict__ partial, int64_t Z, int block, int first_part,
@@ -1100,7 +1101,7 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
     // wide second operands: the sums so far are put away in grad_x1 now and then, so that the runs of additions stay short
     int run = 0;
     bool away = false;
-    float* orow = NEED1 ? g1 + (z0 + min(ty, live - 1)) * d1row + x1off + u0 * D1 : nullptr;
+    float* orow = RUNS ? g1 + (z0 + min(ty, live - 1)) * d1row + x1off + u0 * D1 : nullptr;
     for (int buf = 0;; buf ^= 1) {
         BwdXStep next = step;
         const bool more = bwd_x_next(P, in, next);
@@ -1117,7 +1118,7 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
         }
         __syncthreads();      // the buffers and the coupling are written again
         if (!more) break;
-        if (NEED1 && (run += step.path[2]) >= kBxRun) {
+        if (RUNS && (run += step.path[2]) >= kBxRun) {
 #pragma unroll
             for (int u = 0; u < kBxU; ++u)
 #pragma unroll
@@ -1143,7 +1144,7 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
             const int zl = warp * 8 + r;
             if (z0 + zl >= Z) break;
             float* o = g1 + (z0 + zl) * d1row + x1off + u0 * D1;
-            for (int e = lane; e < nu * D1; e += 32) o[e] = away ? o[e] + S.g[zl * ld + e] : S.g[zl * ld + e];
+            for (int e = lane; e < nu * D1; e += 32) o[e] = RUNS && away ? o[e] + S.g[zl * ld + e] : S.g[zl * ld + e];
         }
     }
     if (NEED2) {
@@ -1160,7 +1161,7 @@ __device__ __forceinline__ void bwd_x_block(const Part2& P, const int32_t* in, c
     }
 }
 
-template <bool NEED1, bool NEED2>
+template <bool NEED1, bool NEED2, bool RUNS>
 __global__ void __launch_bounds__(kThreads, 3) dense_tile_bwd_x_kernel(const int32_t* __restrict__ plan, const float* __restrict__ x1,
                                                                        const float* __restrict__ x2, const float* __restrict__ W,
                                                                        const float* __restrict__ gout, float* __restrict__ g1,
@@ -1183,10 +1184,10 @@ __global__ void __launch_bounds__(kThreads, 3) dense_tile_bwd_x_kernel(const int
     const int32_t* in = P.in_group(L.group[s]);
     const int block = static_cast<int>(blockIdx.x) - L.first_block[s];
     switch (in[2]) {
-        case 1: bwd_x_block<1, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
-        case 3: bwd_x_block<3, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
-        case 5: bwd_x_block<5, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
-        default: bwd_x_block<7, NEED1, NEED2>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
+        case 1: bwd_x_block<1, NEED1, NEED2, RUNS>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
+        case 3: bwd_x_block<3, NEED1, NEED2, RUNS>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
+        case 5: bwd_x_block<5, NEED1, NEED2, RUNS>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
+        default: bwd_x_block<7, NEED1, NEED2, RUNS>(P, in, x1, x2, W, gout, g1, g2, partial, Z, block, L.first_part[s], S); break;
     }
 }
 
@@ -1495,6 +1496,16 @@ static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const
                         const float* gout, float* g1, float* g2, float* partial, int64_t Z, cudaStream_t s) {
     const Part2 P(plan_host);
     const size_t bytes = bwd_x_shared(P, NEED2);
+    bool runs = false;
+    for (int n = 0; n < P.n_in(); ++n) {
+        const int32_t* in = P.in_group(n);
+        int64_t adds = 0;
+        for (int q = 0; q < in[4]; ++q) {
+            const int32_t* path = P.path(P.in_path(in[3] + q));
+            adds += static_cast<int64_t>(path[10]) * ((path[12] + kKC - 1) / kKC) * path[2];
+        }
+        runs = runs || adds > kBxRun;
+    }
     int g0 = 0, part = 0;
     while (g0 < P.n_in()) {
         BwdXLaunch L;
@@ -1511,7 +1522,7 @@ static int launch_bwd_x(const int32_t* plan_host, const int32_t* plan_dev, const
             ++L.n;
         }
         L.first_block[L.n] = static_cast<int>(blocks);
-        auto kernel = dense_tile_bwd_x_kernel<NEED1, NEED2>;
+        auto kernel = runs ? dense_tile_bwd_x_kernel<NEED1, NEED2, NEED1> : dense_tile_bwd_x_kernel<NEED1, NEED2, false>;
         E3B_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
         kernel<<<static_cast<unsigned>(blocks), kThreads, bytes, s>>>(plan_dev, x1, x2, weight, gout, g1, g2, partial, Z,
                                                                       bwd_x_g_floats(P.d1max(), P.d3max()), L);
