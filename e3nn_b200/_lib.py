@@ -112,7 +112,8 @@ def _raise_status(code: int, what: str) -> None:
 
 
 def status_after_launch(device: torch.device) -> None:
-    """Nothing to enqueue: the kernels write the word in host memory themselves."""
+    """Nothing to enqueue: the kernels write the word in host memory themselves.  Callers that launch through the C entry
+    points and call this after it need not change."""
 
 
 def poll_status(device: torch.device, what: str = "an earlier e3nn_b200 kernel") -> None:

@@ -15,8 +15,8 @@ the launch that writes it), the two modules run one after the other.
 are the faster choice.  Today that is nowhere: the fused pair moves 46 % fewer bytes, but both Linear kernels are
 bound by their epilogues (strided 4-byte stores of the 2l+1 > 1 irreps; the fp32 kernel by its arithmetic), the
 gate adds loads to exactly that part, and the scalar irreps must run as a launch of their own before the gated
-ones: 7.7 ms fused against 4.1 + 2.0 ms on 1,048,576 rows of ``64x0e+64x1o+64x2e+64x3o`` (tensor cores), 28.9 against
-24.5 + 2.0 ms (fp32).
+ones: 7.7 ms fused against 4.1 + 2.0 ms on 1,048,576 rows of ``64x0e+64x1o+64x2e+64x3o`` (tensor cores), 8.5 against
+7.0 ms (fp32; 20,000 rows: 249 against 160 us).
 """
 from __future__ import annotations
 
