@@ -603,7 +603,7 @@ def secondary_workloads(device, tf32_peak: float):
             tp(x, y2)
         ms = _median_launch_ms(lambda: tp(x, y2), 50)
     out.append({"workload": "uvw_cfg1", "metric": "uvw TP rows/sec (10,000 rows, fp32)", "value": 10_000 / (ms * 1e-3),
-                "unit": "rows/s", "kernel": "dense_fwd_kernel", "kernel_ms": ms, "launches": 50,
+                "unit": "rows/s", "kernel": "dense_rows_fwd_kernel", "kernel_ms": ms, "launches": 50,
                 "l2": "operands are L2 resident: launch latency, not bandwidth"})
     del x, y2, tp, flush
     torch.cuda.empty_cache()
@@ -1196,7 +1196,7 @@ def run_uvw_cfg1(args, rank, world, device):
                    "l2": "23 MB of operands, L2 resident: a latency measurement, not a bandwidth one"},
         "roofline": {"bound": "hbm", "achieved": nbytes / (ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": nbytes / (ms * 1e-3) / 1e9 / peak, "traffic": None, "peak_kind": f"of {peak_kind}",
-                     "kernel": "dense_fwd_kernel", "note": "launch bound (3 launches, one per output irrep)"},
+                     "kernel": "dense_rows_fwd_kernel", "note": "launch bound (one launch for the output irreps)"},
         "gpu_launches": max(20, args.steps) * 3,
     }), flush=True)
 
