@@ -1197,7 +1197,7 @@ def run_uvw_cfg1(args, rank, world, device):
         "roofline": {"bound": "hbm", "achieved": nbytes / (ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": nbytes / (ms * 1e-3) / 1e9 / peak, "traffic": None, "peak_kind": f"of {peak_kind}",
                      "kernel": "dense_rows_fwd_kernel", "note": "launch bound (one launch for the output irreps)"},
-        "gpu_launches": max(20, args.steps) * 3,
+        "gpu_launches": max(20, args.steps),
     }), flush=True)
 
 
